@@ -46,34 +46,72 @@ __device__ __forceinline__ double bip_exact_field(const BipFixed &B, int y, int 
                   : exact_field_thread(B.J + i, (size_t)B.N0, qb, B.NB);
 }
 
+// the same, summed by a warp
+__device__ __forceinline__ double bip_exact_field_warp(const BipFixed &B, int y, int i) {
+    const int8_t *qb = B.qB + (size_t)y * B.NB;
+    if (B.J64)
+        return B.side ? exact_field_warp(B.J64 + (size_t)i * B.N0, qb, B.NB)
+                      : exact_field_warp_strided(B.J64 + i, (size_t)B.N0, qb, B.NB);
+    return B.side ? exact_field_warp(B.J + (size_t)i * B.N0, qb, B.NB)
+                  : exact_field_warp_strided(B.J + i, (size_t)B.N0, qb, B.NB);
+}
+
 __device__ __forceinline__ double bip_exact_h(const BipFixed &B, const float *h, int i) {
     return B.h64 ? B.h64[i] : (double)h[i];
 }
 
-// one colour-phase trial of spin i of trotter y on the moving side; returns 1 if accepted
-__device__ __forceinline__ int bip_trial(int8_t *qA, const float *F, const float *h, int Ns, int m, int y, int i,
-                                         uint64_t seed, uint32_t step, uint32_t tag, const StepConst &sc, int algo,
-                                         uint32_t *trace, unsigned long long bitBase, const BipFixed &B) {
-    u32x4 r = draw(seed, (uint32_t)i, (uint32_t)y, step, tag);
-    float u = draw_unit(r.y);
-    size_t o = (size_t)y * Ns + i;
-    float qyx = qA[o];
-    float dE, qL = 0.f, qR = 0.f;
+// one colour-phase trial of spin i of trotter y on the moving side; returns 1 if
+// accepted.
+// kWarp: every lane of the warp calls it, the inactive ones with active = false,
+// and the warp sums the exact field of a flagged lane's trial together.  Most
+// half-steps of a full-grid launch flag some trial, and one thread walking its
+// row or column set the launch's time: bip_flip_half took 30 us at N0 = N1 =
+// 1024, m = 64 and 204 us at 3001 x 2047, m = 200 (means over whole schedules),
+// and takes 7.4 and 21.6 us this way.
+// Else each thread sums its own, which is the faster one in the persistent batch
+// kernel (a served mix of 24 requests: 84.8 ms, 86.8 ms with kWarp): there a CTA
+// spends its time in the field tiles and flags few trials of a phase.
+template <bool kWarp>
+__device__ __forceinline__ int bip_trial(bool active, int8_t *qA, const float *F, const float *h, int Ns, int m, int y,
+                                         int i, uint64_t seed, uint32_t step, uint32_t tag, const StepConst &sc,
+                                         int algo, uint32_t *trace, unsigned long long bitBase, const BipFixed &B) {
     const bool sa = algo == kSAColoring;
-    if (sa) {
-        dE = bip_sa_dE(qyx, h[i], F[o]);
-    } else {
-        int yl = y == 0 ? m - 1 : y - 1, yr = y == m - 1 ? 0 : y + 1;
-        qL = qA[(size_t)yl * Ns + i];
-        qR = qA[(size_t)yr * Ns + i];
-        dE = bip_sqa_dE(qyx, h[i], F[o], qL, qR, sc.twoDivM, sc.coef);
-    }
-    int nearT = 0;
-    const float L = neg_log_unit(u);
     const DecisionTol tol = decision_tol(sa, false, sc.twoDivM, sc.coef, sc.rate);
-    int acc = metropolis_log(dE, sc.rate, L, trial_xtol(tol, h[i], F[o], L), nearT);
-    if (nearT)
-        acc = exact_accept(sa, false, qyx, bip_exact_h(B, h, i), bip_exact_field(B, y, i), qL, qR, m, B.G, B.beta, u);
+    int acc = 0, nearT = 0;
+    float u = 0.f, qyx = 1.f, qL = 0.f, qR = 0.f, L = 0.f;
+    size_t o = 0;
+    if (active) {
+        u32x4 r = draw(seed, (uint32_t)i, (uint32_t)y, step, tag);
+        u = draw_unit(r.y);
+        o = (size_t)y * Ns + i;
+        qyx = qA[o];
+        float dE;
+        if (sa) {
+            dE = bip_sa_dE(qyx, h[i], F[o]);
+        } else {
+            int yl = y == 0 ? m - 1 : y - 1, yr = y == m - 1 ? 0 : y + 1;
+            qL = qA[(size_t)yl * Ns + i];
+            qR = qA[(size_t)yr * Ns + i];
+            dE = bip_sqa_dE(qyx, h[i], F[o], qL, qR, sc.twoDivM, sc.coef);
+        }
+        L = neg_log_unit(u);
+        acc = metropolis_log(dE, sc.rate, L, trial_xtol(tol, h[i], F[o], L), nearT);
+    }
+    auto decide = [&](double Fx) {
+        const double hx = bip_exact_h(B, h, i);
+        acc = exact_accept_log(sa, false, qyx, hx, Fx, (int)qL + (int)qR, sc, tol, L);
+        if (acc < 0) acc = exact_accept(sa, false, qyx, hx, Fx, qL, qR, m, B.G, B.beta, u);
+    };
+    if (kWarp) {
+        for (unsigned flagged = __ballot_sync(0xffffffffu, nearT); flagged; flagged &= flagged - 1u) {
+            const int l = __ffs(flagged) - 1;
+            const double Fx = bip_exact_field_warp(B, __shfl_sync(0xffffffffu, y, l), __shfl_sync(0xffffffffu, i, l));
+            if ((threadIdx.x & 31) == l) decide(Fx);
+            __syncwarp();
+        }
+    } else if (nearT) {
+        decide(bip_exact_field(B, y, i));
+    }
     if (!acc) return 0;
     qA[o] = (int8_t)(-qyx);
     if (trace) {
@@ -90,15 +128,12 @@ __global__ void __launch_bounds__(256) bip_flip_phase(int8_t *qA, const float *F
                                                       unsigned long long *accepted, BipFixed B) {
     long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     bool active = idx < (long long)cnt * Ns;
-    int acc = 0;
-    if (active) {
-        const float G = Gp ? *Gp : Gsc, beta = bp ? *bp : bsc;
-        StepConst sc = step_const(algo, m, G, beta);
-        int t = (int)(idx / Ns), i = (int)(idx - (long long)t * Ns);
-        B.G = G;
-        B.beta = beta;
-        acc = bip_trial(qA, F, h, Ns, m, yb + t * ys, i, seed, step, tag, sc, algo, trace, bitBase, B);
-    }
+    const float G = Gp ? *Gp : Gsc, beta = bp ? *bp : bsc;
+    const StepConst sc = step_const(algo, m, G, beta);
+    const int t = (int)(idx / Ns), i = (int)(idx - (long long)t * Ns);
+    B.G = G;
+    B.beta = beta;
+    const int acc = bip_trial<true>(active, qA, F, h, Ns, m, yb + t * ys, i, seed, step, tag, sc, algo, trace, bitBase, B);
     if (accepted) {
         unsigned ballot = __ballot_sync(0xffffffffu, acc);
         if ((threadIdx.x & 31) == 0 && ballot) atomicAdd(accepted, (unsigned long long)__popc(ballot));
@@ -130,13 +165,13 @@ __global__ void __launch_bounds__(256) bip_flip_half(int8_t *qA, const float *F,
     unsigned long long acc = 0;
     for (int ph = 0; ph < 3; ++ph) {
         if (ph == 1 && !(m & 1)) continue;
-        if (col) {
-            if (ph == 1) {
-                if (p0 == 0) acc += bip_trial(qA, F, h, Ns, m, m - 1, i, seed, step, tag, sc, algo, trace, bitBase, B);
-            } else {
-                for (int p = p0; p < pairs; p += pStride)
-                    acc += bip_trial(qA, F, h, Ns, m, 2 * p + (ph == 2 ? 1 : 0), i, seed, step, tag, sc, algo, trace,
-                                     bitBase, B);
+        if (ph == 1) {
+            acc += bip_trial<true>(col && p0 == 0, qA, F, h, Ns, m, m - 1, i, seed, step, tag, sc, algo, trace, bitBase, B);
+        } else {
+            for (int pb = 0; pb < pairs; pb += pStride) {  // the same trips for every thread
+                const int p = pb + p0;
+                acc += bip_trial<true>(col && p < pairs, qA, F, h, Ns, m, 2 * p + (ph == 2 ? 1 : 0), i, seed, step, tag, sc,
+                                 algo, trace, bitBase, B);
             }
         }
         __syncthreads();
@@ -307,8 +342,8 @@ __global__ void __launch_bounds__(256) bip_batch_persistent(const sq103_bipartit
                     }
                     for (long long k = threadIdx.x; k < (long long)cnt * Ns; k += blockDim.x) {
                         int t = (int)(k / Ns), i = (int)(k - (long long)t * Ns);
-                        accepted += bip_trial(qA, F, h, Ns, m, yb + t * ys, i, T.seed, step, tag, sc, T.algo, nullptr, 0,
-                                              B);
+                        accepted += bip_trial<false>(true, qA, F, h, Ns, m, yb + t * ys, i, T.seed, step, tag, sc,
+                                                     T.algo, nullptr, 0, B);
                     }
                     __syncthreads();
                 }

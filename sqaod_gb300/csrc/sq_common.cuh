@@ -240,22 +240,29 @@ static __device__ SQ103_EXACT_ATTR double exact_field_thread(const R *Jx, size_t
     return exact_value(s, S);
 }
 
-// warp-wide: every lane of the (converged) warp calls it and gets the sum
+// warp-wide: every lane of the (converged) warp calls it and gets the sum; the
+// couplings are Jx[j * stride], as in exact_field_thread
 template <class R>
-static __device__ SQ103_EXACT_ATTR double exact_field_warp(const R *Jx, const int8_t *q, int N) {
+static __device__ SQ103_EXACT_ATTR double exact_field_warp_strided(const R *Jx, size_t stride, const int8_t *q, int N) {
     const int lane = threadIdx.x & 31;
     unsigned e = 0;
-    for (int j = lane; j < N; j += 32) e = max(e, ExactFx<R>::expo(Jx[j]));
+#pragma unroll 8
+    for (int j = lane; j < N; j += 32) e = max(e, ExactFx<R>::expo(__ldg(Jx + j * stride)));
     e = __reduce_max_sync(0xffffffffu, e);
     const int S = ExactFx<R>::shift(e, log2_ceil(N));
     long long s = 0;
+#pragma unroll 8
     for (int j = lane; j < N; j += 32) {
-        const long long v = ExactFx<R>::term(Jx[j], S);
+        const long long v = ExactFx<R>::term(__ldg(Jx + j * stride), S);
         s += q[j] > 0 ? v : -v;
     }
 #pragma unroll
     for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     return exact_value(s, S);
+}
+template <class R>
+static __device__ SQ103_EXACT_ATTR double exact_field_warp(const R *Jx, const int8_t *q, int N) {
+    return exact_field_warp_strided<R>(Jx, 1, q, N);
 }
 
 // fp32 rows on a 16-byte boundary are read as float4 with eight loads in flight
@@ -330,6 +337,24 @@ static __device__ SQ103_EXACT_ATTR int exact_accept(bool sa, bool twoF, float q,
                                                 int m, float G, float beta, float u) {
     const double coef = sa ? 0.0 : exact_ring_coef(G, beta, m);
     return exact_accept_coef(sa, twoF, q, h, F, (int)qL + (int)qR, m, G, beta, coef, u);
+}
+
+// The same decision without FP64 functions where that is possible: with the
+// exact field the only errors left in x = rate dE and L are those of the fp32
+// step constants and of L, which kC + 2.4e-7 L of the trial's tolerance bounds.
+// Returns 0 or 1 outside that bound, -1 inside it (about one flagged trial in a
+// hundred; exact_accept then decides).  FP64 runs at 1/64 of the fp32 rate, and
+// log, tanh and exp in it take about 8 us of a lone warp's time; this takes six
+// FP64 operations.
+__device__ __forceinline__ int exact_accept_log(bool sa, bool twoF, float q, double h, double F, int sum,
+                                                const StepConst &sc, const DecisionTol &tol, float L) {
+    const double t = __dadd_rn(h, twoF ? __dadd_rn(F, F) : F);
+    const double a = __dmul_rn((double)(sa ? 2.f * q : sc.twoDivM * q), t);
+    const double b = __dmul_rn((double)(q * (float)sum), (double)sc.coef);  // coef = 0 for SA
+    const double d = __dsub_rn(__dmul_rn(__dsub_rn(a, b), (double)sc.rate), (double)L);
+    const float bound = __fadd_rn(tol.kC, __fmul_rn(2.4e-7f, fminf(L, 1e30f)));
+    if (fabs(d) <= (double)bound) return -1;
+    return d < 0.0 ? 1 : 0;
 }
 #endif
 
