@@ -51,7 +51,6 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
-#include <array>
 #include <mutex>
 
 // the exact warp's helpers inlined: measured 1.8 % faster at N=4096 m=256
@@ -231,8 +230,14 @@ struct McPack {
 // p - 2 drawn again from the neighbours' Philox streams, instead of a ballot per
 // hit over the hashed-site bitmaps of the other prefetcher's batches (which
 // makes the prefetchers wait for each other).  Both give the same candidates.
-template <bool kHooks, bool kSmall>
-__global__ void __launch_bounds__(kMcThreads, 2) dense_sweep_multi(const McPack P) {
+// kPerSm: the CTAs per SM the registers are allotted for.  The trotters of a launch
+// are all resident, so the limit on m is kPerSm * 152 (where shared memory allows
+// as many: N <= 3100 for four).  Two leave 118 registers a thread and the fastest
+// decider; four have 64 (8 bytes spilled) and take the launches that exceed two.
+// N = 2000, m = 500, 8 steps: 7.4 ms with four per SM; one CTA for the whole
+// instance, which such sizes fell back to before, 1090 ms.
+template <bool kHooks, bool kSmall, int kPerSm>
+__global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const McPack P) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ McShared S;
     __shared__ sq103_dense_task task;
@@ -1004,39 +1009,51 @@ static size_t multi_smem_bytes(int N) {
            32 * 8 + (size_t)((N + 15) & ~15) + 16 + (N <= kSmallN ? (size_t)kPf * kSmallN * 4 : 0);
 }
 
-static std::array<const void *, 4> multi_kernels() {
-    return {(const void *)dense_sweep_multi<false, false>, (const void *)dense_sweep_multi<true, false>,
-            (const void *)dense_sweep_multi<false, true>, (const void *)dense_sweep_multi<true, true>};
+// every instance, by kHooks, kSmall (bits 0, 1) and register allotment (2 or 4 CTAs per SM)
+static const void *multi_kernel(bool hooks, bool small, int perSm) {
+    static const void *const k[2][4] = {
+        {(const void *)dense_sweep_multi<false, false, 2>, (const void *)dense_sweep_multi<true, false, 2>,
+         (const void *)dense_sweep_multi<false, true, 2>, (const void *)dense_sweep_multi<true, true, 2>},
+        {(const void *)dense_sweep_multi<false, false, 4>, (const void *)dense_sweep_multi<true, false, 4>,
+         (const void *)dense_sweep_multi<false, true, 4>, (const void *)dense_sweep_multi<true, true, 4>}};
+    return k[perSm > 2][(hooks ? 1 : 0) + (small ? 2 : 0)];
 }
 
-static int multi_capacity(int N) {
+// resident CTAs of rows of N spins, with the registers allotted for two and for four per SM
+struct MultiCapacity {
+    int two, four;
+};
+
+static MultiCapacity multi_capacity(int N) {
     // the last answer is cached; callers on several host threads share it
     static std::mutex mu;
-    static int cachedN = -1, cachedCap = 0;
+    static int cachedN = -1;
+    static MultiCapacity cached = {0, 0};
     std::lock_guard<std::mutex> lock(mu);
-    if (N == cachedN) return cachedCap;
-    int dev = 0, sms = 0, perSm = 0, optin = 0;
+    if (N == cachedN) return cached;
+    int dev = 0, sms = 0, optin = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    size_t smem = multi_smem_bytes(N);
+    const size_t smem = multi_smem_bytes(N);
     cudaFuncAttributes fa;
-    cudaFuncGetAttributes(&fa, dense_sweep_multi<false, false>);
-    if (smem + fa.sharedSizeBytes > (size_t)optin) return 0;
+    cudaFuncGetAttributes(&fa, multi_kernel(false, false, 2));
+    if (smem + fa.sharedSizeBytes > (size_t)optin) return {0, 0};
     // every instance: the launch takes the one the tasks' flags and sizes ask for
-    perSm = 1 << 30;
-    for (const void *k : multi_kernels()) {
+    int perSm[2] = {1 << 30, 1 << 30};
+    for (int i = 0; i < 8; ++i) {
+        const void *k = multi_kernel(i & 1, i & 2, i & 4 ? 4 : 2);
         int ps = 0;
         if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ps, k, kMcThreads, smem) != cudaSuccess) {
             cudaGetLastError();
-            return 0;
+            return {0, 0};
         }
-        perSm = std::min(perSm, ps);
+        perSm[i >> 2] = std::min(perSm[i >> 2], ps);
     }
     cachedN = N;
-    cachedCap = perSm * sms;
-    return cachedCap;
+    cached = {perSm[0] * sms, std::max(perSm[0], perSm[1]) * sms};
+    return cached;
 }
 
 }  // namespace sq103
@@ -1053,7 +1070,7 @@ SQ103_API unsigned long long sq103_dense_ws_bytes(int N, int m, int nSteps) {
 SQ103_API int sq103_dense_multicta_ok(int N, int m, int algo) {
     if (algo != kColoring && algo != kSANaive) return 0;
     if (N < 64 || m < 2) return 0;
-    return m <= multi_capacity(N) ? 1 : 0;
+    return m <= multi_capacity(N).four ? 1 : 0;
 }
 
 // n instances in one cooperative launch (see McPack)
@@ -1083,18 +1100,15 @@ static int launch_pack(const sq103_dense_task *tasks, int n, void *stream) {
     }
     for (int i = n; i <= kMaxPack; ++i) P.base[i] = ctas;
     // every CTA resident at once (cooperative launch); also sets the kernel's shared-memory limit
-    if (multi_capacity(maxN) < ctas) return kErrCapacity;
+    const MultiCapacity cap = multi_capacity(maxN);
+    if (cap.four < ctas) return kErrCapacity;
     for (int i = 0; i < n; ++i) {
         // the accept words carry their batch tag; zero means "not published"
         cudaError_t e = cudaMemsetAsync(P.outLog[i], 0, (size_t)tasks[i].m * P.nWords[i] * 8, st);
         if (e != cudaSuccess) return (int)e;
     }
     void *args[] = {&P};
-    const bool small = maxN <= kSmallN;
-    const void *kernel = small ? (hooks ? (const void *)dense_sweep_multi<true, true>
-                                        : (const void *)dense_sweep_multi<false, true>)
-                               : (hooks ? (const void *)dense_sweep_multi<true, false>
-                                        : (const void *)dense_sweep_multi<false, false>);
+    const void *kernel = multi_kernel(hooks, maxN <= kSmallN, ctas <= cap.two ? 2 : 4);
     return (int)cudaLaunchCooperativeKernel(kernel, dim3(ctas), dim3(kMcThreads), args, multi_smem_bytes(maxN), st);
 }
 
@@ -1106,6 +1120,7 @@ SQ103_API int sq103_dense_anneal_pack(const sq103_dense_task *tasks, int n, void
     return launch_pack(tasks, n, stream);
 }
 
-SQ103_API int sq103_dense_multicta_capacity(int N) { return N >= 64 ? multi_capacity(N) : 0; }
+// trotters of one packed launch that keep two CTAs per SM
+SQ103_API int sq103_dense_multicta_capacity(int N) { return N >= 64 ? multi_capacity(N).two : 0; }
 
 }  // extern "C"

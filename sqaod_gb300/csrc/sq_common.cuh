@@ -240,8 +240,25 @@ static __device__ SQ103_EXACT_ATTR double exact_field_thread(const R *Jx, size_t
     return exact_value(s, S);
 }
 
-// warp-wide: every lane of the (converged) warp calls it and gets the sum; the
-// couplings are Jx[j * stride], as in exact_field_thread
+// warp-wide: every lane of the (converged) warp calls it and gets the sum
+template <class R>
+static __device__ SQ103_EXACT_ATTR double exact_field_warp(const R *Jx, const int8_t *q, int N) {
+    const int lane = threadIdx.x & 31;
+    unsigned e = 0;
+    for (int j = lane; j < N; j += 32) e = max(e, ExactFx<R>::expo(Jx[j]));
+    e = __reduce_max_sync(0xffffffffu, e);
+    const int S = ExactFx<R>::shift(e, log2_ceil(N));
+    long long s = 0;
+    for (int j = lane; j < N; j += 32) {
+        const long long v = ExactFx<R>::term(Jx[j], S);
+        s += q[j] > 0 ? v : -v;
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return exact_value(s, S);
+}
+
+// the same over couplings Jx[j * stride] (a column of J), eight loads in flight per lane
 template <class R>
 static __device__ SQ103_EXACT_ATTR double exact_field_warp_strided(const R *Jx, size_t stride, const int8_t *q, int N) {
     const int lane = threadIdx.x & 31;
@@ -259,10 +276,6 @@ static __device__ SQ103_EXACT_ATTR double exact_field_warp_strided(const R *Jx, 
 #pragma unroll
     for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     return exact_value(s, S);
-}
-template <class R>
-static __device__ SQ103_EXACT_ATTR double exact_field_warp(const R *Jx, const int8_t *q, int N) {
-    return exact_field_warp_strided<R>(Jx, 1, q, N);
 }
 
 // fp32 rows on a 16-byte boundary are read as float4 with eight loads in flight
