@@ -101,7 +101,7 @@ SQ103_API unsigned long long sq103_dense_ws_bytes(int N, int m, int nSteps);
 /* 1 if the one-CTA-per-trotter sweep can run this shape on the current device (N >= 64, m >= 2;
  * the launch also needs ldJ % 4 == 0 and a 16-byte aligned J) */
 SQ103_API int sq103_dense_multicta_ok(int N, int m, int algo);
-/* No counterpart in the reference.  Up to 16 independent instances in one
+/* No counterpart in the reference.  Up to 64 independent instances in one
  * cooperative launch of the one-CTA-per-trotter sweep (their trotter counts
  * summed within sq103_dense_multicta_capacity of the largest N); each task
  * needs its own ws.  Every instance ends exactly as when launched alone. */

@@ -58,8 +58,9 @@ class DenseBatchAnnealer:
 
     def set_multicta_min_n(self, N):
         """Instances of at least N spins run on the one-CTA-per-trotter sweep
-        (packed launches); 0 keeps all on the persistent kernel.  Default 1024;
-        results do not depend on it.  Takes effect at the next prepare()."""
+        (packed launches); 0 keeps all on the persistent kernel.  Default 1024,
+        with smaller ones taken along where that is faster; results do not
+        depend on it.  Takes effect at the next prepare()."""
         self._call("set_multicta_min_n", ctypes.c_int(N))
 
     def multicta_count(self):

@@ -208,11 +208,12 @@ __device__ __forceinline__ void window_bits(int x, int Ji, int j0, int pLast, in
     }
 }
 
-// Up to kMaxPack independent instances in one cooperative launch: CTAs
+// Up to kMaxPack independent instances in one cooperative launch (small ones of few
+// trotters fill it only in numbers: 64 of m = 8 take 512 CTAs): CTAs
 // [base[i], base[i+1]) are the trotters of task t[i], whose accept words live in
 // outLog[i] (nWords[i] per trotter).  Instances do not interact (the prologue's
 // grid sync is the only common step), so each runs exactly as alone.
-constexpr int kMaxPack = 16;
+constexpr int kMaxPack = 64;  // 12 KB of launch parameters, indexed in place
 struct McPack {
     sq103_dense_task t[kMaxPack];
     unsigned long long *outLog[kMaxPack];
@@ -237,35 +238,27 @@ struct McPack {
 // N = 2000, m = 500, 8 steps: 7.4 ms with four per SM; one CTA for the whole
 // instance, which such sizes fell back to before, 1090 ms.
 template <bool kHooks, bool kSmall, int kPerSm>
-__global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const McPack P) {
+__global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const __grid_constant__ McPack P) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ McShared S;
     __shared__ sq103_dense_task task;
     __shared__ unsigned long long *sLog;
     __shared__ int sWords, sBase;
     if (threadIdx.x == 0) {
-        int ti = 0;
-#pragma unroll
-        for (int i = 1; i < kMaxPack; ++i)
-            if (i < P.n && (int)blockIdx.x >= P.base[i]) ti = i;
-        // constant indices only (a runtime index into the parameters would copy them all)
-        switch (ti) {
-#define SQ103_PICK(i)            \
-    case i:                      \
-        task = P.t[i];           \
-        sLog = P.outLog[i];      \
-        sWords = P.nWords[i];    \
-        sBase = P.base[i];       \
-        break;
-            SQ103_PICK(0) SQ103_PICK(1) SQ103_PICK(2) SQ103_PICK(3)
-            SQ103_PICK(4) SQ103_PICK(5) SQ103_PICK(6) SQ103_PICK(7)
-            SQ103_PICK(8) SQ103_PICK(9) SQ103_PICK(10) SQ103_PICK(11)
-            SQ103_PICK(12) SQ103_PICK(13) SQ103_PICK(14) SQ103_PICK(15)
-#undef SQ103_PICK
+        int lo = 0, hi = P.n - 1;  // the instance whose CTAs [base[i], base[i + 1]) hold this one
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if ((int)blockIdx.x >= P.base[mid])
+                lo = mid;
+            else
+                hi = mid - 1;
         }
+        task = P.t[lo];
+        sLog = P.outLog[lo];
+        sWords = P.nWords[lo];
+        sBase = P.base[lo];
     }
     __syncthreads();
-    static_assert(kMaxPack == 16, "one case per pack entry");
     const sq103_dense_task &T = task;
     unsigned long long *const outLog = sLog;
     const int nWords = sWords;
@@ -329,8 +322,11 @@ __global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const Mc
         S.done = 0;
         S.nflip = 0;
     }
-    // every CTA has read its neighbours' rows before any CTA can finish and
-    // write its own row back
+    // the accept words carry their batch's tag; zero means "not published"
+#pragma unroll 1
+    for (int w = tid; w < nWords; w += kMcThreads) outLog[(size_t)y * nWords + w] = 0ull;
+    // every CTA has cleared its accept words before any CTA publishes or polls one,
+    // and read its neighbours' rows before any CTA can finish and write its own back
     cooperative_groups::this_grid().sync();
 
     if (warp == 0) {
@@ -1102,11 +1098,6 @@ static int launch_pack(const sq103_dense_task *tasks, int n, void *stream) {
     // every CTA resident at once (cooperative launch); also sets the kernel's shared-memory limit
     const MultiCapacity cap = multi_capacity(maxN);
     if (cap.four < ctas) return kErrCapacity;
-    for (int i = 0; i < n; ++i) {
-        // the accept words carry their batch tag; zero means "not published"
-        cudaError_t e = cudaMemsetAsync(P.outLog[i], 0, (size_t)tasks[i].m * P.nWords[i] * 8, st);
-        if (e != cudaSuccess) return (int)e;
-    }
     void *args[] = {&P};
     const void *kernel = multi_kernel(hooks, maxN <= kSmallN, ctas <= cap.two ? 2 : 4);
     return (int)cudaLaunchCooperativeKernel(kernel, dim3(ctas), dim3(kMcThreads), args, multi_smem_bytes(maxN), st);
@@ -1120,7 +1111,6 @@ SQ103_API int sq103_dense_anneal_pack(const sq103_dense_task *tasks, int n, void
     return launch_pack(tasks, n, stream);
 }
 
-// trotters of one packed launch that keep two CTAs per SM
-SQ103_API int sq103_dense_multicta_capacity(int N) { return N >= 64 ? multi_capacity(N).two : 0; }
+SQ103_API int sq103_dense_multicta_capacity(int N) { return N >= 64 ? multi_capacity(N).four : 0; }
 
 }  // extern "C"

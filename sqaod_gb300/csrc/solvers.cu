@@ -1860,14 +1860,13 @@ private:
 class DenseBatch : public sq::NullBase {
 public:
     static constexpr int kRefreshPeriod = 8;
-    static constexpr int kPackMax = 8;           // instances per packed launch (16 measured slower on C4)
+    static constexpr int kPackMax = 64;          // instances per packed launch
     static constexpr int kDefaultMultiMinN = 1024;
 
-    // Instances of at least multiMinN_ spins (with m >= 2 that fit the device) run
-    // on the one-CTA-per-trotter sweep in packed cooperative launches: its decider
-    // takes 32 iterations per round trip, where the persistent one-CTA kernel
-    // takes one per colour phase, and the serial chain of the largest instances
-    // sets the batch's step time.  Both kernels give bit-identical results.
+    // Instances of at least a size limit (prepare(); with m >= 2 that fit the device)
+    // run on the one-CTA-per-trotter sweep in packed cooperative launches: its
+    // decider takes 32 iterations per round trip, where the persistent one-CTA
+    // kernel takes one per colour phase.  Both kernels give bit-identical results.
     struct Inst {
         int N, m, ldJ;  // J rows on a 16-byte stride (the one-CTA-per-trotter sweep reads them as float4)
         bool multi = false;
@@ -1945,11 +1944,22 @@ public:
         std::vector<sq103_dense_task> tasks;
         std::vector<Inst *> smallInsts;
         multi_.clear();
+        // Without a limit of the caller's, the packed launches also take the smaller
+        // instances: the persistent kernel's step lasts as long as its longest chain
+        // (two phases of about 4 us per iteration), a packed launch takes 32 iterations
+        // in about 3 us.  Measured, 16 steps of n instances of 64 to 2048 spins, ms by
+        // size limit:    n      1024   512   256   128    64
+        //               16      72.3  31.7   9.9   6.1   4.1
+        //              128       133  43.7  35.6  26.0  25.1
+        //              300       164  89.1  65.3  57.8  59.7
+        //             1024       246   184   178   185   191
+        // so 64 (the kernel's least) for few instances and 128 for many.
+        const int minN = limitGiven_ ? multiMinN_ : nAll <= 152 ? 64 : 128;
         int maxN = 0, maxM = 0;
         for (int i = 0; i < nAll; ++i) {
             Inst &in = *insts_[i];
             SQ_CHECK(sq103_randomize_spins(in.q, in.N, in.m, in.seed, 0, 0, st_.get()));
-            in.multi = multiMinN_ > 0 && in.N >= multiMinN_ && in.m >= 2 && sq103_dense_multicta_ok(in.N, in.m, kColoring);
+            in.multi = minN > 0 && in.N >= minN && in.m >= 2 && sq103_dense_multicta_ok(in.N, in.m, kColoring);
             if (in.multi) {
                 in.wsBytes = sq103_dense_ws_bytes(in.N, in.m, kRefreshPeriod);
                 in.ws.ensure(in.wsBytes);
@@ -2051,6 +2061,7 @@ public:
         for (int i = 0; i < nCands; ++i) {
             throwErrorIf(cands[i] < 0, "size limits must not be negative.");
             multiMinN_ = cands[i];
+            limitGiven_ = true;
             prepare();
             SQ_CHECK(cudaEventRecord(e0, st_.get()));
             anneal(steps, true);
@@ -2151,9 +2162,16 @@ public:
     void setMultiMinN(int N) {
         throwErrorIf(N < 0, "the size limit must not be negative.");
         multiMinN_ = N;
+        limitGiven_ = true;
         prepared_ = false;
     }
-    int multiCount() const { return (int)multi_.size(); }
+    // the instances of at least the size limit (the smaller ones that the packed
+    // launches take along without a limit of the caller's are not counted)
+    int multiCount() const {
+        int n = 0;
+        for (const Inst *in : multi_) n += in->N >= multiMinN_;
+        return n;
+    }
     int size() const { return (int)insts_.size(); }
     int position() const { return pos_; }
     int grid() const { return grid_; }
@@ -2308,6 +2326,7 @@ private:
     std::vector<Inst *> multi_;  // the instances on the one-CTA-per-trotter sweep, by N
     cudaGraphExec_t graph_ = nullptr;
     int nSched_ = 0, pos_ = 0, grid_ = 1, smem_ = -1, nSmall_ = 0, multiMinN_ = kDefaultMultiMinN;
+    bool limitGiven_ = false;
     bool prepared_ = false;
 };
 

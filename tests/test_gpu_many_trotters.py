@@ -19,9 +19,11 @@ def _sym(rng, N):
 def test_many_trotters_replay(orc, N, m, algo):
     import sqaod_gb300 as sq
     from sqaod_gb300 import _lib
+    import torch
     code = {"coloring": orc.ALGO_COLORING, "sa_naive": orc.ALGO_SA_NAIVE}[algo]
     assert _lib.lib().sq103_dense_multicta_ok(N, m, code) == 1
-    assert m > _lib.lib().sq103_dense_multicta_capacity(N)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert 2 * sms < m <= _lib.lib().sq103_dense_multicta_capacity(N)
     rng = np.random.default_rng(N + m)
     a = sq.cuda.dense_graph_annealer(_sym(rng, N), n_trotters=m, algorithm=algo)
     h, J, c = a.get_hamiltonian()
