@@ -120,7 +120,8 @@ public:
         size_t bytes = 0;
         int pos = 0;     // steps done
         int slot = -1;   // batch slot, -1 for the per-instance kernel
-        bool large = false;
+        bool large = false;  // outside the persistent kernels: packed launches (dense), a side stream (bipartite)
+        bool heavy = false;  // large by its size alone (counts against the large-request limit)
         sq103_dense_task dt = {};
         sq103_bipartite_task bt = {};
         double *c64 = nullptr;
@@ -222,14 +223,29 @@ public:
         const int nDone = finalizeReady(false);
         admit();
         const int nD = (int)denseSlots_.size(), nB = (int)bipSlots_.size();
+        // bipartite requests outside the persistent kernel: each one's launches in order
+        // on one of the side streams, the requests side by side (each fills only part of
+        // the GPU) and beside the work below
+        int nBig = 0;
+        for (Request *r : large_) {
+            if (r->kind != 1) continue;
+            if (nBig == 0) fork();
+            sq103_bipartite_task t = r->bt;
+            t.G = r->bt.G + r->pos;
+            t.beta = r->bt.beta + r->pos;
+            t.step0 = 1 + (uint32_t)r->pos;
+            t.nSteps = std::min(kStepsPerTick, r->nSteps - r->pos);
+            SQ_CHECK(sq103_bipartite_anneal(&t, side_[nBig % kRefreshStreams].get()));
+            ++nBig;
+        }
         if (nD > 0)
             SQ_CHECK(sq103_dense_batch_launch(dTasks_.p, nD, counts_.p, nullptr, dPos_.p, queues_.p, kStepsPerTick,
                                               std::min(denseGrid_, nD), stageSmem_, st_.get()));
         if (nB > 0)
             SQ_CHECK(sq103_bipartite_batch_launch(bTasks_.p, nB, counts_.p + 1, nullptr, bPos_.p, queues_.p + 2,
                                                   kStepsPerTick, std::min(bipGrid_, nB), st_.get()));
-        // large dense instances: packed cooperative launches (instances of similar
-        // size together, as many trotters as can be resident); large bipartite: one by one
+        // dense instances outside the persistent kernel: packed cooperative launches
+        // (instances of similar size together, as many trotters as can be resident)
         std::vector<Request *> big;
         for (Request *r : large_)
             if (r->kind == 0) big.push_back(r);
@@ -254,20 +270,6 @@ public:
             packN = std::max(packN, r->N0);
         }
         flush();
-        // large bipartite requests: each one's launches in order on one of the side
-        // streams, the requests side by side (each fills only part of the GPU)
-        int nBig = 0;
-        for (Request *r : large_) {
-            if (r->kind != 1) continue;
-            if (nBig == 0) fork();
-            sq103_bipartite_task t = r->bt;
-            t.G = r->bt.G + r->pos;
-            t.beta = r->bt.beta + r->pos;
-            t.step0 = 1 + (uint32_t)r->pos;
-            t.nSteps = std::min(kStepsPerTick, r->nSteps - r->pos);
-            SQ_CHECK(sq103_bipartite_anneal(&t, side_[nBig % kRefreshStreams].get()));
-            ++nBig;
-        }
         if (nBig > 0) join();
         std::vector<Request *> finished;
         jobs_.clear();
@@ -451,6 +453,22 @@ private:
         return base + (size_t)r.m * r.N0 * 5 + (size_t)r.N0 * 4 <= (size_t)stageSmem_;
     }
 
+    // A request the persistent kernels could hold takes a large one's route while few
+    // are there: one CTA runs a request's whole tick in the persistent kernels (8 steps
+    // of N = 1000, m = 16: 9.9 ms; of a 400 x 300, m = 256 bipartite one: 6.6 ms), and
+    // a tick lasts as long as its longest request.  The packed launch takes 8 steps of
+    // N = 1000 in 0.8 ms, and the per-instance bipartite kernels about 0.3 ms, but each
+    // bipartite request so costs 32 launches a tick, which the limits below keep in
+    // proportion.  Mixed set of 24 requests, 32 steps: 84.8 ms with the persistent
+    // kernels, 20.1 ms this way.
+    bool light_(const Request &r) const {
+        if (r.kind == 1) return nLight_[1] < kMaxLightBip;
+        if (r.kind != 0 || !sq103_dense_multicta_ok(r.N0, r.m, kColoring)) return false;
+        // (dense: with the accept-word workspace inside the budget)
+        return nLight_[0] < (r.N0 >= 128 ? kMaxLightDense : kMaxLightSmall) &&
+               used_ + r.bytes + al(sq103_dense_ws_bytes(r.N0, r.m, kStepsPerTick)) <= budget_;
+    }
+
     // Admits queued requests in arrival order as memory, slots and the large-instance
     // limit allow; a request that cannot start yet keeps its place and does not
     // block the ones behind it.
@@ -461,21 +479,26 @@ private:
             Request *r = queue_[i];
             // bipartite requests whose fields the single-instance annealer computes on the
             // tensor cores take the per-instance kernels, which do the same
-            const bool large = r->kind == kSearch ? false
+            const bool heavy = r->kind == kSearch ? false
                                : r->kind == 0 ? !fitsStaging(*r) && sq103_dense_multicta_ok(r->N0, r->m, kColoring)
                                               : (size_t)r->m * r->N0 * r->N1 > kBipLargeWork ||
                                                     sq103_bipartite_refresh_uses_tc(r->N0, r->N1, r->m);
+            const bool light = !heavy && light_(*r);
             const bool fits =
                 used_ + r->bytes <= budget_ &&
                 (r->kind == kSearch ? (int)searches_.size() < kMaxSearches
-                 : large            ? (int)large_.size() < maxLarge_  // each steps with the whole GPU every tick
+                 : heavy            ? nHeavy_ < maxLarge_  // each steps with the whole GPU every tick
+                 : light            ? true
                                     : (int)(r->kind == 0 ? denseSlots_.size() : bipSlots_.size()) < maxSlots_);
             if (!fits) {
                 ++i;
                 continue;
             }
             queue_.erase(queue_.begin() + i);
-            r->large = large;
+            r->large = heavy || light;
+            r->heavy = heavy;
+            if (heavy) ++nHeavy_;
+            if (light) ++nLight_[r->kind];
             setup(r);
             used_ += r->bytes;
             r->state = kActive;
@@ -647,7 +670,10 @@ private:
         // free the slot now (the kernels skip finished instances anyway): the last slot moves into it
         if (r->kind == 0 && !r->large) removeSlot(denseSlots_, r, dTasks_.p, dPos_.p, 0);
         if (r->kind == 1 && !r->large) removeSlot(bipSlots_, r, bTasks_.p, bPos_.p, 1);
-        if (r->large) large_.erase(std::find(large_.begin(), large_.end(), r));
+        if (r->large) {
+            large_.erase(std::find(large_.begin(), large_.end(), r));
+            --(r->heavy ? nHeavy_ : nLight_[r->kind]);
+        }
         finishing_.push_back(r);
     }
 
@@ -761,7 +787,10 @@ private:
     DevBuf<sq103_bipartite_task> bTasks_;
     DevBuf<int> dPos_, bPos_, counts_, queues_;
     DevBuf<float> dW_;
-    static constexpr int kMaxPack = 16;  // instances per packed launch (sq103_dense_anneal_pack)
+    static constexpr int kMaxPack = 64;  // instances per packed launch (sq103_dense_anneal_pack)
+    // light requests on the large ones' routes at a time: dense of N >= 128, dense below, bipartite
+    static constexpr int kMaxLightDense = 512, kMaxLightSmall = 64, kMaxLightBip = 32;
+    int nHeavy_ = 0, nLight_[2] = {0, 0};
 };
 
 }  // namespace sq103
