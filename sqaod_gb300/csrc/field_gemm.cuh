@@ -1,16 +1,12 @@
-// field_gemm.cuh -- dense local fields and energy row sums without FP64 arithmetic.
+// field_gemm.cuh -- dense local fields without FP64 arithmetic.
 //
-// Both compute C[y][n] = sum_k A[y][k] B[k][n] with A in {-1, +1} (int8 spins,
-// M x K) and B fp32 (K x N, row stride ldb): every product is an exact fp32
-// value (+-B or 0 past the edge), so only the summation rounds.  GB300 runs
-// FP64 at 1/64 of the fp32 rate, so both kernels sum in fp32 with error-free
-// transformations instead:
-//   fields (fp32 out): fp32 partial sums over 32-wide k chunks (sequential,
-//     k ascending), the chunk sums added with TwoSum into a (sum, compensation)
-//     pair; the result is sum + compensation.  About 1e-7 of the row scale.
-//   energies (FP64 out): every product added with TwoSum into a (sum,
-//     compensation) pair -- a double-float accumulator, about 2^-44 relative --
-//     returned as sum + compensation in FP64.
+// C[y][n] = sum_k A[y][k] B[k][n] with A in {-1, +1} (int8 spins, M x K) and B
+// fp32 (K x N, row stride ldb): every product is an exact fp32 value (+-B or 0
+// past the edge), so only the summation rounds.  GB300 runs FP64 at 1/64 of the
+// fp32 rate, so the sums are fp32 with error-free transformations: partial sums
+// over 32-wide k chunks (sequential, k ascending), the chunk sums added with
+// TwoSum into a (sum, compensation) pair; the result is sum + compensation,
+// about 1e-7 of the row scale.  (The energies use the tiles of bip_field.cuh.)
 // Tiles of 64 x 64 outputs per CTA of 256 threads (4 x 4 per thread), k in
 // chunks of 32 staged in shared memory with the next chunk's loads in flight.
 // The order of every addition is fixed, so results do not depend on the launch.
@@ -29,10 +25,8 @@ __device__ __forceinline__ void two_sum_acc(float &s, float &c, float x) {
 }
 
 // The 64 x 64 output tile at rows y0.., columns n0.. of C = A B, by a CTA of 256
-// threads.  EXACT = false: fp32 fields; true: double-float energy row sums (OutT
-// double).
-template <bool EXACT, typename OutT>
-__device__ __forceinline__ void field_gemm_tile(const int8_t *A, int lda, const float *B, int ldb, OutT *C, int ldc,
+// threads.
+__device__ __forceinline__ void field_gemm_tile(const int8_t *A, int lda, const float *B, int ldb, float *C, int ldc,
                                                 int M, int Nn, int K, int y0, int n0) {
     __shared__ __align__(16) float As[2][32][68];  // rows padded against store conflicts
     __shared__ __align__(16) float Bs[2][32][68];
@@ -120,19 +114,12 @@ __device__ __forceinline__ void field_gemm_tile(const int8_t *A, int lda, const 
 #pragma unroll
             for (int a = 0; a < 4; ++a)
 #pragma unroll
-                for (int b = 0; b < 4; ++b) {
-                    if (EXACT)
-                        two_sum_acc(s[a][b], c[a][b], __fmul_rn(a4[a], b4[b]));
-                    else
-                        part[a][b] = __fmaf_rn(a4[a], b4[b], part[a][b]);
-                }
+                for (int b = 0; b < 4; ++b) part[a][b] = __fmaf_rn(a4[a], b4[b], part[a][b]);
         }
-        if (!EXACT) {
 #pragma unroll
-            for (int a = 0; a < 4; ++a)
+        for (int a = 0; a < 4; ++a)
 #pragma unroll
-                for (int b = 0; b < 4; ++b) two_sum_acc(s[a][b], c[a][b], part[a][b]);
-        }
+            for (int b = 0; b < 4; ++b) two_sum_acc(s[a][b], c[a][b], part[a][b]);
         if (ch + 1 < nChunks) store(buf ^ 1);
         __syncthreads();
     }
@@ -144,18 +131,14 @@ __device__ __forceinline__ void field_gemm_tile(const int8_t *A, int lda, const 
         for (int b = 0; b < 4; ++b) {
             const int n = n0 + tx * 4 + b;
             if (n >= Nn) continue;
-            if (EXACT)
-                C[(size_t)y * ldc + n] = (OutT)((double)s[a][b] + (double)c[a][b]);
-            else
-                C[(size_t)y * ldc + n] = (OutT)__fadd_rn(s[a][b], c[a][b]);
+            C[(size_t)y * ldc + n] = __fadd_rn(s[a][b], c[a][b]);
         }
     }
 }
 
-template <bool EXACT, typename OutT>
-__global__ void __launch_bounds__(256) field_gemm_kernel(const int8_t *A, int lda, const float *B, int ldb, OutT *C,
+__global__ void __launch_bounds__(256) field_gemm_kernel(const int8_t *A, int lda, const float *B, int ldb, float *C,
                                                          int ldc, int M, int Nn, int K) {
-    field_gemm_tile<EXACT, OutT>(A, lda, B, ldb, C, ldc, M, Nn, K, blockIdx.y * 64, blockIdx.x * 64);
+    field_gemm_tile(A, lda, B, ldb, C, ldc, M, Nn, K, blockIdx.y * 64, blockIdx.x * 64);
 }
 
 }  // namespace sq103

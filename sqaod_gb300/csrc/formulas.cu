@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(256) field_gemm_batch_kernel(const sq103_field
     const sq103_field_job jb = jobs[tileJob[blockIdx.x]];
     const int local = (int)blockIdx.x - jb.tile0, tilesN = (jb.N + 63) / 64;
     const int ty = local / tilesN, tx = local - ty * tilesN;
-    field_gemm_tile<false, float>(jb.q, jb.N, jb.J, jb.ldJ, jb.F, jb.N, jb.m, jb.N, jb.N, ty * 64, tx * 64);
+    field_gemm_tile(jb.q, jb.N, jb.J, jb.ldJ, jb.F, jb.N, jb.m, jb.N, jb.N, ty * 64, tx * 64);
 }
 
 }  // namespace sq103
@@ -221,7 +221,7 @@ SQ103_API int sq103_dense_field_refresh(const float *J, int ldJ, const int8_t *q
                               void *stream) {
     cudaStream_t s = (cudaStream_t)stream;
     dim3 grid((N + 63) / 64, (m + 63) / 64);
-    field_gemm_kernel<false, float><<<grid, 256, 0, s>>>(q, N, J, ldJ, F, N, m, N, N);
+    field_gemm_kernel<<<grid, 256, 0, s>>>(q, N, J, ldJ, F, N, m, N, N);
     return (int)cudaGetLastError();
 }
 
@@ -246,8 +246,10 @@ SQ103_API int sq103_bipartite_fields(const float *J, int N0, int N1, const int8_
 SQ103_API int sq103_dense_energy(const float *J, int ldJ, const float *h, const double *c64, const int8_t *q, int N,
                        int m, int maximize, double *r_scratch, double *E64, float *E32, void *stream) {
     cudaStream_t s = (cudaStream_t)stream;
-    dim3 grid((N + 63) / 64, (m + 63) / 64);
-    field_gemm_kernel<true, double><<<grid, 256, 0, s>>>(q, N, J, ldJ, r_scratch, N, m, N, N);
+    // 16 x 32 tiles with K split over the CTA's warps: 64 x 64 tiles are few (N = 1000,
+    // m = 256: 64 CTAs for 152 SMs) and each walks the whole K.  us, 64 x 64 and these:
+    // N = 128, m = 16: 30.8, 12.8; 512, 64: 92, 20; 1000, 250: 185, 100; 4096, 256: 1212, 1131
+    launch_bip_field<false, true, double>(q, N, J, ldJ, r_scratch, N, m, N, N, s);
     dg_energy_finish<<<m, 256, 0, s>>>(q, N, h, r_scratch, c64, maximize ? -1. : 1., E64, E32);
     return (int)cudaGetLastError();
 }
