@@ -136,9 +136,4 @@ __device__ __forceinline__ void field_gemm_tile(const int8_t *A, int lda, const 
     }
 }
 
-__global__ void __launch_bounds__(256) field_gemm_kernel(const int8_t *A, int lda, const float *B, int ldb, float *C,
-                                                         int ldc, int M, int Nn, int K) {
-    field_gemm_tile(A, lda, B, ldb, C, ldc, M, Nn, K, blockIdx.y * 64, blockIdx.x * 64);
-}
-
 }  // namespace sq103

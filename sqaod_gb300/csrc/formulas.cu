@@ -180,6 +180,11 @@ __global__ void __launch_bounds__(256) ring_dot(const int8_t *q, int N, int m, l
     if (threadIdx.x == 0) atomicAdd((unsigned long long *)out, (unsigned long long)(long long)t);
 }
 
+__global__ void __launch_bounds__(256) field_gemm_kernel(const int8_t *A, int lda, const float *B, int ldb, float *C,
+                                                         int ldc, int M, int Nn, int K) {
+    field_gemm_tile(A, lda, B, ldb, C, ldc, M, Nn, K, blockIdx.y * 64, blockIdx.x * 64);
+}
+
 // One 64 x 64 tile of one job's fields per CTA; the tile arithmetic is the one
 // of field_gemm_kernel, so each job's fields equal its own refresh bit for bit.
 __global__ void __launch_bounds__(256) field_gemm_batch_kernel(const sq103_field_job *jobs, const int *tileJob) {
