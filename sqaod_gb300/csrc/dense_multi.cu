@@ -135,6 +135,24 @@ __host__ __device__ __forceinline__ int colour_phase(int y, int m) {
     return (y & 1) ? 2 : 0;
 }
 
+// A prefetched trial (lane i of a batch): its site, h at the site, L = -ln u, and
+// the constants of its step: dE's factors of h + 2F and of the spin sum times the
+// rate, and the part of the decision's tolerance that does not depend on the
+// field; its neighbour candidates, one byte each (two per neighbour, the latest
+// first: 32 p + 31 - j for iteration j of the window of batch p).
+struct __align__(16) PreTrial {
+    int x;
+    float h, L, cz;
+    float cb, tolC, u;
+    uint32_t cand;
+};
+constexpr uint32_t kNoCand = 127, kManyCand = 126;
+constexpr uint32_t kNoCands = 0x7f7f7f7fu;
+// bytes of the field row, the h row and the in-batch gathers, up to a 16-byte boundary
+__host__ __device__ __forceinline__ constexpr size_t pre_offset(int N) {
+    return ((size_t)N * 8 + (size_t)kPre * kJgStride * 4 + 15) & ~(size_t)15;
+}
+
 struct McShared {
     volatile unsigned long long logAvail;  // neighbour accept bits known below (lo: neighbour 0, hi: 1) (helper)
     volatile int applied[2];               // neighbour iterations applied to the ghost rows (decider)
@@ -283,16 +301,12 @@ __global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const __
     float *Fs = reinterpret_cast<float *>(smem);                        // N
     float *hs = Fs + N;                                                 // N
     float *Jg = hs + N;                                                 // kPre x 32 x 33
-    float *preU = Jg + kPre * kJgStride;                                // kPre x 32
-    float *preC = preU + kPre * 32;                                     // kPre x 3 x 32
-    float *preL = preC + kPre * 96;                                     // kPre x 32: -ln u
-    int *preX = reinterpret_cast<int *>(preL + kPre * 32);              // kPre x 32
-    uint32_t *ghost = reinterpret_cast<uint32_t *>(preX + kPre * 32);   // 2 x ghostStride
-    uint32_t *bm = ghost + 2 * ghostStride;                             // 2 x kBmSlots x kBmWords
+    PreTrial *pre = reinterpret_cast<PreTrial *>(smem + pre_offset(N));  // kPre x 32
+    uint2 *ghost = reinterpret_cast<uint2 *>(pre + kPre * 32);          // nWG: spin bits of both neighbours
+    uint32_t *bm = reinterpret_cast<uint32_t *>(ghost + ghostStride);   // 2 x kBmSlots x kBmWords
     int *ring = reinterpret_cast<int *>(bm + 2 * kBmSlots * kBmWords);  // 2 x kRing
     uint32_t *nlog = reinterpret_cast<uint32_t *>(ring + 2 * kRing);    // 2 x kLogWords
-    int *cand = reinterpret_cast<int *>(nlog + 2 * kLogWords);          // kPre x 2 x kCand x 32
-    unsigned *prePred = reinterpret_cast<unsigned *>(cand + kPre * 2 * kCand * 32);  // kPre
+    unsigned *prePred = reinterpret_cast<unsigned *>(nlog + 2 * kLogWords);  // kPre
     int2 *flips = reinterpret_cast<int2 *>(prePred + kPre);             // 32
     int8_t *qs = reinterpret_cast<int8_t *>(flips + 32);                // N
     // kSmall: one site table of kSmallN words per prefetcher (positions of a batch by site)
@@ -310,7 +324,7 @@ __global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const __
         for (int w = tid; w < nWG; w += kMcThreads) {
             uint32_t bits = 0;
             for (int b = 0; b < 32 && w * 32 + b < N; ++b) bits |= (qn[w * 32 + b] > 0 ? 1u : 0u) << b;
-            ghost[n * ghostStride + w] = bits;
+            (n ? ghost[w].y : ghost[w].x) = bits;
         }
     }
     if (tid == 0) {
@@ -335,7 +349,7 @@ __global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const __
         unsigned long long accepted = 0;
         bool aborted = false;
         int nfPrev = 0;      // flips of the previous batch still to be added to Fv
-        int qb0 = 0, qb1 = 0, nd0 = -1, nd1 = -1;  // neighbour bits of the lane's site, unknown iterations
+        int nd0 = -1, nd1 = -1;  // the unknown neighbour iterations of the lane's site
         int x = 0;                                  // the lane's site in the current batch
         float gv[kGv];       // their gathers J[x_f][x] (at this batch's sites)
 #pragma unroll
@@ -350,87 +364,89 @@ __global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const __
             const unsigned long long av = uniform_acquire64(&S.logAvail);
             lim0 = min(avail_of(av, 0), lim0);
             lim1 = nNbr > 1 ? min(avail_of(av, 1), lim1) : 0;
-            const int span = max(lim0 - A0, lim1 - A1);
-            for (int j0 = 0; j0 < span; j0 += 32) {
+            if (lim0 <= A0 && lim1 <= A1) return av;
 #pragma unroll
-                for (int n = 0; n < 2; ++n) {
-                    const int j = (n ? A1 : A0) + j0 + lane;
-                    if (n < nNbr && j < (n ? lim1 : lim0) &&
-                        ((nlog[n * kLogWords + ((j >> 5) & (kLogWords - 1))] >> (j & 31)) & 1u)) {
-                        const int site = ring[n * kRing + (j & (kRing - 1))];
-                        atomicXor(&ghost[n * ghostStride + (site >> 5)], 1u << (site & 31));
+            for (int n = 0; n < 2; ++n) {
+                const int A = n ? A1 : A0, lim = n ? lim1 : lim0;
+                for (int w = A >> 5; w * 32 < lim; ++w) {
+                    uint32_t bits = nlog[n * kLogWords + (w & (kLogWords - 1))];
+                    if (w * 32 < A) bits &= ~0u << (A & 31);
+                    if (w * 32 + 32 > lim) bits &= (1u << (lim & 31)) - 1u;
+                    if ((bits >> lane) & 1u) {
+                        const int site = ring[n * kRing + ((w * 32 + lane) & (kRing - 1))];
+                        atomicXor(n ? &ghost[site >> 5].y : &ghost[site >> 5].x, 1u << (site & 31));
                     }
                 }
             }
-            if (span > 0) {
-                A0 = max(A0, lim0);
-                if (nNbr > 1) A1 = max(A1, lim1);
-                __syncwarp();
-                if (lane == 0) {
-                    S.applied[0] = A0;
-                    S.applied[1] = A1;
-                }
+            A0 = max(A0, lim0);
+            A1 = max(A1, lim1);
+            __syncwarp();
+            if (lane == 0) {
+                S.applied[0] = A0;
+                S.applied[1] = A1;
             }
             return av;
         };
 
-        // Neighbour bits at the lane's site for batch b: the ghost row (iterations
+        // Neighbour spins at the lane's site x for batch b: the ghost rows (iterations
         // < A applied) corrected by the neighbour iterations in [A, Ji] at the site,
         // which the prefetchers listed (the latest kCand of the last three batches).
-        // A neighbour more than two batches behind, or a longer list, takes the
-        // bitmap scan of window_bits.  need: latest unpublished such iteration (-1: none).
-        auto nbr_bits = [&](int b, int g0, bool valid, unsigned long long av) {
-            const int buf = b & (kPre - 1);
-            bool slow = false;
+        // A neighbour more than two batches behind, or a longer list, takes the bitmap
+        // scan of window_bits.  sum: the known spins' sum; nd0, nd1: the latest
+        // unpublished such iteration of each neighbour (-1: its spin is known).
+        auto nbr_spins = [&](int b, int g0, bool valid, uint32_t cand, unsigned long long av, int &sum) {
+            const uint2 g = ghost[x >> 5];
+            int b0 = (g.x >> (x & 31)) & 1, b1 = (g.y >> (x & 31)) & 1;
+            nd0 = nd1 = -1;
+            bool slow = A0 < 32 * (b - 2) || (nNbr > 1 && A1 < 32 * (b - 2));
+            if (!valid) cand = kNoCands;
+            if (cand != kNoCands) {
 #pragma unroll
-            for (int n = 0; n < 2; ++n) {
-                if (n >= nNbr) break;
-                const int A = n ? A1 : A0, avail = avail_of(av, n);
-                int bit = (ghost[n * ghostStride + (x >> 5)] >> (x & 31)) & 1, need = -1;
-                const int ca = cand[((buf * 2 + n) * kCand) * 32 + lane];
-                const int cb = cand[((buf * 2 + n) * kCand + 1) * 32 + lane];
-                slow |= ca == -2 || A < 32 * (b - 2);
-#pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                    const int j = c ? cb : ca;
-                    if (j >= A) {
-                        if (j < avail)
-                            bit ^= (nlog[n * kLogWords + ((j >> 5) & (kLogWords - 1))] >> (j & 31)) & 1u;
-                        else
-                            need = max(need, j);
+                for (int c = 0; c < 4; ++c) {
+                    const int n = c >> 1, v = (cand >> (8 * c)) & 0xff, j = g0 + 31 - v;
+                    if (v == (int)kManyCand) slow = true;
+                    if (v < (int)kManyCand && j >= (n ? A1 : A0)) {
+                        if (j < avail_of(av, n)) {
+                            const int f = (nlog[n * kLogWords + ((j >> 5) & (kLogWords - 1))] >> (j & 31)) & 1u;
+                            if (n)
+                                b1 ^= f;
+                            else
+                                b0 ^= f;
+                        } else if (n) {
+                            nd1 = max(nd1, j);
+                        } else {
+                            nd0 = max(nd0, j);
+                        }
                     }
-                }
-                if (n) {
-                    qb1 = bit;
-                    nd1 = valid ? need : -1;
-                } else {
-                    qb0 = bit;
-                    nd0 = valid ? need : -1;
                 }
             }
             slow = slow && valid;
             if (__any_sync(FULL, slow)) {
-#pragma unroll
-                for (int n = 0; n < 2; ++n) {
-                    if (n >= nNbr) break;
-                    int bit = (ghost[n * ghostStride + (x >> 5)] >> (x & 31)) & 1, need;
+#pragma unroll 1
+                for (int n = 0; n < nNbr; ++n) {
+                    int bit = ((n ? g.y : g.x) >> (x & 31)) & 1, need;
                     window_bits(x, g0 + lane - 1 + (n ? before1 : before0), n ? A1 : A0, b, avail_of(av, n), slow,
                                 bm + n * kBmSlots * kBmWords, ring + n * kRing, nlog + n * kLogWords, Itot, bit, need);
                     if (slow) {
                         if (n) {
-                            qb1 = bit;
+                            b1 = bit;
                             nd1 = need;
                         } else {
-                            qb0 = bit;
+                            b0 = bit;
                             nd0 = need;
                         }
                     }
                 }
             }
+            if (nNbr == 1) {  // m = 2: the one neighbour on both sides
+                b1 = b0;
+                nd1 = nd0;
+            }
+            sum = (nd0 >= 0 ? 0 : 2 * b0 - 1) + (nd1 >= 0 ? 0 : 2 * b1 - 1);
         };
 
         aborted = !wait_until(waitNs, [&] { return uniform_acquire(&S.readyTag[0]) == 1; });
-        x = preX[lane];
+        x = pre[lane].x;
         float Fv = Fs[x];
 
         for (int b = 0; b < nBatches && !aborted; ++b) {
@@ -438,22 +454,20 @@ __global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const __
             const int buf = b & (kPre - 1);
             const int nValid = min(32, Itot - g0);
             const bool valid = lane < nValid;
-            const float u = preU[buf * 32 + lane], Lu = preL[buf * 32 + lane];
-            const StepConst sc = {preC[buf * 96 + lane], preC[buf * 96 + 32 + lane], preC[buf * 96 + 64 + lane]};
+            const PreTrial tr = pre[buf * 32 + lane];
             const float *jg = Jg + buf * kJgStride + lane * 33;
             const unsigned pred = prePred[buf];  // lanes whose row of in-batch gathers is in jg
-            const float hx = valid ? hs[x] : 0.f;
-            float qx = valid ? (float)qs[x] : 1.f;
+            float qx = (float)qs[x];
 
             // neighbour spins at this batch's sites: apply the published neighbour
             // iterations before this batch's first trial (their sites are in the ring
-            // since this batch's buffer is ready); each lane's site is corrected at the
-            // top of the first round
-            qb0 = qb1 = 0;
+            // since this batch's buffer is ready); each lane's site is then corrected
+            int sum = 0;
             nd0 = nd1 = -1;
-            unsigned blocked = 0;
-            unsigned long long avEval = 0;  // availability the lanes' neighbour bits are evaluated with
-            if (nNbr > 0) avEval = apply_nbr(g0 + before0, g0 + before1);
+            if (nNbr > 0) {
+                const unsigned long long av = apply_nbr(g0 + before0, g0 + before1);
+                nbr_spins(b, g0, valid, tr.cand, av, sum);
+            }
 
             // the previous batch's flips (gathered at the end of that batch)
 #pragma unroll
@@ -462,62 +476,51 @@ __global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const __
                 Fv = __fmaf_rn(__int_as_float(flips[t].y), gv[t], Fv);
             }
 
+            // The trial accepts when z = rate dE - L < 0.  z = zA - ring, zA = cz q (h + 2F) - L
+            // and ring = cb q (qL + qR); unknown neighbour spins leave it in [z - sp, z + sp].
+            // A lane is decided when that interval lies outside [-tol, tol], the fp32 error
+            // bound (sq_common.cuh; the ring's part four times as wide here, for the sums kept
+            // over a batch's flips).  A flip adds cz q 2 d J to zA, and changes the signs of a
+            // later trial at its site.  (A round that evaluated dE anew, with up to four
+            // evaluations for unknown spins, took 970 cycles at two CTAs per SM; the decider is
+            // the critical path, at 10 cycles an instruction.  N = 4096, m = 256, 64 steps: 24.2
+            // ms before, 20.3 with this; N = 1000, m = 250: 8.0, 6.8.)
+            float zA, ring_, sp, tol;
+            const float kF = fabsf(tr.cz) * 1.52587890625e-5f;
+            float c2 = 2.f * tr.cz * qx;
+            {
+                const float t = __fmaf_rn(2.f, Fv, tr.h), cbq = tr.cb * qx;
+                zA = __fmaf_rn(tr.cz * qx, t, -tr.L);
+                ring_ = cbq * (float)sum;
+                sp = fabsf(cbq) * (float)((nd0 >= 0) + (nd1 >= 0));
+                tol = __fmaf_rn(kF, fabsf(tr.h) + 2.f * fabsf(Fv) + 1.f, tr.tolC);
+            }
+
             // decide the batch in rounds
             unsigned pending = __ballot_sync(FULL, valid), accBits = 0;
             float d = 0.f;
-            bool exValid = false;  // exBits holds the FP64 outcomes of the lane's trial
-            int exBits = 0;
-            const DecisionTol tolD = decision_tol(sa, true, sc.twoDivM, sc.coef, sc.rate);
-            float xt = trial_xtol(tolD, hx, __fmul_rn(2.f, Fv), Lu);  // updated when Fv changes
-            bool evalNbr = nNbr > 0;  // (one instance of nbr_bits keeps the loop's code small)
-            while (pending) {
-                if (evalNbr) {
-                    nbr_bits(b, g0, valid, avEval);
-                    blocked = __ballot_sync(FULL, nd0 >= 0 || nd1 >= 0) & pending;
-                    evalNbr = false;
-                }
-                // a lane with unknown neighbour bits is decided anyway when every value
-                // those bits can take gives the same outcome; it blocks otherwise.  The
-                // outcomes come from the fp32 field, or from the FP64 outcomes of a
-                // flagged lane's trial; a flagged lane (one whose fp32 outcome the field's
-                // rounding could change) blocks too, until it has its FP64 outcomes
-                int acc = 0, amb = 0, nearT = 0;
-                if ((pending >> lane) & 1u) {
-                    const float qn0 = qb0 ? 1.f : -1.f, qn1 = nNbr == 1 ? qn0 : (qb1 ? 1.f : -1.f);
-                    auto accept = [&](float a, float c) -> int {
-                        if (exValid) return (exBits >> (((int)a + (int)c + 2) >> 1)) & 1;
-                        const float dE = sa ? dense_sa_dE(qx, hx, Fv)
-                                            : dense_sqa_dE(qx, hx, Fv, a, c, sc.twoDivM, sc.coef);
-                        return metropolis_log(dE, sc.rate, Lu, xt, nearT);
-                    };
-                    acc = accept(qn0, qn1);
-                    if ((blocked >> lane) & 1u) {
-                        const bool u0 = nd0 >= 0, u1 = nNbr > 1 && nd1 >= 0;
-                        if (u0 && accept(-qn0, nNbr == 1 ? -qn0 : qn1) != acc) amb = 1;
-                        if (u1 && accept(qn0, -qn1) != acc) amb = 1;
-                        if (u0 && u1 && accept(-qn0, -qn1) != acc) amb = 1;
-                    }
-                }
-                amb |= nearT;
-                const unsigned accM = __ballot_sync(FULL, acc && !amb) & pending;
-                const unsigned blkM = __ballot_sync(FULL, amb) & pending;
+            for (;;) {
+                const float z = zA - ring_;
+                const unsigned accM = __ballot_sync(FULL, z + sp < -tol) & pending;
+                const unsigned blkM = __ballot_sync(FULL, z - sp <= tol) & pending & ~accM;
                 const int fa = accM ? __ffs(accM) - 1 : 32;
                 const int fb = blkM ? __ffs(blkM) - 1 : 32;
                 if (fb < fa) {
                     // undecided lanes below fb reject
                     pending &= ~((1u << fb) - 1u);
                     if (lane == 0 && publish) st_relaxed_u64(outLog + (size_t)y * nWords + b, log_word(b, fb, accBits));
-                    if (__shfl_sync(FULL, nearT, fb)) {
-                        // fb is flagged: the exact warp decides its trial in FP64 from the
-                        // exact field (every flip before the trial is in qs), for each value
-                        // of the neighbours' spin sum; then the round is evaluated again.
+                    const int w0 = __shfl_sync(FULL, nd0, fb), w1 = __shfl_sync(FULL, nd1, fb);
+                    if (w0 < 0 && w1 < 0) {
+                        // fb is too near its threshold: the exact warp decides its trial in FP64
+                        // from the exact field (every flip before the trial is in qs), for each
+                        // value of the neighbours' spin sum; then the round is evaluated again.
                         // (The decider's arrival on a named barrier wakes the exact warp, which
                         // sleeps there between requests; the decider's wait is bounded.)
                         if (lane == fb) {
                             const int sl = (g0 + lane) / N;
                             S.exX = x;
                             S.exQ = qx;
-                            S.exU = u;
+                            S.exU = tr.u;
                             S.exG = T.G ? T.G[sl] : T.Gs;
                             S.exBeta = T.beta ? T.beta[sl] : T.betas;
                         }
@@ -529,14 +532,10 @@ __global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const __
                             aborted = true;
                             break;
                         }
-                        if (lane == fb) {
-                            exBits = S.exBits;
-                            exValid = true;
-                        }
+                        if (lane == fb) zA = (S.exBits >> ((sum + 2) >> 1)) & 1 ? -3e38f : 3e38f;
                         continue;
                     }
                     // fb waits for its neighbour trials
-                    const int w0 = __shfl_sync(FULL, nd0, fb), w1 = __shfl_sync(FULL, nd1, fb);
                     unsigned long long av = 0;
                     if (!wait_until(waitNs, [&] {
                             av = uniform_acquire64(&S.logAvail);
@@ -545,15 +544,21 @@ __global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const __
                         aborted = true;
                         break;
                     }
-                    // re-evaluate (the ghost rows and A are unchanged within the batch)
-                    avEval = av;
-                    evalNbr = true;
+                    // evaluate again (the ghost rows and A are unchanged within the batch)
+                    nbr_spins(b, g0, valid, tr.cand, av, sum);
+                    const float cbq = tr.cb * qx;
+                    ring_ = cbq * (float)sum;
+                    sp = fabsf(cbq) * (float)((nd0 >= 0) + (nd1 >= 0));
                     continue;
                 }
                 if (fa == 32) break;  // every undecided lane rejects
                 // undecided lanes below fa reject; fa flips
                 const int xf = __shfl_sync(FULL, x, fa);
                 const float df = -2.f * __shfl_sync(FULL, qx, fa);
+                accBits |= 1u << fa;
+                pending &= ~((2u << fa) - 1u);
+                // trials through fa are decided: make them visible to the neighbours
+                if (lane == 0 && pending && publish) st_relaxed_u64(outLog + (size_t)y * nWords + b, log_word(b, fa + 1, accBits));
                 if (lane == fa) {
                     qs[x] = (int8_t)(qx > 0.f ? -1 : 1);
                     d = df;
@@ -563,17 +568,18 @@ __global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const __
                         atomicOr(&T.trace[(size_t)s * wordsPerStep + (bitIdx >> 5)], 1u << (bitIdx & 31));
                     }
                 }
+                if (!pending) break;
                 if (lane > fa) {
-                    const float jv = ((pred >> fa) & 1u) ? jg[fa] : __ldg(T.J + (size_t)xf * T.ldJ + x);
-                    Fv = __fmaf_rn(df, jv, Fv);
-                    xt = trial_xtol(tolD, hx, __fmul_rn(2.f, Fv), Lu);
-                    if (x == xf) qx = -qx;
-                    exValid = false;  // the trial now follows another flip
+                    const float dJ = df * (((pred >> fa) & 1u) ? jg[fa] : __ldg(T.J + (size_t)xf * T.ldJ + x));
+                    zA = __fmaf_rn(c2, dJ, zA);
+                    tol = __fmaf_rn(2.f * kF, fabsf(dJ), tol);
+                    if (x == xf) {
+                        qx = -qx;
+                        c2 = -c2;
+                        zA = -(zA + tr.L) - tr.L;
+                        ring_ = -ring_;
+                    }
                 }
-                accBits |= 1u << fa;
-                pending &= ~((2u << fa) - 1u);
-                // trials through fa are decided: make them visible to the neighbours
-                if (lane == 0 && pending && publish) st_relaxed_u64(outLog + (size_t)y * nWords + b, log_word(b, fa + 1, accBits));
             }
             if (aborted) break;
             __syncwarp();
@@ -596,24 +602,24 @@ __global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const __
                 aborted = true;
                 break;
             }
-            const int xN = more ? preX[((b + 1) & (kPre - 1)) * 32 + lane] : 0;
-            const bool validN = g0 + 32 + lane < Itot;
+            const int xN = more ? pre[((b + 1) & (kPre - 1)) * 32 + lane].x : 0;
             // the next batch's fields start from the resident row once the updaters
             // are done with the previous batch's flips; this batch's flips are
             // gathered now and added after the next batch's neighbour work
+            // (lanes beyond the last trial have site 0)
             const bool defer = nf <= kGv;
             if (defer && accBits) {
                 unsigned rem = accBits;
 #pragma unroll
                 for (int t = 0; t < kGv; ++t) {
                     const int xf = __shfl_sync(FULL, x, __ffs(rem) - 1);
-                    gv[t] = validN ? __ldg(T.J + (size_t)xf * T.ldJ + xN) : 0.f;
+                    gv[t] = __ldg(T.J + (size_t)xf * T.ldJ + xN);
                     rem &= rem - 1u;
                     if (!rem) break;
                 }
             }
             bar_sync(2, kBarCount);
-            float FvN = validN ? Fs[xN] : 0.f;
+            float FvN = Fs[xN];
             if ((accBits >> lane) & 1u) flips[__popc(accBits & ((1u << lane) - 1u))] = make_int2(x, __float_as_int(d));
             if (lane == 0) S.nflip = nf;
             __syncwarp();
@@ -628,7 +634,7 @@ __global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const __
                     rem &= rem - 1u;
                     const int xf = __shfl_sync(FULL, x, f);
                     const float df = __shfl_sync(FULL, d, f);
-                    if (validN) FvN = __fmaf_rn(df, __ldg(T.J + (size_t)xf * T.ldJ + xN), FvN);
+                    FvN = __fmaf_rn(df, __ldg(T.J + (size_t)xf * T.ldJ + xN), FvN);
                 }
             }
             x = xN;
@@ -756,10 +762,10 @@ __global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const __
             {
                 const volatile float *vF = Fs, *vh = hs;
                 const volatile int8_t *vq = qs;
-                const volatile uint32_t *vg = ghost;
+                const volatile uint32_t *vg = reinterpret_cast<const volatile uint32_t *>(ghost);
                 const float qx = (float)vq[x], hx = vh[x], fx = vF[x];
-                float qn0 = ((vg[x >> 5] >> (x & 31)) & 1u) ? 1.f : -1.f;
-                float qn1 = nNbr > 1 ? (((vg[ghostStride + (x >> 5)] >> (x & 31)) & 1u) ? 1.f : -1.f) : qn0;
+                float qn0 = ((vg[2 * (x >> 5)] >> (x & 31)) & 1u) ? 1.f : -1.f;
+                float qn1 = nNbr > 1 ? (((vg[2 * (x >> 5) + 1] >> (x & 31)) & 1u) ? 1.f : -1.f) : qn0;
                 const float dE = sa ? dense_sa_dE(qx, hx, fx) : dense_sqa_dE(qx, hx, fx, qn0, qn1, sc.twoDivM, sc.coef);
                 const float margin = (sa ? 4.f : 2.f * sc.twoDivM) * kFieldDrift;
                 const float dEm = dE - margin;
@@ -781,6 +787,12 @@ __global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const __
             // flight): ring entries and the batch's site bitmaps; then, per lane and
             // neighbour, the latest kCand iterations of batches p - 2 .. p that hit
             // the lane's site up to its limit (-2: more than kCand)
+            uint32_t cands = kNoCands;
+            auto put_cands = [&](int nn, int c0, int c1) {
+                const uint32_t e0 = c0 == -2 ? kManyCand : c0 < 0 ? kNoCand : (uint32_t)(32 * p + 31 - c0);
+                const uint32_t e1 = c1 < 0 ? kNoCand : (uint32_t)(32 * p + 31 - c1);
+                cands = nn ? (cands & 0xffffu) | (e0 << 16) | (e1 << 24) : (cands & 0xffff0000u) | e0 | (e1 << 8);
+            };
             if (nNbr > 0) {
                 uint32_t *bp = bm + (p & (kBmSlots - 1)) * kBmWords;
                 bp[lane] = 0u;
@@ -858,8 +870,7 @@ __global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const __
                             }
                         }
                         if (cnt > kCand) c0 = -2;
-                        cand[((buf * 2 + nn) * kCand) * 32 + lane] = c0;
-                        cand[((buf * 2 + nn) * kCand + 1) * 32 + lane] = cnt > kCand ? -1 : c1;
+                        put_cands(nn, c0, cnt > kCand ? -1 : c1);
                     }
                 } else {
 #pragma unroll
@@ -902,8 +913,7 @@ __global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const __
                             }
                         }
                     }
-                    cand[((buf * 2 + nn) * kCand) * 32 + lane] = c0;
-                    cand[((buf * 2 + nn) * kCand + 1) * 32 + lane] = c1;
+                    put_cands(nn, c0, c1);
                 }
                 }
             }
@@ -924,12 +934,20 @@ __global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const __
                 }
             }
             if (lane == 0) prePred[buf] = pred;
-            preX[buf * 32 + lane] = x;
-            preU[buf * 32 + lane] = u;
-            preL[buf * 32 + lane] = neg_log_unit(u);
-            preC[buf * 96 + lane] = sc.twoDivM;
-            preC[buf * 96 + 32 + lane] = sc.coef;
-            preC[buf * 96 + 64 + lane] = sc.rate;
+            {
+                PreTrial tr;
+                tr.x = x;
+                tr.h = hs[x];
+                tr.L = fminf(neg_log_unit(u), 1e30f);
+                tr.cz = sc.rate * (sa ? 2.f : sc.twoDivM);
+                // (0 for SA; G = 0 or beta = 0 make coef infinite: its sign then decides)
+                const float cb = sc.rate * sc.coef;
+                tr.cb = sa ? 0.f : isfinite(cb) ? cb : copysignf(1e30f, sc.coef);
+                tr.tolC = 4e-6f * fabsf(tr.cb) + 2e-6f + 1e-6f * tr.L;
+                tr.u = u;
+                tr.cand = cands;
+                pre[buf * 32 + lane] = tr;
+            }
             __syncwarp();
             if (lane == 0) st_release_cta(&S.readyTag[buf], p + 1);
             k += 32 * kPf;
@@ -1000,8 +1018,8 @@ __global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const __
 
 static size_t multi_smem_bytes(int N) {
     size_t ghostStride = (size_t)((N + 31) / 32 + 1) & ~(size_t)1;
-    return (size_t)N * 4 * 2 + (size_t)kPre * (kJgStride + 32 + 96 + 32 + 32) * 4 + 2 * ghostStride * 4 +
-           (size_t)2 * kBmSlots * kBmWords * 4 + 2 * kRing * 4 + 2 * kLogWords * 4 + (size_t)kPre * 2 * kCand * 32 * 4 + kPre * 4 +
+    return pre_offset(N) + (size_t)kPre * 32 * sizeof(PreTrial) + 2 * ghostStride * 4 +
+           (size_t)2 * kBmSlots * kBmWords * 4 + 2 * kRing * 4 + 2 * kLogWords * 4 + kPre * 4 +
            32 * 8 + (size_t)((N + 15) & ~15) + 16 + (N <= kSmallN ? (size_t)kPf * kSmallN * 4 : 0);
 }
 
