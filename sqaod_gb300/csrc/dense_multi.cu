@@ -52,6 +52,7 @@
 
 #include <algorithm>
 #include <mutex>
+#include <vector>
 
 // the exact warp's helpers inlined: measured 1.8 % faster at N=4096 m=256
 #define SQ103_EXACT_ATTR __forceinline__
@@ -60,12 +61,12 @@
 
 namespace sq103 {
 
-constexpr int kMcThreads = 256;
 constexpr int kPf = 2;                            // prefetcher warps (2 .. 1 + kPf)
 constexpr int kUpdWarp0 = 2 + kPf;                // first updater warp
-constexpr int kExactWarp = kMcThreads / 32 - 1;   // the last warp: exact decisions
-constexpr int kMcUpdaters = kMcThreads - 32 * kUpdWarp0 - 32;
-constexpr int kBarCount = 32 + kMcUpdaters;       // decider + updaters (barriers 1, 2)
+// threads of a CTA: three updater warps at two CTAs per SM, two at four (the registers
+// of the third go to the others: N = 2000, m = 500 6.6 -> 6.3 ms; at two per SM the
+// third is worth it, N = 4096, m = 256 20.3 -> 19.5 ms)
+__host__ __device__ constexpr int mc_threads(int perSm) { return perSm > 2 ? 224 : 256; }
 constexpr int kBarExReq = 3;                      // wakes the exact warp (decider + exact warp, 64 threads)
 constexpr int kRing = 256;      // neighbour sites kept per neighbour (power of two)
 constexpr int kLogWords = 32;   // neighbour accept words kept per neighbour (power of two)
@@ -74,7 +75,6 @@ constexpr int kBmWords = kBmBits / 32;
 constexpr int kBmSlots = kRing / 32;  // bitmaps kept per neighbour (one per ring batch)
 constexpr int kPre = 4;         // prefetched batches (power of two)
 constexpr int kJgStride = 32 * 33;
-constexpr int kGv = 8;          // flips of a batch whose gathers are deferred to the next batch
 constexpr int kCand = 2;        // neighbour iterations per lane and batch found by the prefetchers
 constexpr int kPredRows = 8;    // predicted accepting lanes whose gathers are kept in registers
 constexpr float kFieldDrift = 1.f;  // assumed field change between prefetch and decision
@@ -139,14 +139,14 @@ __host__ __device__ __forceinline__ int colour_phase(int y, int m) {
 // the constants of its step: dE's factors of h + 2F and of the spin sum times the
 // rate, and the part of the decision's tolerance that does not depend on the
 // field; its neighbour candidates, one byte each (two per neighbour, the latest
-// first: 32 p + 31 - j for iteration j of the window of batch p).
+// first: 32 p + 32 - j for iteration j of the window of batch p).
 struct __align__(16) PreTrial {
     int x;
     float h, L, cz;
     float cb, tolC, u;
     uint32_t cand;
 };
-constexpr uint32_t kNoCand = 127, kManyCand = 126;
+constexpr uint32_t kNoCand = 127, kManyCand = 0;
 constexpr uint32_t kNoCands = 0x7f7f7f7fu;
 // bytes of the field row, the h row and the in-batch gathers, up to a 16-byte boundary
 __host__ __device__ __forceinline__ constexpr size_t pre_offset(int N) {
@@ -163,7 +163,8 @@ struct McShared {
     // exact decisions (rare): the decider posts a trial, the exact warp answers
     int exX, exBits;       // the trial's site; its FP64 outcomes for qL + qR = -2, 0, +2 (bits 0-2)
     volatile int exDone;   // number of the latest answer (exact warp; the decider counts its requests)
-    float exQ, exU, exG, exBeta;
+    float exQ, exU;
+    int exIter;
 };
 
 // every lane loads the flag with acquire semantics (one broadcast access); the
@@ -240,8 +241,12 @@ struct McPack {
     int n;
 };
 
-// kHooks: the test hooks of the task flags are compiled in (short waits, a
-// trotter that withholds its accept words); the production instance has none.
+// kHooks: the acceptance trace and the test hooks of the task flags are compiled in
+// (short waits, a trotter that withholds its accept words).  kSA: simulated
+// annealing, without the neighbours' code.  Code that never runs is not free here:
+// the warps' roles share the instruction caches, and SA at N = 1501, m = 63 took
+// 3.24 ms for 64 steps with the neighbours' and the trace's code compiled in,
+// 3.12 ms without.
 // kSmall: rows of at most kSmallN spins, where the neighbours' sites hit a lane's
 // site often: each prefetcher finds a lane's neighbour candidates from a table
 // of the positions at each site of batches p - 2 .. p (one per batch and
@@ -251,12 +256,16 @@ struct McPack {
 // makes the prefetchers wait for each other).  Both give the same candidates.
 // kPerSm: the CTAs per SM the registers are allotted for.  The trotters of a launch
 // are all resident, so the limit on m is kPerSm * 152 (where shared memory allows
-// as many: N <= 3100 for four).  Two leave 118 registers a thread and the fastest
-// decider; four have 64 (8 bytes spilled) and take the launches that exceed two.
-// N = 2000, m = 500, 8 steps: 7.4 ms with four per SM; one CTA for the whole
+// as many: N <= 3100 for four).  Two leave 116 registers a thread and the fastest
+// decider; four have 72 and take the launches that exceed two.
+// N = 2000, m = 500, 8 steps: 5.9 ms with four per SM; one CTA for the whole
 // instance, which such sizes fell back to before, 1090 ms.
-template <bool kHooks, bool kSmall, int kPerSm>
-__global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const __grid_constant__ McPack P) {
+template <bool kHooks, bool kSmall, bool kSA, int kPerSm>
+__global__ void __launch_bounds__(mc_threads(kPerSm), kPerSm) dense_sweep_multi(const __grid_constant__ McPack P) {
+    constexpr int kMcThreads = mc_threads(kPerSm);
+    constexpr int kExactWarp = kMcThreads / 32 - 1;  // the last warp: exact decisions
+    constexpr int kMcUpdaters = kMcThreads - 32 * kUpdWarp0 - 32;
+    constexpr int kBarCount = 32 + kMcUpdaters;      // decider + updaters (barriers 1, 2)
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ McShared S;
     __shared__ sq103_dense_task task;
@@ -282,7 +291,7 @@ __global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const __
     const int nWords = sWords;
     const int y = (int)blockIdx.x - sBase, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int N = T.N, m = T.m;
-    const bool sa = T.algo == kSANaive;
+    constexpr bool sa = kSA;
     const int nNbr = sa ? 0 : (m == 2 ? 1 : 2);
     const int nbr0 = (y + m - 1) % m, nbr1 = (y + 1) % m;
     const int myPh = colour_phase(y, m);
@@ -346,14 +355,16 @@ __global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const __
     if (warp == 0) {
         // ------------------------------------------------------------ decider
         const uint32_t wordsPerStep = (uint32_t)(((size_t)N * m + 31) / 32);
+        const float *const J = T.J;
+        const int ldJ = T.ldJ;
+        const bool traced = kHooks && T.trace != nullptr;
+        unsigned long long *const myLog = outLog + (size_t)y * nWords;
         unsigned long long accepted = 0;
         bool aborted = false;
-        int nfPrev = 0;      // flips of the previous batch still to be added to Fv
-        int nd0 = -1, nd1 = -1;  // the unknown neighbour iterations of the lane's site
-        int x = 0;                                  // the lane's site in the current batch
-        float gv[kGv];       // their gathers J[x_f][x] (at this batch's sites)
-#pragma unroll
-        for (int t = 0; t < kGv; ++t) gv[t] = 0.f;
+        unsigned accBits = 0;  // the previous batch's flips (lanes), their sites x and changes d = -2 q
+        float d = 0.f;
+        int x = 0;                 // the lane's site
+        int nd0 = -1, nd1 = -1;    // the unknown neighbour iterations at the lane's site
 
         int A0 = 0, A1 = 0;  // neighbour iterations applied to the ghost rows
         int exSeq = 0;       // exact-decision requests posted
@@ -365,18 +376,13 @@ __global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const __
             lim0 = min(avail_of(av, 0), lim0);
             lim1 = nNbr > 1 ? min(avail_of(av, 1), lim1) : 0;
             if (lim0 <= A0 && lim1 <= A1) return av;
-#pragma unroll
-            for (int n = 0; n < 2; ++n) {
-                const int A = n ? A1 : A0, lim = n ? lim1 : lim0;
-                for (int w = A >> 5; w * 32 < lim; ++w) {
-                    uint32_t bits = nlog[n * kLogWords + (w & (kLogWords - 1))];
-                    if (w * 32 < A) bits &= ~0u << (A & 31);
-                    if (w * 32 + 32 > lim) bits &= (1u << (lim & 31)) - 1u;
-                    if ((bits >> lane) & 1u) {
-                        const int site = ring[n * kRing + ((w * 32 + lane) & (kRing - 1))];
-                        atomicXor(n ? &ghost[site >> 5].y : &ghost[site >> 5].x, 1u << (site & 31));
-                    }
-                }
+            // both neighbours a word at a time, their loads in flight together
+            for (int w0 = A0 >> 5, w1 = A1 >> 5; w0 * 32 < lim0 || w1 * 32 < lim1; ++w0, ++w1) {
+                const int j0 = w0 * 32 + lane, j1 = w1 * 32 + lane;
+                const uint32_t a0 = nlog[w0 & (kLogWords - 1)], a1 = nlog[kLogWords + (w1 & (kLogWords - 1))];
+                const int s0 = ring[j0 & (kRing - 1)], s1 = ring[kRing + (j1 & (kRing - 1))];
+                if (j0 >= A0 && j0 < lim0 && ((a0 >> lane) & 1u)) atomicXor(&ghost[s0 >> 5].x, 1u << (s0 & 31));
+                if (j1 >= A1 && j1 < lim1 && ((a1 >> lane) & 1u)) atomicXor(&ghost[s1 >> 5].y, 1u << (s1 & 31));
             }
             A0 = max(A0, lim0);
             A1 = max(A1, lim1);
@@ -400,23 +406,26 @@ __global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const __
             nd0 = nd1 = -1;
             bool slow = A0 < 32 * (b - 2) || (nNbr > 1 && A1 < 32 * (b - 2));
             if (!valid) cand = kNoCands;
-            if (cand != kNoCands) {
-#pragma unroll
+            // the candidates not yet applied: bytes up to 32 p + 32 - A (few lanes have one)
+            const uint32_t m0 = min(g0 + 32 - A0, 96), m1 = min(g0 + 32 - A1, 96);
+            if (__vcmpleu4(cand, m0 | m0 << 8 | m1 << 16 | m1 << 24)) {
+#pragma unroll(kSmall ? 4 : 1)
                 for (int c = 0; c < 4; ++c) {
-                    const int n = c >> 1, v = (cand >> (8 * c)) & 0xff, j = g0 + 31 - v;
-                    if (v == (int)kManyCand) slow = true;
-                    if (v < (int)kManyCand && j >= (n ? A1 : A0)) {
-                        if (j < avail_of(av, n)) {
-                            const int f = (nlog[n * kLogWords + ((j >> 5) & (kLogWords - 1))] >> (j & 31)) & 1u;
-                            if (n)
-                                b1 ^= f;
-                            else
-                                b0 ^= f;
-                        } else if (n) {
+                    const int n = c >> 1, v = (cand >> (8 * c)) & 0xff, j = g0 + 32 - v;
+                    if (v == (int)kManyCand) {
+                        slow = true;
+                    } else if (v <= 96 && j >= (n ? A1 : A0)) {
+                        int f = 0;
+                        if (j < avail_of(av, n))
+                            f = (nlog[n * kLogWords + ((j >> 5) & (kLogWords - 1))] >> (j & 31)) & 1u;
+                        else if (n)
                             nd1 = max(nd1, j);
-                        } else {
+                        else
                             nd0 = max(nd0, j);
-                        }
+                        if (n)
+                            b1 ^= f;
+                        else
+                            b0 ^= f;
                     }
                 }
             }
@@ -445,36 +454,70 @@ __global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const __
             sum = (nd0 >= 0 ? 0 : 2 * b0 - 1) + (nd1 >= 0 ? 0 : 2 * b1 - 1);
         };
 
-        aborted = !wait_until(waitNs, [&] { return uniform_acquire(&S.readyTag[0]) == 1; });
-        x = pre[lane].x;
-        float Fv = Fs[x];
-
-        for (int b = 0; b < nBatches && !aborted; ++b) {
+        for (int b = 0; b < nBatches; ++b) {
             const int g0 = b * 32;
             const int buf = b & (kPre - 1);
             const int nValid = min(32, Itot - g0);
             const bool valid = lane < nValid;
-            const PreTrial tr = pre[buf * 32 + lane];
+
+            // this batch's trials, once its buffer is ready, and the published neighbour
+            // iterations before its first trial (their sites are in the ring once the buffer
+            // is ready; while it is not, those of earlier batches are applied, since the
+            // prefetchers may need their ring slots)
+            PreTrial tr;
+            unsigned long long av = 0, t0 = 0;
+            for (;;) {
+                const int tag = ld_acquire_cta(&S.readyTag[buf]);
+                tr = pre[buf * 32 + lane];
+                const bool ready = __shfl_sync(FULL, tag, 0) == b + 1;
+                if (nNbr > 0) av = apply_nbr(g0 + (ready ? before0 : 0), g0 + (ready ? before1 : 0));
+                if (ready) break;
+                if (t0 == 0) t0 = global_ns();
+                if (global_ns() - t0 > waitNs) {
+                    aborted = true;
+                    break;
+                }
+                __nanosleep(32);
+            }
+            if (aborted) break;
+            const int xN = tr.x;  // (0 beyond the last trial)
+
+            // The fields start from the resident row, which the updaters keep one batch
+            // behind, plus the previous batch's flips: a lone flip's coupling is fetched now
+            // and added after the neighbour work, several are added here in trial order.
+            const bool lone = accBits && !(accBits & (accBits - 1u));
+            float dLone = 0.f, gLone = 0.f;
+            if (lone) {
+                const int f = __ffs(accBits) - 1;
+                dLone = __shfl_sync(FULL, d, f);
+                gLone = __ldg(J + (size_t)__shfl_sync(FULL, x, f) * ldJ + xN);
+            }
+            if (b > 0) bar_sync(2, kBarCount);
+            float Fv = Fs[xN];
+            if (b > 0) {
+                if ((accBits >> lane) & 1u)
+                    flips[__popc(accBits & ((1u << lane) - 1u))] = make_int2(x, __float_as_int(d));
+                if (lane == 0) S.nflip = __popc(accBits);
+                __syncwarp();
+                __threadfence_block();
+                bar_arrive(1, kBarCount);
+            }
+            if (!lone)
+                for (unsigned rem = accBits; rem;) {
+                    // two at a time, their couplings in flight together
+                    const int f = __ffs(rem) - 1;
+                    rem &= rem - 1u;
+                    const int f2 = rem ? __ffs(rem) - 1 : f;
+                    const float j = __ldg(J + (size_t)__shfl_sync(FULL, x, f) * ldJ + xN);
+                    const float j2 = __ldg(J + (size_t)__shfl_sync(FULL, x, f2) * ldJ + xN);
+                    Fv = __fmaf_rn(__shfl_sync(FULL, d, f), j, Fv);
+                    if (rem) Fv = __fmaf_rn(__shfl_sync(FULL, d, f2), j2, Fv);
+                    rem &= rem - 1u;
+                }
+            x = xN;
             const float *jg = Jg + buf * kJgStride + lane * 33;
             const unsigned pred = prePred[buf];  // lanes whose row of in-batch gathers is in jg
             float qx = (float)qs[x];
-
-            // neighbour spins at this batch's sites: apply the published neighbour
-            // iterations before this batch's first trial (their sites are in the ring
-            // since this batch's buffer is ready); each lane's site is then corrected
-            int sum = 0;
-            nd0 = nd1 = -1;
-            if (nNbr > 0) {
-                const unsigned long long av = apply_nbr(g0 + before0, g0 + before1);
-                nbr_spins(b, g0, valid, tr.cand, av, sum);
-            }
-
-            // the previous batch's flips (gathered at the end of that batch)
-#pragma unroll
-            for (int t = 0; t < kGv; ++t) {
-                if (t >= nfPrev) break;
-                Fv = __fmaf_rn(__int_as_float(flips[t].y), gv[t], Fv);
-            }
 
             // The trial accepts when z = rate dE - L < 0.  z = zA - ring, zA = cz q (h + 2F) - L
             // and ring = cb q (qL + qR); unknown neighbour spins leave it in [z - sp, z + sp].
@@ -485,21 +528,31 @@ __global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const __
             // evaluations for unknown spins, took 970 cycles at two CTAs per SM; the decider is
             // the critical path, at 10 cycles an instruction.  N = 4096, m = 256, 64 steps: 24.2
             // ms before, 20.3 with this; N = 1000, m = 250: 8.0, 6.8.)
-            float zA, ring_, sp, tol;
             const float kF = fabsf(tr.cz) * 1.52587890625e-5f;
-            float c2 = 2.f * tr.cz * qx;
-            {
-                const float t = __fmaf_rn(2.f, Fv, tr.h), cbq = tr.cb * qx;
-                zA = __fmaf_rn(tr.cz * qx, t, -tr.L);
-                ring_ = cbq * (float)sum;
-                sp = fabsf(cbq) * (float)((nd0 >= 0) + (nd1 >= 0));
-                tol = __fmaf_rn(kF, fabsf(tr.h) + 2.f * fabsf(Fv) + 1.f, tr.tolC);
-            }
+            float c2 = 2.f * tr.cz * qx, ring_ = 0.f, sp = 0.f, zA, tol;
+            int sum = 0;
+            bool evalNbr = nNbr > 0;  // (one instance of nbr_spins: the loop's code stays small)
 
             // decide the batch in rounds
-            unsigned pending = __ballot_sync(FULL, valid), accBits = 0;
-            float d = 0.f;
+            unsigned pending = __ballot_sync(FULL, valid);
+            accBits = 0;
+            d = 0.f;
+            nd0 = nd1 = -1;
+            bool first = true;
             for (;;) {
+                if (evalNbr) {
+                    nbr_spins(b, g0, valid, tr.cand, av, sum);
+                    evalNbr = false;
+                    const float cbq = tr.cb * qx;
+                    ring_ = cbq * (float)sum;
+                    sp = fabsf(cbq) * (float)((nd0 >= 0) + (nd1 >= 0));
+                }
+                if (first) {
+                    if (lone) Fv = __fmaf_rn(dLone, gLone, Fv);
+                    zA = __fmaf_rn(tr.cz * qx, __fmaf_rn(2.f, Fv, tr.h), -tr.L);
+                    tol = __fmaf_rn(kF, fabsf(tr.h) + 2.f * fabsf(Fv) + 1.f, tr.tolC);
+                    first = false;
+                }
                 const float z = zA - ring_;
                 const unsigned accM = __ballot_sync(FULL, z + sp < -tol) & pending;
                 const unsigned blkM = __ballot_sync(FULL, z - sp <= tol) & pending & ~accM;
@@ -508,7 +561,7 @@ __global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const __
                 if (fb < fa) {
                     // undecided lanes below fb reject
                     pending &= ~((1u << fb) - 1u);
-                    if (lane == 0 && publish) st_relaxed_u64(outLog + (size_t)y * nWords + b, log_word(b, fb, accBits));
+                    if (lane == 0 && publish) st_relaxed_u64(myLog + b, log_word(b, fb, accBits));
                     const int w0 = __shfl_sync(FULL, nd0, fb), w1 = __shfl_sync(FULL, nd1, fb);
                     if (w0 < 0 && w1 < 0) {
                         // fb is too near its threshold: the exact warp decides its trial in FP64
@@ -517,12 +570,10 @@ __global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const __
                         // (The decider's arrival on a named barrier wakes the exact warp, which
                         // sleeps there between requests; the decider's wait is bounded.)
                         if (lane == fb) {
-                            const int sl = (g0 + lane) / N;
                             S.exX = x;
                             S.exQ = qx;
                             S.exU = tr.u;
-                            S.exG = T.G ? T.G[sl] : T.Gs;
-                            S.exBeta = T.beta ? T.beta[sl] : T.betas;
+                            S.exIter = g0 + lane;
                         }
                         ++exSeq;
                         __syncwarp();
@@ -536,7 +587,6 @@ __global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const __
                         continue;
                     }
                     // fb waits for its neighbour trials
-                    unsigned long long av = 0;
                     if (!wait_until(waitNs, [&] {
                             av = uniform_acquire64(&S.logAvail);
                             return avail_of(av, 0) > w0 && (nNbr < 2 || avail_of(av, 1) > w1);
@@ -544,11 +594,7 @@ __global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const __
                         aborted = true;
                         break;
                     }
-                    // evaluate again (the ghost rows and A are unchanged within the batch)
-                    nbr_spins(b, g0, valid, tr.cand, av, sum);
-                    const float cbq = tr.cb * qx;
-                    ring_ = cbq * (float)sum;
-                    sp = fabsf(cbq) * (float)((nd0 >= 0) + (nd1 >= 0));
+                    evalNbr = true;  // (the ghost rows and A are unchanged within the batch)
                     continue;
                 }
                 if (fa == 32) break;  // every undecided lane rejects
@@ -558,11 +604,11 @@ __global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const __
                 accBits |= 1u << fa;
                 pending &= ~((2u << fa) - 1u);
                 // trials through fa are decided: make them visible to the neighbours
-                if (lane == 0 && pending && publish) st_relaxed_u64(outLog + (size_t)y * nWords + b, log_word(b, fa + 1, accBits));
+                if (lane == 0 && pending && publish) st_relaxed_u64(myLog + b, log_word(b, fa + 1, accBits));
                 if (lane == fa) {
                     qs[x] = (int8_t)(qx > 0.f ? -1 : 1);
                     d = df;
-                    if (T.trace) {
+                    if (traced) {
                         const int s = (g0 + lane) / N, k = g0 + lane - s * N;
                         uint32_t bitIdx = (uint32_t)k * (uint32_t)m + (uint32_t)y;
                         atomicOr(&T.trace[(size_t)s * wordsPerStep + (bitIdx >> 5)], 1u << (bitIdx & 31));
@@ -570,7 +616,7 @@ __global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const __
                 }
                 if (!pending) break;
                 if (lane > fa) {
-                    const float dJ = df * (((pred >> fa) & 1u) ? jg[fa] : __ldg(T.J + (size_t)xf * T.ldJ + x));
+                    const float dJ = df * (((pred >> fa) & 1u) ? jg[fa] : __ldg(J + (size_t)xf * ldJ + x));
                     zA = __fmaf_rn(c2, dJ, zA);
                     tol = __fmaf_rn(2.f * kF, fabsf(dJ), tol);
                     if (x == xf) {
@@ -585,61 +631,17 @@ __global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const __
             __syncwarp();
             if (lane == 0) {
                 S.decDone = b + 1;  // this batch's buffer is free
-                if (publish) st_relaxed_u64(outLog + (size_t)y * nWords + b, log_word(b, nValid, accBits));
+                if (publish) st_relaxed_u64(myLog + b, log_word(b, nValid, accBits));
             }
-            const int nf = __popc(accBits);
-            accepted += (unsigned long long)nf;
-
-            // the next batch's sites
-            const bool more = b + 1 < nBatches;
-            // (while waiting, keep applying published neighbour iterations of this and
-            // earlier batches: the prefetchers may need those ring slots)
-            if (more && !wait_until(waitNs, [&] {
-                    if (uniform_acquire(&S.readyTag[(b + 1) & (kPre - 1)]) == b + 2) return true;
-                    if (nNbr > 0) apply_nbr(g0 + 32, g0 + 32);
-                    return false;
-                })) {
-                aborted = true;
-                break;
-            }
-            const int xN = more ? pre[((b + 1) & (kPre - 1)) * 32 + lane].x : 0;
-            // the next batch's fields start from the resident row once the updaters
-            // are done with the previous batch's flips; this batch's flips are
-            // gathered now and added after the next batch's neighbour work
-            // (lanes beyond the last trial have site 0)
-            const bool defer = nf <= kGv;
-            if (defer && accBits) {
-                unsigned rem = accBits;
-#pragma unroll
-                for (int t = 0; t < kGv; ++t) {
-                    const int xf = __shfl_sync(FULL, x, __ffs(rem) - 1);
-                    gv[t] = __ldg(T.J + (size_t)xf * T.ldJ + xN);
-                    rem &= rem - 1u;
-                    if (!rem) break;
-                }
-            }
-            bar_sync(2, kBarCount);
-            float FvN = Fs[xN];
-            if ((accBits >> lane) & 1u) flips[__popc(accBits & ((1u << lane) - 1u))] = make_int2(x, __float_as_int(d));
-            if (lane == 0) S.nflip = nf;
-            __syncwarp();
-            __threadfence_block();
-            bar_arrive(1, kBarCount);
-            nfPrev = defer ? nf : 0;
-            if (!defer) {
-                // many flips: add them all now, in trial order
-                unsigned rem = accBits;
-                while (rem) {
-                    const int f = __ffs(rem) - 1;
-                    rem &= rem - 1u;
-                    const int xf = __shfl_sync(FULL, x, f);
-                    const float df = __shfl_sync(FULL, d, f);
-                    FvN = __fmaf_rn(df, __ldg(T.J + (size_t)xf * T.ldJ + xN), FvN);
-                }
-            }
-            x = xN;
-            Fv = FvN;
+            accepted += (unsigned long long)__popc(accBits);
         }
+        // the last batch's flips, as at the head of the next
+        bar_sync(2, kBarCount);
+        if ((accBits >> lane) & 1u) flips[__popc(accBits & ((1u << lane) - 1u))] = make_int2(x, __float_as_int(d));
+        if (lane == 0) S.nflip = __popc(accBits);
+        __syncwarp();
+        __threadfence_block();
+        bar_arrive(1, kBarCount);
         bar_sync(2, kBarCount);  // the updaters are done with the last flips
         if (lane == 0) {
             if (aborted && T.status) atomicExch(T.status, (int)kErrTimeout);
@@ -699,7 +701,9 @@ __global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const __
             bar_sync(kBarExReq, 64);
             if (S.done) break;
             const int xr = S.exX;
-            const float qr = S.exQ, ur = S.exU, Gr = S.exG, br = S.exBeta;
+            const float qr = S.exQ, ur = S.exU;
+            const int sl = S.exIter / N;
+            const float Gr = T.G ? T.G[sl] : T.Gs, br = T.beta ? T.beta[sl] : T.betas;
             const double hr = T.h64 ? T.h64[xr] : (double)hs[xr];
             const double F = T.J64 ? exact_field_warp(T.J64 + (size_t)xr * N, qs, N)
                                    : exact_field_warp(T.J + (size_t)xr * T.ldJ, qs, N);
@@ -789,8 +793,8 @@ __global__ void __launch_bounds__(kMcThreads, kPerSm) dense_sweep_multi(const __
             // the lane's site up to its limit (-2: more than kCand)
             uint32_t cands = kNoCands;
             auto put_cands = [&](int nn, int c0, int c1) {
-                const uint32_t e0 = c0 == -2 ? kManyCand : c0 < 0 ? kNoCand : (uint32_t)(32 * p + 31 - c0);
-                const uint32_t e1 = c1 < 0 ? kNoCand : (uint32_t)(32 * p + 31 - c1);
+                const uint32_t e0 = c0 == -2 ? kManyCand : c0 < 0 ? kNoCand : (uint32_t)(32 * p + 32 - c0);
+                const uint32_t e1 = c1 < 0 ? kNoCand : (uint32_t)(32 * p + 32 - c1);
                 cands = nn ? (cands & 0xffffu) | (e0 << 16) | (e1 << 24) : (cands & 0xffff0000u) | e0 | (e1 << 8);
             };
             if (nNbr > 0) {
@@ -1023,14 +1027,18 @@ static size_t multi_smem_bytes(int N) {
            32 * 8 + (size_t)((N + 15) & ~15) + 16 + (N <= kSmallN ? (size_t)kPf * kSmallN * 4 : 0);
 }
 
-// every instance, by kHooks, kSmall (bits 0, 1) and register allotment (2 or 4 CTAs per SM)
-static const void *multi_kernel(bool hooks, bool small, int perSm) {
-    static const void *const k[2][4] = {
-        {(const void *)dense_sweep_multi<false, false, 2>, (const void *)dense_sweep_multi<true, false, 2>,
-         (const void *)dense_sweep_multi<false, true, 2>, (const void *)dense_sweep_multi<true, true, 2>},
-        {(const void *)dense_sweep_multi<false, false, 4>, (const void *)dense_sweep_multi<true, false, 4>,
-         (const void *)dense_sweep_multi<false, true, 4>, (const void *)dense_sweep_multi<true, true, 4>}};
-    return k[perSm > 2][(hooks ? 1 : 0) + (small ? 2 : 0)];
+// every instance: bit 0 kHooks, bit 1 kSmall, bit 2 kSA, bit 3 four CTAs per SM (else two)
+template <int I>
+static const void *multi_instance() {
+    return (const void *)dense_sweep_multi<(I & 1) != 0, (I & 2) != 0, (I & 4) != 0, (I & 8) ? 4 : 2>;
+}
+static const void *multi_kernel(int i) {
+    static const void *const k[16] = {
+        multi_instance<0>(),  multi_instance<1>(),  multi_instance<2>(),  multi_instance<3>(),
+        multi_instance<4>(),  multi_instance<5>(),  multi_instance<6>(),  multi_instance<7>(),
+        multi_instance<8>(),  multi_instance<9>(),  multi_instance<10>(), multi_instance<11>(),
+        multi_instance<12>(), multi_instance<13>(), multi_instance<14>(), multi_instance<15>()};
+    return k[i];
 }
 
 // resident CTAs of rows of N spins, with the registers allotted for two and for four per SM
@@ -1051,19 +1059,19 @@ static MultiCapacity multi_capacity(int N) {
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     const size_t smem = multi_smem_bytes(N);
     cudaFuncAttributes fa;
-    cudaFuncGetAttributes(&fa, multi_kernel(false, false, 2));
+    cudaFuncGetAttributes(&fa, multi_kernel(0));
     if (smem + fa.sharedSizeBytes > (size_t)optin) return {0, 0};
     // every instance: the launch takes the one the tasks' flags and sizes ask for
     int perSm[2] = {1 << 30, 1 << 30};
-    for (int i = 0; i < 8; ++i) {
-        const void *k = multi_kernel(i & 1, i & 2, i & 4 ? 4 : 2);
+    for (int i = 0; i < 16; ++i) {
+        const void *k = multi_kernel(i);
         int ps = 0;
         if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ps, k, kMcThreads, smem) != cudaSuccess) {
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ps, k, mc_threads(i & 8 ? 4 : 2), smem) != cudaSuccess) {
             cudaGetLastError();
             return {0, 0};
         }
-        perSm[i >> 2] = std::min(perSm[i >> 2], ps);
+        perSm[i >> 3] = std::min(perSm[i >> 3], ps);
     }
     cachedN = N;
     cached = {perSm[0] * sms, std::max(perSm[0], perSm[1]) * sms};
@@ -1095,9 +1103,11 @@ static int launch_pack(const sq103_dense_task *tasks, int n, void *stream) {
     P.n = n;
     int maxN = 0, ctas = 0;
     bool hooks = false;
+    int sas = 0;
     for (int i = 0; i < n; ++i) {
         const sq103_dense_task &t = tasks[i];
-        hooks |= (t.flags & (kFlagShortWaits | kFlagWithholdTrotter0)) != 0;
+        hooks |= (t.flags & (kFlagShortWaits | kFlagWithholdTrotter0)) != 0 || t.trace;
+        sas += t.algo == kSANaive;
         const int N = t.N, m = t.m;
         if (t.algo != kColoring && t.algo != kSANaive) return kErrBadShape;
         if (N < 64 || m < 2 || t.nSteps < 1) return kErrBadShape;
@@ -1112,13 +1122,19 @@ static int launch_pack(const sq103_dense_task *tasks, int n, void *stream) {
         ctas += m;
         maxN = std::max(maxN, N);
     }
+    if (sas && sas < n) {  // one algorithm per launch
+        std::vector<sq103_dense_task> part[2];
+        for (int i = 0; i < n; ++i) part[tasks[i].algo == kSANaive].push_back(tasks[i]);
+        const int rc = launch_pack(part[0].data(), (int)part[0].size(), stream);
+        return rc != 0 ? rc : launch_pack(part[1].data(), (int)part[1].size(), stream);
+    }
     for (int i = n; i <= kMaxPack; ++i) P.base[i] = ctas;
     // every CTA resident at once (cooperative launch); also sets the kernel's shared-memory limit
     const MultiCapacity cap = multi_capacity(maxN);
     if (cap.four < ctas) return kErrCapacity;
     void *args[] = {&P};
-    const void *kernel = multi_kernel(hooks, maxN <= kSmallN, ctas <= cap.two ? 2 : 4);
-    return (int)cudaLaunchCooperativeKernel(kernel, dim3(ctas), dim3(kMcThreads), args, multi_smem_bytes(maxN), st);
+    const void *kernel = multi_kernel((hooks ? 1 : 0) | (maxN <= kSmallN ? 2 : 0) | (sas ? 4 : 0) | (ctas <= cap.two ? 0 : 8));
+    return (int)cudaLaunchCooperativeKernel(kernel, dim3(ctas), dim3(mc_threads(ctas <= cap.two ? 2 : 4)), args, multi_smem_bytes(maxN), st);
 }
 
 // launched from sq103_dense_anneal (dense.cu) when the shape and workspace allow it
