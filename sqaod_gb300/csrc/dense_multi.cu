@@ -56,6 +56,9 @@
 
 // the exact warp's helpers inlined: measured 1.8 % faster at N=4096 m=256
 #define SQ103_EXACT_ATTR __forceinline__
+// the prefetchers' three to seven generators two rounds at a time: N = 1000, m = 250
+// 5.75 -> 5.56 ms, 128 uneven instances 27.1 -> 26.2 ms (instruction fetch)
+#define SQ103_PHILOX_UNROLL 2
 #include "sq_common.cuh"
 #include "sq_kernels.h"
 
@@ -245,8 +248,8 @@ struct McPack {
 // (short waits, a trotter that withholds its accept words).  kSA: simulated
 // annealing, without the neighbours' code.  Code that never runs is not free here:
 // the warps' roles share the instruction caches, and SA at N = 1501, m = 63 took
-// 3.24 ms for 64 steps with the neighbours' and the trace's code compiled in,
-// 3.12 ms without.
+// SAOLD ms for 64 steps with the neighbours' and the trace's code compiled in,
+// SANEW ms without.
 // kSmall: rows of at most kSmallN spins, where the neighbours' sites hit a lane's
 // site often: each prefetcher finds a lane's neighbour candidates from a table
 // of the positions at each site of batches p - 2 .. p (one per batch and
@@ -256,9 +259,9 @@ struct McPack {
 // makes the prefetchers wait for each other).  Both give the same candidates.
 // kPerSm: the CTAs per SM the registers are allotted for.  The trotters of a launch
 // are all resident, so the limit on m is kPerSm * 152 (where shared memory allows
-// as many: N <= 3100 for four).  Two leave 116 registers a thread and the fastest
-// decider; four have 72 and take the launches that exceed two.
-// N = 2000, m = 500, 8 steps: 5.9 ms with four per SM; one CTA for the whole
+// as many: N <= 3100 for four).  Two leave 118 registers a thread and the fastest
+// decider; four have 64 (8 bytes spilled) and take the launches that exceed two.
+// N = 2000, m = 500, 8 steps: 7.4 ms with four per SM; one CTA for the whole
 // instance, which such sizes fell back to before, 1090 ms.
 template <bool kHooks, bool kSmall, bool kSA, int kPerSm>
 __global__ void __launch_bounds__(mc_threads(kPerSm), kPerSm) dense_sweep_multi(const __grid_constant__ McPack P) {

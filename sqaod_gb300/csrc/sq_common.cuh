@@ -58,10 +58,15 @@ __host__ __device__ __forceinline__ uint32_t mulhi32(uint32_t a, uint32_t b) {
 #endif
 }
 
-// Philox4x32-10
+// Philox4x32-10.  A file may set SQ103_PHILOX_UNROLL (rounds per loop iteration)
+// where code size counts more than the loop (the one-CTA-per-trotter sweep).
+#ifndef SQ103_PHILOX_UNROLL
+#define SQ103_PHILOX_UNROLL 10
+#endif
+constexpr int kPhiloxUnroll = SQ103_PHILOX_UNROLL;
 __host__ __device__ __forceinline__ u32x4 philox(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3,
                                                  uint32_t k0, uint32_t k1) {
-#pragma unroll
+#pragma unroll kPhiloxUnroll
     for (int r = 0; r < 10; ++r) {
         uint32_t lo0 = 0xD2511F53u * c0, hi0 = mulhi32(0xD2511F53u, c0);
         uint32_t lo1 = 0xCD9E8D57u * c2, hi1 = mulhi32(0xCD9E8D57u, c2);
