@@ -39,22 +39,37 @@ namespace sq = sqaod;
 
 // Exact W == W^T on the device (the host check of sqaodc/common/Common.cpp:97-104,
 // `!=` per element pair): each 32 x 32 tile on or below the diagonal is
-// compared with its mirror tile, staged transposed in shared memory.
-__global__ void sym_check_kernel(const float *W, int N, int ld, int *bad) {
-    __shared__ float t[32][33];
+// compared with its mirror tile, staged transposed in shared memory.  `diagonal`:
+// a diagonal value that differs from itself (a NaN) counts as a mismatch too.
+template <class real>
+__global__ void sym_check_kernel(const real *W, int N, int ld, bool diagonal, int *bad) {
+    __shared__ real t[32][33];
     const int bx = blockIdx.x, by = blockIdx.y, tx = threadIdx.x, ty = threadIdx.y;
     if (bx > by) return;
     for (int j = ty; j < 32; j += 8) {
         const int r = bx * 32 + j, c = by * 32 + tx;
-        t[j][tx] = (r < N && c < N) ? W[(size_t)r * ld + c] : 0.f;
+        t[j][tx] = (r < N && c < N) ? W[(size_t)r * ld + c] : (real)0;
     }
     __syncthreads();
     int mismatch = 0;
     for (int j = ty; j < 32; j += 8) {
         const int r = by * 32 + j, c = bx * 32 + tx;
-        if (r < N && c < N && W[(size_t)r * ld + c] != t[tx][j]) mismatch = 1;
+        if (r < N && c < N && (diagonal || r != c) && W[(size_t)r * ld + c] != t[tx][j]) mismatch = 1;
     }
     if (__syncthreads_or(mismatch) && tx == 0 && ty == 0) atomicOr(bad, 1);
+}
+
+template <class real>
+static bool device_symmetric(const real *dW, int N, int ld, bool diagonal, DevBuf<int> &flag, Stream &st) {
+    flag.ensure(1);
+    SQ_CHECK(cudaMemsetAsync(flag.p, 0, sizeof(int), st.get()));
+    const int nT = (N + 31) / 32;
+    sym_check_kernel<<<dim3(nT, nT), dim3(32, 8), 0, st.get()>>>(dW, N, ld, diagonal, flag.p);
+    SQ_CHECK(cudaGetLastError());
+    int bad = 0;
+    SQ_CHECK(cudaMemcpyAsync(&bad, flag.p, sizeof(int), cudaMemcpyDeviceToHost, st.get()));
+    st.sync();
+    return bad == 0;
 }
 
 // dst (rows x cols, row stride ldd) = fp32 rounding of src (row stride lds): the
@@ -226,7 +241,7 @@ public:
         DevBuf<float> dW;
         dW.ensure((size_t)N * N);
         upload(dW.p, N, W);
-        throwErrorIf(!deviceSymmetric(dW.p, N, N), "%s, Matrix is not symmetric.", __func__);
+        throwErrorIf(!device_symmetric(dW.p, N, N, true, d_flag_, st_), "%s, Matrix is not symmetric.", __func__);
         clearState(solProblemSet);
         N_ = N;
         m_ = N_ / 4;
@@ -238,18 +253,6 @@ public:
         st_.sync();
         dropFP64();
         setState(solProblemSet);
-    }
-
-    bool deviceSymmetric(const float *dW, int N, int ld) {
-        d_flag_.ensure(1);
-        SQ_CHECK(cudaMemsetAsync(d_flag_.p, 0, sizeof(int), st_.get()));
-        const int nT = (N + 31) / 32;
-        sym_check_kernel<<<dim3(nT, nT), dim3(32, 8), 0, st_.get()>>>(dW, N, ld, d_flag_.p);
-        SQ_CHECK(cudaGetLastError());
-        int bad = 0;
-        SQ_CHECK(cudaMemcpyAsync(&bad, d_flag_.p, sizeof(int), cudaMemcpyDeviceToHost, st_.get()));
-        st_.sync();
-        return bad == 0;
     }
 
     void setHamiltonian(const Vector &h, const Matrix &J, float c) override {
@@ -362,8 +365,8 @@ public:
     void makeSolution() override {
         throwErrorIfQNotSet();
         syncBits();
-        setState(solSolutionAvailable);
         calculate_E();
+        solverState_ |= solSolutionAvailable;  // (setState would clear the energies just computed)
     }
 
     float getSystemE(float G, float beta) const override {
@@ -905,8 +908,8 @@ public:
         throwErrorIfNotPrepared();
         throwErrorIfQNotSet();
         syncBits();
-        setState(solSolutionAvailable);
         calculate_E();
+        solverState_ |= solSolutionAvailable;  // (setState would clear the energies just computed)
     }
 
     float getSystemE(float G, float beta) const override {
@@ -2396,31 +2399,28 @@ public:
     // E[i] = x_i W x_i^T for the m rows of x (int8 bits, row stride N)
     void quboEnergies(const real *W, int ldW, int N, const int8_t *x, int m, double *E) {
         check_shape(N, m, __func__);
-        throwErrorIf(!sq::isSymmetric(W, (size_t)N, (size_t)ldW), "%s, Matrix is not symmetric.", __func__);
+        uploadSymmetric(dJ_, W, ldW, N, __func__);
         check_values(x, (size_t)m * N, false, __func__);
-        energies(W, ldW, nullptr, 0.0, N, x, m, /*maximize*/ true, E);
+        energies(nullptr, 0.0, N, x, m, /*maximize*/ true, E);
     }
 
     // E[i] = -c - h q_i^T - q_i J q_i^T (int8 spins)
     void isingEnergies(const real *h, const real *J, int ldJ, real c, int N, const int8_t *q, int m, double *E) {
         check_shape(N, m, __func__);
-        throwErrorIf(!sq::isSymmetric(J, (size_t)N, (size_t)ldJ), "%s, Matrix is not symmetric.", __func__);
+        uploadSymmetric(dJ_, J, ldJ, N, __func__);
         check_values(q, (size_t)m * N, true, __func__);
-        energies(J, ldJ, h, (double)c, N, q, m, false, E);
+        energies(h, (double)c, N, q, m, false, E);
     }
 
     void hamiltonian(const real *W, int ldW, int N, real *h, real *J, real *c) {
         check_shape(N, 1, __func__);
-        throwErrorIf(!sq::isSymmetric(W, (size_t)N, (size_t)ldW), "%s, Matrix is not symmetric.", __func__);
+        uploadSymmetric(dW_, W, ldW, N, __func__);
         cudaStream_t s = st_.get();
-        dW_.ensure((size_t)N * N);
         dh_.ensure(N);
         dJ_.ensure((size_t)N * N);
         dc_.ensure(1);
         dc64_.ensure(1);
         dscr_.ensure(N);
-        SQ_CHECK(cudaMemcpy2DAsync(dW_.p, sizeof(real) * N, W, sizeof(real) * ldW, sizeof(real) * N, N,
-                                   cudaMemcpyHostToDevice, s));
         if constexpr (kF64)
             SQ_CHECK(sq103_dense_hamiltonian64(dW_.p, N, dh_.p, dJ_.p, dc_.p, dscr_.p, s));
         else
@@ -2484,15 +2484,19 @@ private:
         throwErrorIf(N <= 0 || m <= 0, "%s, Shape does not match.", fn);
     }
 
-    // sign * (-c - h q^T - q J q^T) of every row, h = 0 when null
-    void energies(const real *J, int ldJ, const real *h, double c, int N, const int8_t *q, int m, bool maximize,
-                  double *E) {
+    // the N x N matrix M into d, checked for exact symmetry there
+    void uploadSymmetric(DevBuf<real> &d, const real *M, int ld, int N, const char *fn) {
+        d.ensure((size_t)N * N);
+        SQ_CHECK(cudaMemcpy2DAsync(d.p, sizeof(real) * N, M, sizeof(real) * ld, sizeof(real) * N, N,
+                                   cudaMemcpyHostToDevice, st_.get()));
+        throwErrorIf(!device_symmetric(d.p, N, N, false, dflag_, st_), "%s, Matrix is not symmetric.", fn);
+    }
+
+    // sign * (-c - h q^T - q J q^T) of every row, J uploaded to dJ_, h = 0 when null
+    void energies(const real *h, double c, int N, const int8_t *q, int m, bool maximize, double *E) {
         cudaStream_t s = st_.get();
-        dJ_.ensure((size_t)N * N);
         dh_.ensure(N);
         dc64_.ensure(1);
-        SQ_CHECK(cudaMemcpy2DAsync(dJ_.p, sizeof(real) * N, J, sizeof(real) * ldJ, sizeof(real) * N, N,
-                                   cudaMemcpyHostToDevice, s));
         if (h)
             SQ_CHECK(cudaMemcpyAsync(dh_.p, h, sizeof(real) * N, cudaMemcpyHostToDevice, s));
         else
@@ -2516,6 +2520,7 @@ private:
     }
 
     Stream st_;
+    DevBuf<int> dflag_;
     DevBuf<real> dW_, dh_, dJ_, dc_;
     DevBuf<double> dc64_, dscr_, dr_, dE_;
     DevBuf<int8_t> dq_;

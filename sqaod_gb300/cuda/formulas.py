@@ -152,10 +152,10 @@ def dense_graph_batch_calculate_E(W, x, dtype):
     dtype = _check_dtype(dtype)
     W = common.fix_type(W, dtype)
     _square('W', W)
-    W = common.symmetrize(W)
     x = _dense_rows(W, common.fix_type(x, np.int8), 'W, x')
     E = np.empty(x.shape[0], np.float64)
-    _dg(dtype)('calculate_E', ptr(W), _c_int(W.shape[0]), ptr(x), _c_int(x.shape[0]), ptr(E))
+    common.submit_symmetric(W, dtype, lambda W: _dg(dtype)('calculate_E', ptr(W), _c_int(W.shape[0]), ptr(x),
+                                                           _c_int(x.shape[0]), ptr(E)))
     return E.astype(dtype)
 
 
@@ -164,12 +164,12 @@ def dense_graph_calculate_hamiltonian(W, dtype):
     dtype = _check_dtype(dtype)
     W = common.fix_type(W, dtype)
     _square('W', W)
-    W = common.symmetrize(W)
     N = W.shape[0]
     h = np.empty(N, dtype)
     J = np.empty((N, N), dtype)
     c = np.empty(1, dtype)
-    _dg(dtype)('calculate_hamiltonian', ptr(W), _c_int(N), ptr(h), ptr(J), ptr(c))
+    common.submit_symmetric(W, dtype, lambda W: _dg(dtype)('calculate_hamiltonian', ptr(W), _c_int(N), ptr(h), ptr(J),
+                                                           ptr(c)))
     return h, J, c[0]
 
 
@@ -184,14 +184,14 @@ def dense_graph_batch_calculate_E_from_spin(h, J, c, q, dtype):
     h, J = common.fix_type([h, J], dtype)
     _vector('h', h)
     _square('J', J)
-    J = common.symmetrize(J)
     _scalar('c', c)
     if h.shape[0] != J.shape[0]:
         _dims('h, J', h, J)
     q = _dense_rows(J, q, 'J, q')
     E = np.empty(q.shape[0], np.float64)
-    _dg(dtype)('calculate_E_from_spin', ptr(h), ptr(J), _real(dtype)(float(c)), _c_int(J.shape[0]),
-               ptr(q), _c_int(q.shape[0]), ptr(E))
+    common.submit_symmetric(J, dtype, lambda J: _dg(dtype)('calculate_E_from_spin', ptr(h), ptr(J),
+                                                           _real(dtype)(float(c)), _c_int(J.shape[0]), ptr(q),
+                                                           _c_int(q.shape[0]), ptr(E)))
     return E.astype(dtype)
 
 
