@@ -102,10 +102,13 @@ __device__ __forceinline__ unsigned long long global_ns() {
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
+// bar.sync and bar.arrive count whole warps: the lanes meet first
 __device__ __forceinline__ void bar_sync(int id, int n) {
+    __syncwarp();
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
 }
 __device__ __forceinline__ void bar_arrive(int id, int n) {
+    __syncwarp();
     asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory");
 }
 __device__ __forceinline__ unsigned smem_addr(const volatile void *p) {
@@ -472,7 +475,9 @@ __global__ void __launch_bounds__(mc_threads(kPerSm), kPerSm) dense_sweep_multi(
             for (;;) {
                 const int tag = ld_acquire_cta(&S.readyTag[buf]);
                 tr = pre[buf * 32 + lane];
-                const bool ready = __shfl_sync(FULL, tag, 0) == b + 1;
+                // every lane's own tag: lanes may run apart here (lane 0 has just published), and
+                // a lane's trial is valid only if its own load followed the tag
+                const bool ready = __all_sync(FULL, tag == b + 1);
                 if (nNbr > 0) av = apply_nbr(g0 + (ready ? before0 : 0), g0 + (ready ? before1 : 0));
                 if (ready) break;
                 if (t0 == 0) t0 = global_ns();
