@@ -85,7 +85,7 @@ constexpr unsigned long long kWaitLimitNs = 4000000000ull;
 constexpr unsigned long long kShortWaitNs = 1000000ull;  // task flag kFlagShortWaits (tests)
 // the prefetchers run ahead and mostly wait: they poll gently, which leaves the
 // SM's shared load/store path to the decider
-constexpr int kPrefetchSleepNs = 128;
+constexpr int kPrefetchSleepNs = 32;
 constexpr unsigned FULL = 0xffffffffu;
 constexpr int kSmallN = 1024;  // rows up to this many spins take the kSmall instance (measured: 1024 faster, 2048 slower)
 
@@ -102,7 +102,8 @@ __device__ __forceinline__ unsigned long long global_ns() {
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
-// bar.sync and bar.arrive count whole warps: the lanes meet first
+// bar.sync and bar.arrive count whole warps: a warp whose lanes reach one apart would
+// count more than once and let the other side run early, so the lanes meet first
 __device__ __forceinline__ void bar_sync(int id, int n) {
     __syncwarp();
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
@@ -163,6 +164,7 @@ struct McShared {
     volatile unsigned long long logAvail;  // neighbour accept bits known below (lo: neighbour 0, hi: 1) (helper)
     volatile int applied[2];               // neighbour iterations applied to the ghost rows (decider)
     volatile int readyTag[kPre];           // p + 1 once buffer p % kPre holds batch p (prefetchers)
+    volatile int ringTag[kPre];            // p + 1 once the neighbours' sites of batch p are in the ring (prefetchers)
     volatile int decDone;                  // batches [0, decDone) no longer read from the buffers (decider)
     volatile int done;
     int nflip;
@@ -324,28 +326,33 @@ __global__ void __launch_bounds__(mc_threads(kPerSm), kPerSm) dense_sweep_multi(
     unsigned *prePred = reinterpret_cast<unsigned *>(nlog + 2 * kLogWords);  // kPre
     int2 *flips = reinterpret_cast<int2 *>(prePred + kPre);             // 32
     int8_t *qs = reinterpret_cast<int8_t *>(flips + 32);                // N
-    // kSmall: one site table of kSmallN words per prefetcher (positions of a batch by site)
+    // kSmall: two site tables of kSmallN words per prefetcher (positions of a batch by site, one per neighbour)
     uint32_t *siteTab = reinterpret_cast<uint32_t *>(qs + ((N + 15) & ~15));
 
+    for (int i = tid; i < kPre * 32; i += kMcThreads) pre[i].x = 0;  // (read before the first batch is ready)
     if (kSmall)
-        for (int i = tid; i < kPf * kSmallN; i += kMcThreads) siteTab[i] = 0u;
+        for (int i = tid; i < kPf * 2 * kSmallN; i += kMcThreads) siteTab[i] = 0u;
     for (int i = tid; i < N; i += kMcThreads) {
         Fs[i] = T.F[(size_t)y * N + i];
         hs[i] = T.h[i];
         qs[i] = T.q[(size_t)y * N + i];
     }
+    // a word of a neighbour's spin bits per warp and turn (a thread per word, 32 byte loads
+    // after one another, took most of a short launch: N = 128, m = 16, one step, 22.0 us a
+    // call before, 19.9 with this)
     for (int n = 0; n < nNbr; ++n) {
         const int8_t *qn = T.q + (size_t)(n ? nbr1 : nbr0) * N;
-        for (int w = tid; w < nWG; w += kMcThreads) {
-            uint32_t bits = 0;
-            for (int b = 0; b < 32 && w * 32 + b < N; ++b) bits |= (qn[w * 32 + b] > 0 ? 1u : 0u) << b;
-            (n ? ghost[w].y : ghost[w].x) = bits;
+#pragma unroll 4
+        for (int w = warp; w < nWG; w += kMcThreads / 32) {
+            const int i = w * 32 + lane;
+            const uint32_t bits = __ballot_sync(FULL, i < N && qn[i] > 0);
+            if (lane == 0) (n ? ghost[w].y : ghost[w].x) = bits;
         }
     }
     if (tid == 0) {
         S.logAvail = 0;
         S.applied[0] = S.applied[1] = 0;
-        for (int i = 0; i < kPre; ++i) S.readyTag[i] = 0;
+        for (int i = 0; i < kPre; ++i) S.readyTag[i] = S.ringTag[i] = 0;
         S.decDone = 0;
         S.exDone = 0;
         S.done = 0;
@@ -470,14 +477,41 @@ __global__ void __launch_bounds__(mc_threads(kPerSm), kPerSm) dense_sweep_multi(
             // iterations before its first trial (their sites are in the ring once the buffer
             // is ready; while it is not, those of earlier batches are applied, since the
             // prefetchers may need their ring slots)
+            // The loads of the trial's site, and the flips handed to the updaters, come before
+            // the ghost rows' work, which hides their latency.
+            // The fields start from the resident row, which the updaters keep one batch
+            // behind, plus the previous batch's flips: a lone flip's coupling is fetched here
+            // and added after the neighbour work, several are added below in trial order.
+            const bool lone = accBits && !(accBits & (accBits - 1u));
             PreTrial tr;
             unsigned long long av = 0, t0 = 0;
+            unsigned pred = 0;  // lanes whose row of in-batch gathers is in jg
+            float qx = 0.f, Fv = 0.f, dLone = 0.f, gLone = 0.f;
             for (;;) {
                 const int tag = ld_acquire_cta(&S.readyTag[buf]);
-                tr = pre[buf * 32 + lane];
+                tr = pre[buf * 32 + lane];  // (site 0 beyond the last trial)
                 // every lane's own tag: lanes may run apart here (lane 0 has just published), and
                 // a lane's trial is valid only if its own load followed the tag
                 const bool ready = __all_sync(FULL, tag == b + 1);
+                if (ready) {
+                    pred = prePred[buf];
+                    qx = (float)qs[tr.x];
+                    if (lone) {
+                        const int f = __ffs(accBits) - 1;
+                        dLone = __shfl_sync(FULL, d, f);
+                        gLone = __ldg(J + (size_t)__shfl_sync(FULL, x, f) * ldJ + tr.x);
+                    }
+                    if (b > 0) bar_sync(2, kBarCount);
+                    Fv = Fs[tr.x];
+                    if (b > 0) {
+                        if ((accBits >> lane) & 1u)
+                            flips[__popc(accBits & ((1u << lane) - 1u))] = make_int2(x, __float_as_int(d));
+                        if (lane == 0) S.nflip = __popc(accBits);
+                        __syncwarp();
+                        __threadfence_block();
+                        bar_arrive(1, kBarCount);
+                    }
+                }
                 if (nNbr > 0) av = apply_nbr(g0 + (ready ? before0 : 0), g0 + (ready ? before1 : 0));
                 if (ready) break;
                 if (t0 == 0) t0 = global_ns();
@@ -488,44 +522,23 @@ __global__ void __launch_bounds__(mc_threads(kPerSm), kPerSm) dense_sweep_multi(
                 __nanosleep(32);
             }
             if (aborted) break;
-            const int xN = tr.x;  // (0 beyond the last trial)
-
-            // The fields start from the resident row, which the updaters keep one batch
-            // behind, plus the previous batch's flips: a lone flip's coupling is fetched now
-            // and added after the neighbour work, several are added here in trial order.
-            const bool lone = accBits && !(accBits & (accBits - 1u));
-            float dLone = 0.f, gLone = 0.f;
-            if (lone) {
-                const int f = __ffs(accBits) - 1;
-                dLone = __shfl_sync(FULL, d, f);
-                gLone = __ldg(J + (size_t)__shfl_sync(FULL, x, f) * ldJ + xN);
-            }
-            if (b > 0) bar_sync(2, kBarCount);
-            float Fv = Fs[xN];
-            if (b > 0) {
-                if ((accBits >> lane) & 1u)
-                    flips[__popc(accBits & ((1u << lane) - 1u))] = make_int2(x, __float_as_int(d));
-                if (lane == 0) S.nflip = __popc(accBits);
-                __syncwarp();
-                __threadfence_block();
-                bar_arrive(1, kBarCount);
-            }
+            const int xN = tr.x;
             if (!lone)
                 for (unsigned rem = accBits; rem;) {
-                    // two at a time, their couplings in flight together
-                    const int f = __ffs(rem) - 1;
-                    rem &= rem - 1u;
-                    const int f2 = rem ? __ffs(rem) - 1 : f;
-                    const float j = __ldg(J + (size_t)__shfl_sync(FULL, x, f) * ldJ + xN);
-                    const float j2 = __ldg(J + (size_t)__shfl_sync(FULL, x, f2) * ldJ + xN);
-                    Fv = __fmaf_rn(__shfl_sync(FULL, d, f), j, Fv);
-                    if (rem) Fv = __fmaf_rn(__shfl_sync(FULL, d, f2), j2, Fv);
-                    rem &= rem - 1u;
+                    // 4 at a time, their couplings in flight together
+                    float j[4], dj[4];
+#pragma unroll
+                    for (int t = 0; t < 4; ++t) {
+                        const int f = rem ? __ffs(rem) - 1 : 0;
+                        dj[t] = rem ? __shfl_sync(FULL, d, f) : 0.f;
+                        j[t] = rem ? __ldg(J + (size_t)__shfl_sync(FULL, x, f) * ldJ + xN) : 0.f;
+                        rem &= rem - 1u;
+                    }
+#pragma unroll
+                    for (int t = 0; t < 4; ++t) Fv = __fmaf_rn(dj[t], j[t], Fv);
                 }
             x = xN;
             const float *jg = Jg + buf * kJgStride + lane * 33;
-            const unsigned pred = prePred[buf];  // lanes whose row of in-batch gathers is in jg
-            float qx = (float)qs[x];
 
             // The trial accepts when z = rate dE - L < 0.  z = zA - ring, zA = cz q (h + 2F) - L
             // and ring = cb q (qL + qR); unknown neighbour spins leave it in [z - sp, z + sp].
@@ -734,6 +747,7 @@ __global__ void __launch_bounds__(mc_threads(kPerSm), kPerSm) dense_sweep_multi(
             ++s;
         }
         StepConst sc = {0.f, 0.f, 0.f};
+        int own0 = -1, own1 = -1;  // kSmall: the neighbours' sites of this warp's last batch (p - 2)
         for (int p = pw; p < nBatches; p += kPf) {
             // buffer p % kPre is free once the decider has finished batch p - kPre,
             // and ring slots j - kRing are applied for the neighbours' iterations j of batch p
@@ -825,65 +839,72 @@ __global__ void __launch_bounds__(mc_threads(kPerSm), kPerSm) dense_sweep_multi(
                         atomicOr(&bp[kBmSlots * kBmWords + ((cur1 & (kBmBits - 1)) >> 5)], 1u << (cur1 & 31));
                     }
                 }
-                // batch p - 1 (the other prefetcher's) must be in the ring; its buffer
-                // slot may already hold a later batch (batch p - 2 is this warp's own)
-                if (!kSmall && p > 0 &&
-                    !wait_until<kPrefetchSleepNs>(waitNs, [&] { return uniform_acquire(&S.readyTag[(p - 1) & (kPre - 1)]) >= p; }))
-                    break;
+                // batch p - 1 (the other prefetcher's) must be in the ring; its tag's slot
+                // may already hold a later batch (batch p - 2 is this warp's own)
+                if (!kSmall) {
+                    __syncwarp();
+                    if (lane == 0) st_release_cta(&S.ringTag[buf], p + 1);
+                    if (p > 0 && !wait_until<kPrefetchSleepNs>(
+                                     waitNs, [&] { return uniform_acquire(&S.ringTag[(p - 1) & (kPre - 1)]) >= p; }))
+                        break;
+                }
                 __syncwarp();
                 const int hb = x & (kBmBits - 1);
                 if (kSmall) {
-                    // the sites of the neighbours' iterations 32 (p - q) + lane, q = 1, 2,
-                    // drawn again (the ring's entries for them are the other prefetcher's)
+                    // the sites of the neighbours' iterations of batches p - 1 (drawn again: the
+                    // ring's entries for it are the other prefetcher's) and p - 2 (this warp's last)
                     int sites[2][3];
 #pragma unroll
                     for (int nn = 0; nn < 2; ++nn) {
+                        const int j1 = 32 * (p - 1) + lane;
+                        int s1 = -1;
+                        if (nn < nNbr && j1 >= 0) {
+                            const int s2 = k >= 32 ? s : j1 / N, k2 = k >= 32 ? k - 32 : j1 - s2 * N;
+                            s1 = draw_index(draw(T.seed, (uint32_t)k2, (uint32_t)(nn ? nbr1 : nbr0),
+                                                 T.step0 + (uint32_t)s2, tag).x, N);
+                        }
                         sites[nn][0] = nn ? cur1 : cur0;
-#pragma unroll
-                        for (int q = 1; q < 3; ++q) {
-                            const int jq = 32 * (p - q) + lane;
-                            int sq = -1;
-                            if (nn < nNbr && jq >= 0) {
-                                const int s2 = jq / N, k2 = jq - s2 * N;
-                                sq = draw_index(draw(T.seed, (uint32_t)k2, (uint32_t)(nn ? nbr1 : nbr0),
-                                                     T.step0 + (uint32_t)s2, tag).x, N);
-                            }
-                            sites[nn][q] = sq;
-                        }
+                        sites[nn][1] = s1;
+                        sites[nn][2] = nn ? own1 : own0;
                     }
-                    // per batch and neighbour: the positions of each site in a table
-                    // (cleared again after use), read at the lane's own site
-                    uint32_t *tab = siteTab + pw * kSmallN;
+                    own0 = cur0;
+                    own1 = cur1;
+                    // per batch: the positions of each site in a table per neighbour (cleared
+                    // again after use), read at the lane's own site; latest batch first
+                    uint32_t *tab0 = siteTab + pw * 2 * kSmallN, *tab1 = tab0 + kSmallN;
+                    int c0[2] = {-1, -1}, c1[2] = {-1, -1}, cnt[2] = {0, 0};
+#pragma unroll 1
+                    for (int q = 0; q < 3; ++q) {
+                        const int s0 = q == 0 ? sites[0][0] : q == 1 ? sites[0][1] : sites[0][2];
+                        const int s1 = q == 0 ? sites[1][0] : q == 1 ? sites[1][1] : sites[1][2];
+                        if (s0 >= 0) atomicOr(&tab0[s0], 1u << lane);
+                        if (s1 >= 0) atomicOr(&tab1[s1], 1u << lane);
+                        __syncwarp();
+                        unsigned mk[2] = {valid ? tab0[x] : 0u, valid ? tab1[x] : 0u};
+                        __syncwarp();
+                        if (s0 >= 0) tab0[s0] = 0u;
+                        if (s1 >= 0) tab1[s1] = 0u;
+                        __syncwarp();
 #pragma unroll
-                    for (int nn = 0; nn < 2; ++nn) {
-                        if (nn >= nNbr) break;
-                        const int lim = lane - 1 + (nn ? before1 : before0);
-                        int c0 = -1, c1 = -1, cnt = 0;
-                        // latest first: batch p, then p - 1, then p - 2, each from its last iteration
-#pragma unroll
-                        for (int q = 0; q < 3; ++q) {
-                            const int sq = sites[nn][q];
-                            if (sq >= 0) atomicOr(&tab[sq], 1u << lane);
-                            __syncwarp();
-                            unsigned mk = valid ? tab[x] : 0u;
-                            __syncwarp();
-                            if (sq >= 0) tab[sq] = 0u;
-                            __syncwarp();
-                            if (q == 0) mk &= lim < 0 ? 0u : (lim >= 31 ? ~0u : (2u << lim) - 1u);
-                            cnt += __popc(mk);
-                            while (mk) {
-                                const int t = 31 - __clz(mk);
-                                mk &= ~(1u << t);
+                        for (int nn = 0; nn < 2; ++nn) {
+                            const int lim = lane - 1 + (nn ? before1 : before0);
+                            unsigned m = mk[nn];
+                            if (q == 0) m &= lim < 0 ? 0u : (lim >= 31 ? ~0u : (2u << lim) - 1u);
+                            cnt[nn] += __popc(m);
+                            while (m) {  // from the batch's last iteration
+                                const int t = 31 - __clz(m);
+                                m &= ~(1u << t);
                                 const int jj = 32 * (p - q) + t;
-                                if (c0 < 0)
-                                    c0 = jj;
-                                else if (c1 < 0)
-                                    c1 = jj;
+                                if (c0[nn] < 0)
+                                    c0[nn] = jj;
+                                else if (c1[nn] < 0)
+                                    c1[nn] = jj;
                             }
                         }
-                        if (cnt > kCand) c0 = -2;
-                        put_cands(nn, c0, cnt > kCand ? -1 : c1);
                     }
+#pragma unroll
+                    for (int nn = 0; nn < 2; ++nn)
+                        if (nn < nNbr) put_cands(nn, cnt[nn] > kCand ? -2 : c0[nn], cnt[nn] > kCand ? -1 : c1[nn]);
                 } else {
 #pragma unroll
                 for (int nn = 0; nn < 2; ++nn) {
@@ -1032,7 +1053,7 @@ static size_t multi_smem_bytes(int N) {
     size_t ghostStride = (size_t)((N + 31) / 32 + 1) & ~(size_t)1;
     return pre_offset(N) + (size_t)kPre * 32 * sizeof(PreTrial) + 2 * ghostStride * 4 +
            (size_t)2 * kBmSlots * kBmWords * 4 + 2 * kRing * 4 + 2 * kLogWords * 4 + kPre * 4 +
-           32 * 8 + (size_t)((N + 15) & ~15) + 16 + (N <= kSmallN ? (size_t)kPf * kSmallN * 4 : 0);
+           32 * 8 + (size_t)((N + 15) & ~15) + 16 + (N <= kSmallN ? (size_t)kPf * 2 * kSmallN * 4 : 0);
 }
 
 // every instance: bit 0 kHooks, bit 1 kSmall, bit 2 kSA, bit 3 four CTAs per SM (else two)
