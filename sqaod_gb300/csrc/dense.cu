@@ -350,16 +350,22 @@ __global__ void __launch_bounds__(kBlockThreads) dense_batch_persistent(const sq
     }
 }
 
+// A warp per 128-spin chunk, a lane four of its bytes, 32 apart (coalesced stores
+// whatever the row's alignment; a thread per chunk wrote 128 bytes one by one,
+// N = 1000, m = 250: 33.5 -> 2.6 us).  Every lane draws the chunk's words.
 __global__ void randomize_kernel(int8_t *q, int N, int m, uint64_t seed, uint32_t step, uint32_t tag) {
-    int chunks = (N + 127) / 128;
-    long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int chunks = (N + 127) / 128, lane = threadIdx.x & 31;
+    const long long idx = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (idx >= (long long)m * chunks) return;
-    int y = (int)(idx / chunks), c = (int)(idx - (long long)y * chunks);
-    u32x4 r = draw(seed, (uint32_t)c, (uint32_t)y, step, tag);
-    uint32_t w[4] = {r.x, r.y, r.z, r.w};
-    int8_t *qy = q + (size_t)y * N + (size_t)c * 128;
-    int nb = min(128, N - c * 128);
-    for (int b = 0; b < nb; ++b) qy[b] = ((w[b >> 5] >> (b & 31)) & 1u) ? 1 : -1;
+    const int y = (int)(idx / chunks), c = (int)(idx - (long long)y * chunks);
+    const u32x4 r = draw(seed, (uint32_t)c, (uint32_t)y, step, tag);
+    const uint32_t w[4] = {r.x, r.y, r.z, r.w};
+    int8_t *qy = q + (size_t)y * N;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int i = c * 128 + 32 * k + lane;
+        if (i < N) qy[i] = (w[k] >> lane) & 1u ? 1 : -1;
+    }
 }
 
 static int g_max_smem = -1;
@@ -401,7 +407,7 @@ SQ103_API int sq103_randomize_spins(int8_t *q, int N, int m, uint64_t seed, uint
                                     void *stream) {
     if (N <= 0 || m <= 0) return kErrBadShape;
     long long n = (long long)m * ((N + 127) / 128);
-    int blocks = (int)((n + 255) / 256);
+    int blocks = (int)((n + 7) / 8);
     randomize_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>(q, N, m, seed, step,
                                                                (uint32_t)kTagRandomize | ((uint32_t)tagSide << 8));
     return (int)cudaGetLastError();
