@@ -1020,7 +1020,15 @@ private:
         }
     }
 
-    bool useTc() const { return d_digits1_.p && sq103_bipartite_refresh_uses_tc(N0_, N1_, m_); }
+    // Half-step fields on the tensor cores: with the digit planes there, from about 80 M
+    // products a half-step on (m rounded up to a SIMT tile's 16 rows).  ms, SIMT and tensor
+    // cores: 1024 x 1024, m = 64, 64 steps (67 M) 2.89, 3.70; 1100 x 2900, m = 20, 32 steps
+    // (102 M) 3.00, 2.15; 1100 x 1100, m = 150 (194 M) 3.75, 2.62; 2900 x 2900, m = 30
+    // (269 M) 5.01, 3.07.  Decisions are exact on either, so the results are the same.
+    bool useTc() const {
+        return d_digits1_.p && (sq103_bipartite_refresh_uses_tc(N0_, N1_, m_) ||
+                                (double)((m_ + 15) / 16 * 16) * N0_ * N1_ >= 8e7);
+    }
 
     void makeDigits() {
         if (!d_digits1_.p) return;

@@ -23,11 +23,19 @@
 //   thread 0    TMA producer: per 64-wide K block, the spin tile (128 x 64 bf16)
 //               and the four digit tiles (64 x 64 bf16 each) into a 4-stage
 //               shared-memory ring (128B swizzle), mbarrier-tracked;
-//   thread 32   MMA issuer: per K block 4 x 4 tcgen05.mma kind::f16
-//               (M = 128, N = 64, K = 16), one TMEM accumulator per digit;
-//               tcgen05.commit frees each stage;
+//   thread 32   MMA issuer: per K block 4 tcgen05.mma kind::f16 (M = 128, N = 256,
+//               K = 16): the four digit tiles lie one after another in the stage,
+//               so one MMA takes all four as 256 rows of B and reads the spins
+//               once (four MMAs of N = 64 took 1290 cycles per K block, bound by
+//               shared-memory reads: 43 us for 2047 x 3001, m = 200, now 25); tcgen05.commit frees each stage;
 //   all 4 warps epilogue: tcgen05.ld of the four accumulators (a trotter row
-//               per thread), integer combination, fp32 store.
+//               per thread), integer combination, fp32 through a shared tile so
+//               that the stores are whole rows (a thread's own row of 64 stored
+//               directly took 7 to 12 thousand cycles of a launch).
+// Few output tiles (m or R small) would leave most SMs idle and walk the whole K in
+// each: a cluster of 2 or 4 CTAs then takes a tile, each a part of K, and adds the
+// integer sums through distributed shared memory.  Integer addition is exact, so
+// the result does not depend on the split.
 // Every mbarrier wait is bounded by the global timer; on timeout the CTA
 // records status 1, lets the copies it issued land (bounded), frees TMEM and
 // returns.  Two test flags make a wait run out on purpose: the producer skips
@@ -50,6 +58,8 @@ constexpr int kTcATile = kTcBM * kTcBK * 2;  // 16 KB
 constexpr int kTcBTile = kTcBN * kTcBK * 2;  // 8 KB
 constexpr int kTcStageBytes = kTcATile + kTcDigits * kTcBTile;
 constexpr int kTcSmemBytes = kTcStages * kTcStageBytes + 1024 + 256;
+constexpr int kTcOutLd = kTcBN + 1;                                     // row stride of the fp32 tile
+constexpr int kTcOutBytes = (kTcBM * kTcOutLd * 4 + 1023) / 1024 * 1024;  // its bytes
 constexpr int kTcTmemCols = 256;  // 4 accumulators of 64 fp32 columns
 constexpr unsigned long long kTcWaitNs = 2000000000ull, kTcShortWaitNs = 1000000ull;
 constexpr int kTcHeader = 256;  // digit buffer: exponent word, int shift S, then the four planes
@@ -151,7 +161,55 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
 
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// F tile (128 trotters x 64 outputs) = sum_t 2^(8t - S) (q . D_t)
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// the address of a CTA-local shared address in CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t peer_addr(const void *p, uint32_t rank) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr(p)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ long long peer_load64(uint32_t a) {
+    long long v;
+    asm volatile("ld.shared::cluster.b64 %0, [%1];" : "=l"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ int peer_load32(uint32_t a) {
+    int v;
+    asm volatile("ld.shared::cluster.b32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
+
+// columns [cz, cz + 64 / SPLIT) of the tile from the integer shares of the cluster's
+// CTAs, a row per thread, sixteen loads in flight
+template <int SPLIT>
+__device__ __forceinline__ void add_shares(const long long *red, float *out, int cz, int row, float scale) {
+    constexpr int kCols = 64 / SPLIT, kStep = 16 / SPLIT;
+    uint32_t peer[SPLIT];
+#pragma unroll
+    for (int p = 0; p < SPLIT; ++p) peer[p] = peer_addr(&red[cz * kTcBM + row], (uint32_t)p);
+#pragma unroll 1
+    for (int c = 0; c < kCols; c += kStep) {
+        long long v[kStep][SPLIT];
+#pragma unroll
+        for (int k = 0; k < kStep; ++k)
+#pragma unroll
+            for (int p = 0; p < SPLIT; ++p) v[k][p] = peer_load64(peer[p] + (uint32_t)((c + k) * kTcBM * 8));
+#pragma unroll
+        for (int k = 0; k < kStep; ++k) {
+            long long sum = v[k][0];
+#pragma unroll
+            for (int p = 1; p < SPLIT; ++p) sum += v[k][p];
+            out[row * kTcOutLd + cz + c + k] = __fmul_rn(__ll2float_rn(sum), scale);
+        }
+    }
+}
+
+// F tile (128 trotters x 64 outputs) = sum_t 2^(8t - S) (q . D_t); gridDim.z CTAs
+// (a cluster) share the tile, each K blocks [nK z / gridDim.z, nK (z + 1) / gridDim.z)
 __global__ void __launch_bounds__(kTcThreads) tc_digit_gemm(const __grid_constant__ CUtensorMap tmA,
                                                             const __grid_constant__ CUtensorMap tmB,
                                                             const int *shiftPtr, float *F, int ldF, int M, int R,
@@ -162,11 +220,12 @@ __global__ void __launch_bounds__(kTcThreads) tc_digit_gemm(const __grid_constan
     uint64_t *empty = full + kTcStages;
     uint64_t *done = empty + kTcStages;
     uint32_t *tmemSlot = reinterpret_cast<uint32_t *>(done + 1);
-    __shared__ int abortFlag;
+    __shared__ int abortFlag, okFlag;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int m0 = blockIdx.y * kTcBM, n0 = blockIdx.x * kTcBN;
-    const int nK = Kp / kTcBK;
+    const int split = (int)gridDim.z, z = (int)blockIdx.z;
+    const int kb0 = Kp / kTcBK * z / split, nK = Kp / kTcBK * (z + 1) / split - kb0;  // this CTA's K blocks
     const unsigned long long waitNs = (flags & 2) ? kTcShortWaitNs : kTcWaitNs;
 
     if (tid == 0) {
@@ -203,9 +262,9 @@ __global__ void __launch_bounds__(kTcThreads) tc_digit_gemm(const __grid_constan
             if ((flags & 1) && kb == 0) continue;  // test hook: stage 0's first copies never come
             unsigned char *a = smem + s * kTcStageBytes;
             mbar_expect_tx(&full[s], kTcStageBytes);
-            tma_load_2d(a, &tmA, &full[s], kb * kTcBK, m0);
+            tma_load_2d(a, &tmA, &full[s], (kb0 + kb) * kTcBK, m0);
 #pragma unroll
-            for (int t = 0; t < kTcDigits; ++t) tma_load_3d(a + kTcATile + t * kTcBTile, &tmB, &full[s], kb * kTcBK, n0, t);
+            for (int t = 0; t < kTcDigits; ++t) tma_load_3d(a + kTcATile + t * kTcBTile, &tmB, &full[s], (kb0 + kb) * kTcBK, n0, t);
             issued[s] = (kb / kTcStages) & 1;
         }
         // let every copy still in flight land before the CTA can leave
@@ -213,7 +272,7 @@ __global__ void __launch_bounds__(kTcThreads) tc_digit_gemm(const __grid_constan
             if (issued[s] >= 0) mbar_wait(&full[s], (uint32_t)issued[s], waitNs);
     } else if (tid == 32) {
         // ---------------------------------------------------------- MMA issuer
-        constexpr uint32_t idesc = umma_idesc_bf16(kTcBM, kTcBN);
+        constexpr uint32_t idesc = umma_idesc_bf16(kTcBM, kTcDigits * kTcBN);
         bool ok = true;
         for (int kb = 0; kb < nK; ++kb) {
             const int s = kb % kTcStages;
@@ -226,10 +285,7 @@ __global__ void __launch_bounds__(kTcThreads) tc_digit_gemm(const __grid_constan
             const uint64_t adesc = sw128_desc(a);
 #pragma unroll
             for (int kk = 0; kk < kTcBK / 16; ++kk)  // K = 16 per MMA: +32 B in the swizzled row
-#pragma unroll
-                for (int t = 0; t < kTcDigits; ++t)
-                    umma_bf16(tmem + (uint32_t)(t * kTcBN), adesc + 2 * kk,
-                              sw128_desc(a + kTcATile + t * kTcBTile) + 2 * kk, idesc, (kb | kk) ? 1u : 0u);
+                umma_bf16(tmem, adesc + 2 * kk, sw128_desc(a + kTcATile) + 2 * kk, idesc, (kb | kk) ? 1u : 0u);
             umma_commit(&empty[s]);
         }
         if (!ok) abortFlag = 1;
@@ -239,33 +295,70 @@ __global__ void __launch_bounds__(kTcThreads) tc_digit_gemm(const __grid_constan
     // ---------------------------------------------------------------- epilogue
     const bool got = mbar_wait(done, 0, waitNs);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    __syncthreads();
-    if (!got || abortFlag) {
-        if (tid == 0 && status) atomicExch(status, (int)kErrTimeout);
-    } else {
-        const int S = *shiftPtr;
-        const float scale = __int_as_float((127 - S) << 23);  // 2^-S, S in [-126, 126]
-        const int row = m0 + warp * 32 + lane;
-        const uint32_t lanes = (uint32_t)(warp * 32) << 16;
+    bool ok = __syncthreads_and(got ? 1 : 0) && !abortFlag;
+    if (!ok && tid == 0 && status) atomicExch(status, (int)kErrTimeout);
+    const int S = *shiftPtr;
+    const float scale = __int_as_float((127 - S) << 23);  // 2^-S, S in [-126, 126]
+    const uint32_t lanes = (uint32_t)(warp * 32) << 16;
+    // (the ring is idle now) the fp32 tile, rows padded against bank conflicts, and for a
+    // split tile this CTA's integer sums, [64 columns][128 rows]
+    float *out = reinterpret_cast<float *>(smem);
+    long long *red = reinterpret_cast<long long *>(smem + kTcOutBytes);
+    if (ok) {
+        // |P_t| <= 128 Kp: up to 2^22 the sum P + 1.5 2^23 is exact and holds P in its low bits
+        const bool narrow = Kp <= (1 << 15);
 #pragma unroll 1
         for (int c0 = 0; c0 < kTcBN; c0 += 16) {
             uint32_t p[kTcDigits][16];
 #pragma unroll
             for (int t = 0; t < kTcDigits; ++t) tmem_ld16(tmem + lanes + (uint32_t)(t * kTcBN + c0), p[t]);
             tmem_wait_ld();
-            if (row < M) {
-                float *dst = F + (size_t)row * ldF + n0 + c0;
-                const int nv = min(16, R - (n0 + c0));
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    long long v = 0;
+            for (int j = 0; j < 16; ++j) {
+                long long v;
+                if (narrow) {
+                    int d[kTcDigits];
+#pragma unroll
+                    for (int t = 0; t < kTcDigits; ++t)
+                        d[t] = __float_as_int(__fadd_rn(__uint_as_float(p[t][j]), 12582912.f)) - 0x4B400000;
+                    v = ((long long)(d[3] * 256 + d[2]) << 16) + (d[1] * 256 + d[0]);
+                } else {
+                    v = 0;
 #pragma unroll
                     for (int t = kTcDigits - 1; t >= 0; --t)
                         v = (v << 8) + (long long)__float2int_rn(__uint_as_float(p[t][j]));
-                    if (j < nv) dst[j] = __fmul_rn(__ll2float_rn(v), scale);
                 }
+                if (split > 1)
+                    red[(c0 + j) * kTcBM + tid] = v;
+                else
+                    out[tid * kTcOutLd + c0 + j] = __fmul_rn(__ll2float_rn(v), scale);
             }
         }
+    }
+    int cols = kTcBN, cz = 0;  // the columns of the tile that this CTA stores
+    if (split > 1) {
+        if (tid == 0) okFlag = ok ? 1 : 0;
+        __syncwarp();
+        cluster_sync_all();
+        // this CTA's columns: the sums of every CTA's share (none if one gave up)
+        for (int p = 0; p < split; ++p) ok = ok && peer_load32(peer_addr(&okFlag, (uint32_t)p));
+        cols = kTcBN / split;
+        cz = z * cols;
+        if (ok) {
+            if (split == 2)
+                add_shares<2>(red, out, cz, tid, scale);
+            else
+                add_shares<4>(red, out, cz, tid, scale);
+        }
+        __syncwarp();
+        cluster_sync_all();  // a CTA's shared memory stays until its peers have read it
+    } else {
+        __syncthreads();
+    }
+    if (ok) {
+        const int c = cz + tid % cols;  // whole rows of the tile, kTcThreads / cols at a time
+        for (int r = tid / cols; r < kTcBM && m0 + r < M; r += kTcThreads / cols)
+            if (n0 + c < R) F[(size_t)(m0 + r) * ldF + n0 + c] = out[r * kTcOutLd + c];
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -420,9 +513,28 @@ SQ103_API int sq103_tc_refresh(const void *digits, int R, int K, const int8_t *q
             if (dev >= 0 && dev < 256) attrSet[dev] = true;
         }
     }
-    dim3 grid((R + kTcBN - 1) / kTcBN, (m + kTcBM - 1) / kTcBM);
-    tc_digit_gemm<<<grid, kTcThreads, kTcSmemBytes, st>>>(tmA, tmB, reinterpret_cast<const int *>(base + 16), F, ldF,
-                                                          m, R, ldD, flags, status);
+    // K split over a cluster of up to 4 while the tiles times the split stay within one CTA
+    // per SM and a CTA has two K blocks or more.  us per refresh with the spins' conversion,
+    // by largest split 1, 2, 4, 8: R = K = 1501, m = 63 (24 tiles) 20.5, 20.5, 18.5, 18.4;
+    // 2047 x 3001, m = 200 (64 tiles) 28.9, 24.6, 24.6, 24.6; 1024, m = 64 (16 tiles) 18.6,
+    // 18.7, 18.6, 26.8 (a cluster of eight waits for eight free SMs of one GPC)
+    const int tilesX = (R + kTcBN - 1) / kTcBN, tilesY = (m + kTcBM - 1) / kTcBM;
+    int split = 1;
+    while (split < 4 && (long long)tilesX * tilesY * split * 2 <= 152 && ldD / kTcBK >= 4 * split) split *= 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(tilesX, tilesY, split);
+    cfg.blockDim = dim3(kTcThreads);
+    cfg.dynamicSmemBytes = kTcSmemBytes;
+    cfg.stream = st;
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = (unsigned)split;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    const cudaError_t le = cudaLaunchKernelEx(&cfg, tc_digit_gemm, tmA, tmB, reinterpret_cast<const int *>(base + 16), F,
+                                              ldF, m, R, ldD, flags, status);
+    if (le != cudaSuccess) return (int)le;
     return (int)cudaGetLastError();
 }
 
