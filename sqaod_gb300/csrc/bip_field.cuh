@@ -26,6 +26,7 @@
 #include <cstdint>
 
 #include "field_gemm.cuh"
+#include "sq_common.cuh"
 
 namespace sq103 {
 
@@ -41,7 +42,8 @@ static_assert(kBipGroups * 2 * kBipTileM * kBipTileN <= kBipGroups * kBipWarpFlo
 //     for B(k, n) = Bm[k * ldb + n], 4-way for the transposed layout)
 __device__ __forceinline__ int bip_swz_b(int k) { return (k & 7) << 2; }
 
-template <bool TRANS_B, bool EXACT, typename OutT>
+// kDependent: the couplings of the first chunk are loaded before pdl_wait, the spins after.
+template <bool TRANS_B, bool EXACT, typename OutT, bool kDependent = false>
 __device__ __forceinline__ void bip_field_tile(const int8_t *A, int lda, const float *Bm, int ldb, OutT *C, int ldc,
                                                int M, int Nn, int K, int y0, int n0, float *smem) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -60,22 +62,28 @@ __device__ __forceinline__ void bip_field_tile(const int8_t *A, int lda, const f
 
     float ra[16], rb[32];
     const bool rowsIn = y0 + 16 <= M && n0 + 32 <= Nn;
-    auto load = [&](int ch) {
+    auto load = [&](int ch, bool spins, bool couplings) {
         const int k0 = ch << 5, k = k0 + lane;
         if (rowsIn && k0 + 32 <= K) {  // the whole chunk is inside: no bounds checks
-            const int8_t *Ap = A + (size_t)y0 * lda + k;
+            if (spins) {
+                const int8_t *Ap = A + (size_t)y0 * lda + k;
 #pragma unroll
-            for (int i = 0; i < 16; ++i) ra[i] = (float)Ap[(size_t)i * lda];
+                for (int i = 0; i < 16; ++i) ra[i] = (float)Ap[(size_t)i * lda];
+            }
+            if (!couplings) return;
             const float *Bp = TRANS_B ? Bm + (size_t)n0 * ldb + k : Bm + (size_t)k0 * ldb + n0 + lane;
 #pragma unroll
             for (int j = 0; j < 32; ++j) rb[j] = Bp[(size_t)j * ldb];
             return;
         }
+        if (spins) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            const int y = y0 + i;
-            ra[i] = (y < M && k < K) ? (float)A[(size_t)y * lda + k] : 0.f;
+            for (int i = 0; i < 16; ++i) {
+                const int y = y0 + i;
+                ra[i] = (y < M && k < K) ? (float)A[(size_t)y * lda + k] : 0.f;
+            }
         }
+        if (!couplings) return;
         if (!TRANS_B) {  // lane = column
             const int n = n0 + lane;
 #pragma unroll
@@ -105,12 +113,18 @@ __device__ __forceinline__ void bip_field_tile(const int8_t *A, int lda, const f
         }
     };
 
-    if (cb < ce) load(cb);
+    if (kDependent) {
+        if (cb < ce) load(cb, false, true);
+        pdl_wait();
+        if (cb < ce) load(cb, true, false);
+    } else if (cb < ce) {
+        load(cb, true, true);
+    }
     for (int ch = cb; ch < ce; ++ch) {
         __syncwarp();  // the previous chunk's reads are done
         store();
         __syncwarp();
-        if (ch + 1 < ce) load(ch + 1);  // in flight during this chunk
+        if (ch + 1 < ce) load(ch + 1, true, true);  // in flight during this chunk
         float part[4][4];
 #pragma unroll
         for (int a = 0; a < 4; ++a)
@@ -177,7 +191,8 @@ template <bool TRANS_B, bool EXACT, typename OutT>
 __global__ void __launch_bounds__(256) bip_field_kernel(const int8_t *A, int lda, const float *Bm, int ldb, OutT *C,
                                                         int ldc, int M, int Nn, int K) {
     extern __shared__ __align__(16) float bip_smem[];
-    bip_field_tile<TRANS_B, EXACT, OutT>(A, lda, Bm, ldb, C, ldc, M, Nn, K, blockIdx.y * kBipTileM,
+    pdl_trigger();
+    bip_field_tile<TRANS_B, EXACT, OutT, true>(A, lda, Bm, ldb, C, ldc, M, Nn, K, blockIdx.y * kBipTileM,
                                          blockIdx.x * kBipTileN, bip_smem);
 }
 

@@ -119,9 +119,10 @@ __global__ void bg_hamiltonian_cols(const float *W, int N0, int N1, float sign, 
 
 template <bool TRANS_B, bool EXACT, typename OutT>
 static void launch_bip_field(const int8_t *A, int lda, const float *B, int ldb, OutT *C, int ldc, int M, int Nn,
-                             int K, cudaStream_t s) {
+                             int K, cudaStream_t s, bool dependent = false) {
     dim3 grid((Nn + kBipTileN - 1) / kBipTileN, (M + kBipTileM - 1) / kBipTileM);
-    bip_field_kernel<TRANS_B, EXACT, OutT><<<grid, 256, kBipFieldSmem, s>>>(A, lda, B, ldb, C, ldc, M, Nn, K);
+    launch_dependent(dependent, bip_field_kernel<TRANS_B, EXACT, OutT>, grid, dim3(256), kBipFieldSmem, s, A, lda, B,
+                     ldb, C, ldc, M, Nn, K);
 }
 
 // ------------------------------------------------------------ energies
@@ -238,14 +239,18 @@ SQ103_API int sq103_dense_field_refresh_batch(const sq103_field_job *jobs, const
     return (int)cudaGetLastError();
 }
 
+int sq103_bipartite_fields_after(const float *J, int N0, int N1, const int8_t *qFixed, int side, float *F, int m,
+                                 bool dependent, cudaStream_t s) {
+    if (side == 1)  // F1[y][i] = sum_j J[i][j] q0[y][j]
+        launch_bip_field<true, false, float>(qFixed, N0, J, N0, F, N1, m, N1, N0, s, dependent);
+    else  // F0[y][j] = sum_i q1[y][i] J[i][j]
+        launch_bip_field<false, false, float>(qFixed, N1, J, N0, F, N0, m, N0, N1, s, dependent);
+    return (int)cudaGetLastError();
+}
+
 SQ103_API int sq103_bipartite_fields(const float *J, int N0, int N1, const int8_t *qFixed, int side, float *F, int m,
                            void *stream) {
-    cudaStream_t s = (cudaStream_t)stream;
-    if (side == 1)  // F1[y][i] = sum_j J[i][j] q0[y][j]
-        launch_bip_field<true, false, float>(qFixed, N0, J, N0, F, N1, m, N1, N0, s);
-    else  // F0[y][j] = sum_i q1[y][i] J[i][j]
-        launch_bip_field<false, false, float>(qFixed, N1, J, N0, F, N0, m, N0, N1, s);
-    return (int)cudaGetLastError();
+    return sq103_bipartite_fields_after(J, N0, N1, qFixed, side, F, m, false, (cudaStream_t)stream);
 }
 
 SQ103_API int sq103_dense_energy(const float *J, int ldJ, const float *h, const double *c64, const int8_t *q, int N,

@@ -58,6 +58,32 @@ __host__ __device__ __forceinline__ uint32_t mulhi32(uint32_t a, uint32_t b) {
 #endif
 }
 
+#ifdef __CUDACC__
+// Programmatic dependent launch: a kernel launched with launch_dependent may start
+// while the one before it in the stream runs; pdl_wait returns when that one has
+// completed and its writes are visible (at once in a plain launch), pdl_trigger
+// lets the next one start.  What a kernel reads or writes before pdl_wait must not
+// depend on the kernels before it.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... Params, class... Args>
+inline cudaError_t launch_dependent(bool dependent, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
+                                    cudaStream_t st, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = dependent ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+#endif
+
 // Philox4x32-10.  A file may set SQ103_PHILOX_UNROLL (rounds per loop iteration)
 // where code size counts more than the loop (the one-CTA-per-trotter sweep).
 #ifndef SQ103_PHILOX_UNROLL

@@ -247,6 +247,8 @@ __global__ void __launch_bounds__(kTcThreads) tc_digit_gemm(const __grid_constan
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmemSlot;
+    pdl_trigger();
+    pdl_wait();  // the spins, and F's last readers
 
     if (tid == 0) {
         // ---------------------------------------------------------- producer
@@ -409,6 +411,8 @@ __global__ void tc_make_digits(const float *J, int ldJ, int R, int K, int ldD, i
 
 // spins (m x K int8, row stride ldq) -> bf16 (m x ldA), zero beyond K
 __global__ void tc_spins_bf16(const int8_t *q, int ldq, int m, int K, int ldA, __nv_bfloat16 *A) {
+    pdl_trigger();
+    pdl_wait();
     const size_t n = (size_t)m * ldA;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const int y = (int)(i / ldA), k = (int)(i - (size_t)y * ldA);
@@ -467,16 +471,21 @@ SQ103_API int sq103_tc_make_digits(const float *J, int ldJ, int R, int K, int tr
 
 SQ103_API int sq103_tc_refresh(const void *digits, int R, int K, const int8_t *q, int ldq, int m, void *spinsBf16,
                                float *F, int ldF, int flags, int *status, void *stream) {
+    return sq103_tc_refresh_after(digits, R, K, q, ldq, m, spinsBf16, F, ldF, flags, status, false,
+                                  (cudaStream_t)stream);
+}
+
+int sq103_tc_refresh_after(const void *digits, int R, int K, const int8_t *q, int ldq, int m, void *spinsBf16,
+                           float *F, int ldF, int flags, int *status, bool dependent, cudaStream_t st) {
     if (R <= 0 || K <= 0 || m <= 0 || K >= (1 << 17) || !digits || !q || !spinsBf16 || !F ||
         (reinterpret_cast<uintptr_t>(digits) & 255) || (reinterpret_cast<uintptr_t>(spinsBf16) & 15) ||
         (flags & ~3))
         return kErrBadShape;
     auto enc = tensor_map_encoder();
     if (!enc) return kErrBadShape;
-    cudaStream_t st = (cudaStream_t)stream;
     const int ldD = ld_pad(K);
-    tc_spins_bf16<<<grid_for((size_t)m * ldD), 256, 0, st>>>(q, ldq, m, K, ldD,
-                                                            reinterpret_cast<__nv_bfloat16 *>(spinsBf16));
+    launch_dependent(dependent, tc_spins_bf16, dim3(grid_for((size_t)m * ldD)), dim3(256), 0, st, q, ldq, m, K, ldD,
+                     reinterpret_cast<__nv_bfloat16 *>(spinsBf16));
     const unsigned char *base = static_cast<const unsigned char *>(digits);
     CUtensorMap tmA, tmB;
     {
@@ -526,12 +535,14 @@ SQ103_API int sq103_tc_refresh(const void *digits, int R, int K, const int8_t *q
     cfg.blockDim = dim3(kTcThreads);
     cfg.dynamicSmemBytes = kTcSmemBytes;
     cfg.stream = st;
-    cudaLaunchAttribute attr = {};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = attr.val.clusterDim.y = 1;
-    attr.val.clusterDim.z = (unsigned)split;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cudaLaunchAttribute attr[2] = {};
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = (unsigned)split;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // behind the spins' conversion
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
     const cudaError_t le = cudaLaunchKernelEx(&cfg, tc_digit_gemm, tmA, tmB, reinterpret_cast<const int *>(base + 16), F,
                                               ldF, m, R, ldD, flags, status);
     if (le != cudaSuccess) return (int)le;
