@@ -253,6 +253,19 @@ SQ103_API int sq103_bipartite_fields(const float *J, int N0, int N1, const int8_
     return sq103_bipartite_fields_after(J, N0, N1, qFixed, side, F, m, false, (cudaStream_t)stream);
 }
 
+int sq103_dense_energy_of_sums(const double *r, const float *h, const double *c64, const int8_t *q, int N, int m,
+                               int maximize, double *E64, float *E32, cudaStream_t st) {
+    dg_energy_finish<<<m, 256, 0, st>>>(q, N, h, r, c64, maximize ? -1. : 1., E64, E32);
+    return (int)cudaGetLastError();
+}
+
+int sq103_bipartite_energy_of_sums(const double *r, const float *h0, const float *h1, const double *c64,
+                                   const int8_t *q0, const int8_t *q1, int N0, int N1, int m, int maximize,
+                                   double *E64, cudaStream_t st) {
+    bg_energy_finish<<<m, 256, 0, st>>>(q0, q1, N0, N1, h0, h1, r, c64, maximize ? -1. : 1., E64, nullptr);
+    return (int)cudaGetLastError();
+}
+
 SQ103_API int sq103_dense_energy(const float *J, int ldJ, const float *h, const double *c64, const int8_t *q, int N,
                        int m, int maximize, double *r_scratch, double *E64, float *E32, void *stream) {
     cudaStream_t s = (cudaStream_t)stream;

@@ -658,12 +658,39 @@ private:
         if (r->kind == 0) {
             const int N = r->N0;
             double *scratch = (double *)((unsigned char *)r->dt.q + al((size_t)m * N));
-            SQ_CHECK(sq103_dense_energy(r->dt.J, r->dt.ldJ, r->dt.h, r->c64, r->dt.q, N, m, r->optimize, scratch,
-                                        r->dE, nullptr, st_.get()));
+            if (r->digits) {  // as the single annealer; the low digits in a shared scratch
+                low_.ensure(sq103_tc_digits_bytes(N, N));
+                SQ_CHECK(sq103_tc_make_low_digits(r->dt.J, r->dt.ldJ, N, N, low_.p, st_.get()));
+                SQ_CHECK(sq103_tc_row_sums(r->digits, low_.p, N, N, r->dt.q, N, m, r->spinsBf16, scratch, r->dStatus,
+                                           st_.get()));
+                SQ_CHECK(sq103_dense_energy_of_sums(scratch, r->dt.h, r->c64, r->dt.q, N, m, r->optimize, r->dE,
+                                                    nullptr, st_.get()));
+            } else {
+                SQ_CHECK(sq103_dense_energy(r->dt.J, r->dt.ldJ, r->dt.h, r->c64, r->dt.q, N, m, r->optimize, scratch,
+                                            r->dE, nullptr, st_.get()));
+            }
         } else {
             double *scratch = (double *)((unsigned char *)r->bt.F1 + al((size_t)m * r->N1 * 4));
-            SQ_CHECK(sq103_bipartite_energy(r->bt.J, r->bt.h0, r->bt.h1, r->c64, r->bt.q0, r->bt.q1, r->N0, r->N1,
-                                            m, r->optimize, scratch, r->dE, nullptr, st_.get()));
+            if (sq103_bipartite_tc_pays(r->N0, r->N1, m)) {
+                const void *digits = r->bt.digits1;
+                void *bf16 = r->bt.spinsBf16;
+                if (!digits) {  // a request that steps on the SIMT fields
+                    high_.ensure(sq103_tc_digits_bytes(r->N1, r->N0));
+                    bf16_.ensure(sq103_tc_spins_bytes(m, r->N0));
+                    SQ_CHECK(sq103_tc_make_digits(r->bt.J, r->N0, r->N1, r->N0, 0, high_.p, st_.get()));
+                    digits = high_.p;
+                    bf16 = bf16_.p;
+                }
+                low_.ensure(sq103_tc_digits_bytes(r->N1, r->N0));
+                SQ_CHECK(sq103_tc_make_low_digits(r->bt.J, r->N0, r->N1, r->N0, low_.p, st_.get()));
+                SQ_CHECK(sq103_tc_row_sums(digits, low_.p, r->N1, r->N0, r->bt.q0, r->N0, m, bf16, scratch, r->dStatus,
+                                           st_.get()));
+                SQ_CHECK(sq103_bipartite_energy_of_sums(scratch, r->bt.h0, r->bt.h1, r->c64, r->bt.q0, r->bt.q1, r->N0,
+                                                        r->N1, m, r->optimize, r->dE, st_.get()));
+            } else {
+                SQ_CHECK(sq103_bipartite_energy(r->bt.J, r->bt.h0, r->bt.h1, r->c64, r->bt.q0, r->bt.q1, r->N0, r->N1,
+                                                m, r->optimize, scratch, r->dE, nullptr, st_.get()));
+            }
         }
         SQ_CHECK(cudaEventCreateWithFlags(&r->done, cudaEventDisableTiming));
         SQ_CHECK(cudaEventRecord(r->done, st_.get()));
@@ -787,6 +814,7 @@ private:
     DevBuf<sq103_bipartite_task> bTasks_;
     DevBuf<int> dPos_, bPos_, counts_, queues_;
     DevBuf<float> dW_;
+    DevBuf<unsigned char> low_, high_, bf16_;  // digits and spins of the request whose energies are queued
     static constexpr int kMaxPack = 64;  // instances per packed launch (sq103_dense_anneal_pack)
     // light requests on the large ones' routes at a time: dense of N >= 128, dense below, bipartite
     static constexpr int kMaxLightDense = 512, kMaxLightSmall = 64, kMaxLightBip = 32;

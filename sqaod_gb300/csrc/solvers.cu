@@ -352,7 +352,21 @@ public:
         if (fp64_)
             SQ_CHECK(sq103_dense_energy64(d_J64_.p, d_h64_.p, c64h_, d_q_.p, N_, m_, om_ == sq::optMaximize,
                                           d_E64_.p, st_.get()));
-        else
+        else if (d_digits_.p) {
+            // row sums on the tensor cores, to FP64 accuracy with the low digits, which are
+            // made with the first energies of a problem.  N = 4096, m = 256, 64 steps and the
+            // energies: 15.9 ms with the SIMT double-float sums (1.13 ms of it), 14.7 this way.
+            if (!lowMade_) {
+                d_low_.ensure(sq103_tc_digits_bytes(N_, N_));
+                SQ_CHECK(sq103_tc_make_low_digits(d_J_.p, ldJ_, N_, N_, d_low_.p, st_.get()));
+                lowMade_ = true;
+            }
+            SQ_CHECK(sq103_tc_row_sums(d_digits_.p, d_low_.p, N_, N_, d_q_.p, N_, m_, d_Abf_.p, d_r_.p, d_status_.p,
+                                       st_.get()));
+            SQ_CHECK(sq103_dense_energy_of_sums(d_r_.p, d_h_.p, d_c64_.p, d_q_.p, N_, m_, om_ == sq::optMaximize,
+                                                d_E64_.p, d_E32_.p, st_.get()));
+            checkStatus();
+        } else
             SQ_CHECK(sq103_dense_energy(d_J_.p, ldJ_, d_h_.p, d_c64_.p, d_q_.p, N_, m_, om_ == sq::optMaximize,
                                         d_r_.p, d_E64_.p, d_E32_.p, st_.get()));
         SQ_CHECK(cudaMemcpyAsync(h_E64_.p, d_E64_.p, sizeof(double) * m_, cudaMemcpyDeviceToHost, st_.get()));
@@ -481,6 +495,7 @@ private:
     }
 
     void makeDigits() {
+        lowMade_ = false;
         if (d_digits_.p) SQ_CHECK(sq103_tc_make_digits(d_J_.p, ldJ_, N_, N_, 0, d_digits_.p, st_.get()));
     }
 
@@ -613,6 +628,8 @@ private:
     mutable Stream st_;
     DevBuf<float> d_J_, d_h_, d_c_, d_F_, d_E32_, d_sched_;
     DevBuf<unsigned char> d_digits_, d_Abf_;  // tensor-core refresh: digit planes of J, spins in bf16
+    DevBuf<unsigned char> d_low_;             // tensor-core energies: the low digit planes
+    bool lowMade_ = false;
     DevBuf<double> d_J64_, d_h64_;            // FP64 problem of a <double> annealer (J64 row stride N)
     double c64h_ = 0.;
     bool fp64_ = false;
@@ -894,7 +911,24 @@ public:
         if (fp64_)
             SQ_CHECK(sq103_bipartite_energy64(d_J64_.p, d_h0_64_.p, d_h1_64_.p, c64h_, d_q0_.p, d_q1_.p, N0_, N1_, m_,
                                               om_ == sq::optMaximize, d_E64_.p, st_.get()));
-        else
+        else if (useTc()) {  // as DenseAnnealer::calculate_E
+            if (!lowMade_) {
+                d_low1_.ensure(sq103_tc_digits_bytes(N1_, N0_));
+                SQ_CHECK(sq103_tc_make_low_digits(d_J_.p, N0_, N1_, N0_, d_low1_.p, st_.get()));
+                lowMade_ = true;
+            }
+            SQ_CHECK(sq103_tc_row_sums(d_digits1_.p, d_low1_.p, N1_, N0_, d_q0_.p, N0_, m_, d_Abf_.p, d_r_.p,
+                                       d_status_.p, st_.get()));
+            SQ_CHECK(sq103_bipartite_energy_of_sums(d_r_.p, d_h0_.p, d_h1_.p, d_c64_.p, d_q0_.p, d_q1_.p, N0_, N1_, m_,
+                                                    om_ == sq::optMaximize, d_E64_.p, st_.get()));
+            int status = 0;
+            SQ_CHECK(cudaMemcpyAsync(&status, d_status_.p, sizeof(int), cudaMemcpyDeviceToHost, st_.get()));
+            st_.sync();
+            if (status != 0) {
+                SQ_CHECK(cudaMemsetAsync(d_status_.p, 0, sizeof(int), st_.get()));
+                sq::throwError("calculate_E: device wait timed out (status %d); spins are not valid.", status);
+            }
+        } else
             SQ_CHECK(sq103_bipartite_energy(d_J_.p, d_h0_.p, d_h1_.p, d_c64_.p, d_q0_.p, d_q1_.p, N0_, N1_, m_,
                                             om_ == sq::optMaximize, d_r_.p, d_E64_.p, nullptr, st_.get()));
         SQ_CHECK(cudaMemcpyAsync(h_E64_.p, d_E64_.p, sizeof(double) * m_, cudaMemcpyDeviceToHost, st_.get()));
@@ -1020,17 +1054,11 @@ private:
         }
     }
 
-    // Half-step fields on the tensor cores: with the digit planes there, from about 80 M
-    // products a half-step on (m rounded up to a SIMT tile's 16 rows).  ms, SIMT and tensor
-    // cores: 1024 x 1024, m = 64, 64 steps (67 M) 2.89, 3.70; 1100 x 2900, m = 20, 32 steps
-    // (102 M) 3.00, 2.15; 1100 x 1100, m = 150 (194 M) 3.75, 2.62; 2900 x 2900, m = 30
-    // (269 M) 5.01, 3.07.  Decisions are exact on either, so the results are the same.
-    bool useTc() const {
-        return d_digits1_.p && (sq103_bipartite_refresh_uses_tc(N0_, N1_, m_) ||
-                                (double)((m_ + 15) / 16 * 16) * N0_ * N1_ >= 8e7);
-    }
+    // half-step fields and energies on the tensor cores
+    bool useTc() const { return d_digits1_.p && sq103_bipartite_tc_pays(N0_, N1_, m_); }
 
     void makeDigits() {
+        lowMade_ = false;
         if (!d_digits1_.p) return;
         SQ_CHECK(sq103_tc_make_digits(d_J_.p, N0_, N1_, N0_, 0, d_digits1_.p, st_.get()));
         SQ_CHECK(sq103_tc_make_digits(d_J_.p, N0_, N0_, N1_, 1, d_digits0_.p, st_.get()));
@@ -1137,6 +1165,8 @@ private:
     DevBuf<double> d_c64_, d_scratch_, d_E64_, d_r_;
     DevBuf<double> d_J64_, d_h0_64_, d_h1_64_;        // FP64 problem of a <double> annealer
     DevBuf<unsigned char> d_digits1_, d_digits0_, d_Abf_;  // tensor-core half-step fields
+    DevBuf<unsigned char> d_low1_;                         // tensor-core energies
+    bool lowMade_ = false;
     DevBuf<int> d_status_;
     DevBuf<int8_t> d_q0_, d_q1_;
     DevBuf<unsigned long long> d_acc_;
@@ -2196,8 +2226,17 @@ public:
         const Inst &in = inst(i);
         r_.ensure((size_t)in.m * in.N);
         E64_.ensure(in.m);
-        SQ_CHECK(sq103_dense_energy(in.J, in.ldJ, in.h, in.c64, in.q, in.N, in.m, optimize_[i], r_.p, E64_.p,
-                                    nullptr, st_.get()));
+        if (in.digits.p) {  // as the single annealer; the low digits in a shared scratch
+            low_.ensure(sq103_tc_digits_bytes(in.N, in.N));
+            SQ_CHECK(sq103_tc_make_low_digits(in.J, in.ldJ, in.N, in.N, low_.p, st_.get()));
+            SQ_CHECK(sq103_tc_row_sums(in.digits.p, low_.p, in.N, in.N, in.q, in.N, in.m, in.Abf.p, r_.p, in.status,
+                                       st_.get()));
+            SQ_CHECK(sq103_dense_energy_of_sums(r_.p, in.h, in.c64, in.q, in.N, in.m, optimize_[i], E64_.p, nullptr,
+                                                st_.get()));
+        } else {
+            SQ_CHECK(sq103_dense_energy(in.J, in.ldJ, in.h, in.c64, in.q, in.N, in.m, optimize_[i], r_.p, E64_.p,
+                                        nullptr, st_.get()));
+        }
         SQ_CHECK(cudaMemcpyAsync(E, E64_.p, sizeof(double) * in.m, cudaMemcpyDeviceToHost, st_.get()));
         st_.sync();
     }
@@ -2325,6 +2364,7 @@ private:
     std::vector<int> optimize_;
     DevBuf<float> dW_, sched_;
     DevBuf<double> scratch_, r_, E64_;
+    DevBuf<unsigned char> low_;  // low digits of the instance whose energies are computed
     DevBuf<sq103_dense_task> dTasks_;
     DevBuf<int> dOrder_, dPos_, dQueue_, dStatus_;
     DevBuf<sq103_field_job> dJobs_;  // the SIMT refresh of every instance below the tensor-core size

@@ -13,5 +13,17 @@ extern "C" int sq103_tc_refresh_after(const void *digits, int R, int K, const in
                                       void *spinsBf16, float *F, int ldF, int flags, int *status, bool dependent,
                                       cudaStream_t st);
 
+extern "C" int sq103_bipartite_tc_pays(int N0, int N1, int m);
+// the planes of what the digits of J (R x K, row stride ldJ) round away (the layout and size of its digits)
+extern "C" int sq103_tc_make_low_digits(const float *J, int ldJ, int R, int K, void *digits, cudaStream_t st);
+extern "C" int sq103_tc_row_sums(const void *digits, const void *lowDigits, int R, int K, const int8_t *q, int ldq,
+                                 int m, void *spinsBf16, double *r, int *status, cudaStream_t st);
+// the FP64 energies from the row sums r (m x N of q J; m x N1 of q0 J^T)
+extern "C" int sq103_dense_energy_of_sums(const double *r, const float *h, const double *c64, const int8_t *q, int N,
+                                          int m, int maximize, double *E64, float *E32, cudaStream_t st);
+extern "C" int sq103_bipartite_energy_of_sums(const double *r, const float *h0, const float *h1, const double *c64,
+                                              const int8_t *q0, const int8_t *q1, int N0, int N1, int m, int maximize,
+                                              double *E64, cudaStream_t st);
+
 // sets the message returned by sq103_last_error() on this thread
 void sq103_set_error(const char *msg);

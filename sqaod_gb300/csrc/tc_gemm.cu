@@ -19,6 +19,11 @@
 // left is the quantisation of B (below 2^-29 of the largest |B| per element),
 // far below the fp32 rounding of the result.
 //
+// Energies (tc_digit_gemm<double>).  The FP64 energies need the row sums to FP64
+// accuracy.  Four more digit planes hold what the first four round away, 31 bits
+// further down (62 below the largest |B|), and a second contraction adds them: both
+// sums are exact integers, and the row sum is rounded once, in FP64.
+//
 // Kernel (one CTA per 128 x 64 output tile, 128 threads):
 //   thread 0    TMA producer: per 64-wide K block, the spin tile (128 x 64 bf16)
 //               and the four digit tiles (64 x 64 bf16 each) into a 4-stage
@@ -58,10 +63,11 @@ constexpr int kTcATile = kTcBM * kTcBK * 2;  // 16 KB
 constexpr int kTcBTile = kTcBN * kTcBK * 2;  // 8 KB
 constexpr int kTcStageBytes = kTcATile + kTcDigits * kTcBTile;
 constexpr int kTcSmemBytes = kTcStages * kTcStageBytes + 1024 + 256;
-constexpr int kTcOutLd = kTcBN + 1;                                     // row stride of the fp32 tile
-constexpr int kTcOutBytes = (kTcBM * kTcOutLd * 4 + 1023) / 1024 * 1024;  // its bytes
+constexpr int kTcOutLd = kTcBN + 1;                                     // row stride of the output tile
+constexpr int kTcOutBytes = (kTcBM * kTcOutLd * 8 + 1023) / 1024 * 1024;  // its bytes (FP64 row sums)
 constexpr int kTcTmemCols = 256;  // 4 accumulators of 64 fp32 columns
 constexpr unsigned long long kTcWaitNs = 2000000000ull, kTcShortWaitNs = 1000000ull;
+constexpr int kTcAdd = 4;  // launch flag (see tc_digit_gemm)
 constexpr int kTcHeader = 256;  // digit buffer: exponent word, int shift S, then the four planes
 
 __device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -183,10 +189,22 @@ __device__ __forceinline__ int peer_load32(uint32_t a) {
     return v;
 }
 
+// v 2^-S, rounded once
+template <class Out>
+__device__ __forceinline__ Out scaled_sum(long long v, int S);
+template <>
+__device__ __forceinline__ float scaled_sum<float>(long long v, int S) {  // S in [-126, 126]
+    return __fmul_rn(__ll2float_rn(v), __int_as_float((127 - S) << 23));
+}
+template <>
+__device__ __forceinline__ double scaled_sum<double>(long long v, int S) {  // S in [-126, 157]
+    return __dmul_rn(__ll2double_rn(v), __longlong_as_double((long long)(1023 - S) << 52));
+}
+
 // columns [cz, cz + 64 / SPLIT) of the tile from the integer shares of the cluster's
 // CTAs, a row per thread, sixteen loads in flight
-template <int SPLIT>
-__device__ __forceinline__ void add_shares(const long long *red, float *out, int cz, int row, float scale) {
+template <int SPLIT, class Out>
+__device__ __forceinline__ void add_shares(const long long *red, Out *out, int cz, int row, int S) {
     constexpr int kCols = 64 / SPLIT, kStep = 16 / SPLIT;
     uint32_t peer[SPLIT];
 #pragma unroll
@@ -203,16 +221,19 @@ __device__ __forceinline__ void add_shares(const long long *red, float *out, int
             long long sum = v[k][0];
 #pragma unroll
             for (int p = 1; p < SPLIT; ++p) sum += v[k][p];
-            out[row * kTcOutLd + cz + c + k] = __fmul_rn(__ll2float_rn(sum), scale);
+            out[row * kTcOutLd + cz + c + k] = scaled_sum<Out>(sum, S);
         }
     }
 }
 
 // F tile (128 trotters x 64 outputs) = sum_t 2^(8t - S) (q . D_t); gridDim.z CTAs
 // (a cluster) share the tile, each K blocks [nK z / gridDim.z, nK (z + 1) / gridDim.z)
+// Out float: fields.  double: row sums; flag kTcAdd adds to those in F, and a matrix
+// with a non-finite value (its exponent word) gives NaN.
+template <class Out>
 __global__ void __launch_bounds__(kTcThreads) tc_digit_gemm(const __grid_constant__ CUtensorMap tmA,
                                                             const __grid_constant__ CUtensorMap tmB,
-                                                            const int *shiftPtr, float *F, int ldF, int M, int R,
+                                                            const int *shiftPtr, Out *F, int ldF, int M, int R,
                                                             int Kp, int flags, int *status) {
     extern __shared__ __align__(16) unsigned char tc_smem_raw[];
     unsigned char *smem = (unsigned char *)(((uintptr_t)tc_smem_raw + 1023) & ~(uintptr_t)1023);
@@ -300,11 +321,10 @@ __global__ void __launch_bounds__(kTcThreads) tc_digit_gemm(const __grid_constan
     bool ok = __syncthreads_and(got ? 1 : 0) && !abortFlag;
     if (!ok && tid == 0 && status) atomicExch(status, (int)kErrTimeout);
     const int S = *shiftPtr;
-    const float scale = __int_as_float((127 - S) << 23);  // 2^-S, S in [-126, 126]
     const uint32_t lanes = (uint32_t)(warp * 32) << 16;
     // (the ring is idle now) the fp32 tile, rows padded against bank conflicts, and for a
     // split tile this CTA's integer sums, [64 columns][128 rows]
-    float *out = reinterpret_cast<float *>(smem);
+    Out *out = reinterpret_cast<Out *>(smem);
     long long *red = reinterpret_cast<long long *>(smem + kTcOutBytes);
     if (ok) {
         // |P_t| <= 128 Kp: up to 2^22 the sum P + 1.5 2^23 is exact and holds P in its low bits
@@ -333,7 +353,7 @@ __global__ void __launch_bounds__(kTcThreads) tc_digit_gemm(const __grid_constan
                 if (split > 1)
                     red[(c0 + j) * kTcBM + tid] = v;
                 else
-                    out[tid * kTcOutLd + c0 + j] = __fmul_rn(__ll2float_rn(v), scale);
+                    out[tid * kTcOutLd + c0 + j] = scaled_sum<Out>(v, S);
             }
         }
     }
@@ -348,9 +368,9 @@ __global__ void __launch_bounds__(kTcThreads) tc_digit_gemm(const __grid_constan
         cz = z * cols;
         if (ok) {
             if (split == 2)
-                add_shares<2>(red, out, cz, tid, scale);
+                add_shares<2>(red, out, cz, tid, S);
             else
-                add_shares<4>(red, out, cz, tid, scale);
+                add_shares<4>(red, out, cz, tid, S);
         }
         __syncwarp();
         cluster_sync_all();  // a CTA's shared memory stays until its peers have read it
@@ -360,7 +380,14 @@ __global__ void __launch_bounds__(kTcThreads) tc_digit_gemm(const __grid_constan
     if (ok) {
         const int c = cz + tid % cols;  // whole rows of the tile, kTcThreads / cols at a time
         for (int r = tid / cols; r < kTcBM && m0 + r < M; r += kTcThreads / cols)
-            if (n0 + c < R) F[(size_t)(m0 + r) * ldF + n0 + c] = out[r * kTcOutLd + c];
+            if (n0 + c < R) {
+                Out v = out[r * kTcOutLd + c], *dst = &F[(size_t)(m0 + r) * ldF + n0 + c];
+                if (sizeof(Out) == 8) {
+                    if (flags & kTcAdd) v += *dst;
+                    if (*reinterpret_cast<const unsigned *>(shiftPtr - 4) == 0x7f800000u) v = (Out)__int_as_float(0x7fffffff);
+                }
+                *dst = v;
+            }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -388,16 +415,21 @@ __device__ __forceinline__ int tc_shift(unsigned maxExpBits) {
 
 // digit planes D_t[r][k] (r < R rows of output, k < K, row stride ldD, zero padded to ldD):
 // B[r][k] = J[r][k] (transpose = 0) or J[k][r] (transpose = 1), J with row stride ldJ
-__global__ void tc_make_digits(const float *J, int ldJ, int R, int K, int ldD, int transpose, const unsigned *maxExp,
-                               int *shiftOut, __nv_bfloat16 *D) {
+// low: the planes of 2^31 (B 2^S - rint(B 2^S)), the part the planes of B round away (shift S + 31)
+__global__ void tc_make_digits(const float *J, int ldJ, int R, int K, int ldD, int transpose, bool low,
+                               const unsigned *maxExp, int *shiftOut, __nv_bfloat16 *D) {
     const int S = tc_shift(*maxExp);
-    if (blockIdx.x == 0 && threadIdx.x == 0) *shiftOut = S;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *shiftOut = low ? S + 31 : S;
     const float scale = __int_as_float((S + 127) << 23);
     const size_t n = (size_t)R * ldD, plane = n;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const int r = (int)(i / ldD), k = (int)(i - (size_t)r * ldD);
         int v = 0;
-        if (k < K) v = __float2int_rn(__fmul_rn(transpose ? J[(size_t)k * ldJ + r] : J[(size_t)r * ldJ + k], scale));
+        if (k < K) {
+            float x = __fmul_rn(transpose ? J[(size_t)k * ldJ + r] : J[(size_t)r * ldJ + k], scale);
+            if (low) x = __fmul_rn(__fsub_rn(x, rintf(x)), 2147483648.f);  // exact: |x - rint x| <= 1/2
+            v = __float2int_rn(x);
+        }
         // balanced base-256 digits: v = d0 + 2^8 d1 + 2^16 d2 + 2^24 d3, d0..d2 in [-128, 127],
         // |d3| <= 64 since |v| < 2^30
 #pragma unroll
@@ -442,50 +474,13 @@ static int grid_for(size_t n) { return (int)std::min<size_t>((n + 255) / 256, (s
 
 using namespace sq103;
 
-extern "C" {
-
-SQ103_API unsigned long long sq103_tc_digits_bytes(int R, int K) {
-    return (unsigned long long)kTcHeader + (unsigned long long)kTcDigits * R * (unsigned long long)ld_pad(K) * 2ull;
-}
-
-SQ103_API unsigned long long sq103_tc_spins_bytes(int m, int K) {
-    return (unsigned long long)m * (unsigned long long)ld_pad(K) * 2ull;
-}
-
-SQ103_API int sq103_tc_make_digits(const float *J, int ldJ, int R, int K, int transpose, void *digits, void *stream) {
-    if (R <= 0 || K <= 0 || K >= (1 << 17) || !J || !digits || (reinterpret_cast<uintptr_t>(digits) & 255))
-        return kErrBadShape;
-    cudaStream_t st = (cudaStream_t)stream;
-    unsigned char *base = static_cast<unsigned char *>(digits);
-    unsigned *maxExp = reinterpret_cast<unsigned *>(base);
-    int *shift = reinterpret_cast<int *>(base + 16);
-    cudaError_t e = cudaMemsetAsync(maxExp, 0, sizeof(unsigned), st);
-    if (e != cudaSuccess) return (int)e;
-    const int rowsJ = transpose ? K : R, colsJ = transpose ? R : K;
-    tc_max_exponent<<<grid_for((size_t)rowsJ * colsJ), 256, 0, st>>>(J, ldJ, rowsJ, colsJ, maxExp);
-    const int ldD = ld_pad(K);
-    tc_make_digits<<<grid_for((size_t)R * ldD), 256, 0, st>>>(J, ldJ, R, K, ldD, transpose, maxExp, shift,
-                                                              reinterpret_cast<__nv_bfloat16 *>(base + kTcHeader));
-    return (int)cudaGetLastError();
-}
-
-SQ103_API int sq103_tc_refresh(const void *digits, int R, int K, const int8_t *q, int ldq, int m, void *spinsBf16,
-                               float *F, int ldF, int flags, int *status, void *stream) {
-    return sq103_tc_refresh_after(digits, R, K, q, ldq, m, spinsBf16, F, ldF, flags, status, false,
-                                  (cudaStream_t)stream);
-}
-
-int sq103_tc_refresh_after(const void *digits, int R, int K, const int8_t *q, int ldq, int m, void *spinsBf16,
-                           float *F, int ldF, int flags, int *status, bool dependent, cudaStream_t st) {
-    if (R <= 0 || K <= 0 || m <= 0 || K >= (1 << 17) || !digits || !q || !spinsBf16 || !F ||
-        (reinterpret_cast<uintptr_t>(digits) & 255) || (reinterpret_cast<uintptr_t>(spinsBf16) & 15) ||
-        (flags & ~3))
-        return kErrBadShape;
+// F = spins (converted, in spinsBf16) times the digits' matrix, behind the kernel last launched on the stream
+template <class Out>
+static int launch_gemm(const void *digits, int R, int K, int m, void *spinsBf16, Out *F, int ldF, int flags,
+                       int *status, cudaStream_t st) {
     auto enc = tensor_map_encoder();
     if (!enc) return kErrBadShape;
     const int ldD = ld_pad(K);
-    launch_dependent(dependent, tc_spins_bf16, dim3(grid_for((size_t)m * ldD)), dim3(256), 0, st, q, ldq, m, K, ldD,
-                     reinterpret_cast<__nv_bfloat16 *>(spinsBf16));
     const unsigned char *base = static_cast<const unsigned char *>(digits);
     CUtensorMap tmA, tmB;
     {
@@ -511,13 +506,13 @@ int sq103_tc_refresh_after(const void *digits, int R, int K, const int8_t *q, in
     // the shared-memory limit is a per-device kernel attribute: set once per device, under a lock
     {
         static std::mutex mu;
-        static bool attrSet[256] = {};
+        static bool attrSet[256] = {};  // (one per instance of this function: per output type)
         int dev = 0;
         cudaError_t e = cudaGetDevice(&dev);
         if (e != cudaSuccess) return (int)e;
         std::lock_guard<std::mutex> lock(mu);
         if (dev < 0 || dev >= 256 || !attrSet[dev]) {
-            e = cudaFuncSetAttribute(tc_digit_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmemBytes);
+            e = cudaFuncSetAttribute(tc_digit_gemm<Out>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmemBytes);
             if (e != cudaSuccess) return (int)e;
             if (dev >= 0 && dev < 256) attrSet[dev] = true;
         }
@@ -543,10 +538,77 @@ int sq103_tc_refresh_after(const void *digits, int R, int K, const int8_t *q, in
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    const cudaError_t le = cudaLaunchKernelEx(&cfg, tc_digit_gemm, tmA, tmB, reinterpret_cast<const int *>(base + 16), F,
+    const cudaError_t le = cudaLaunchKernelEx(&cfg, tc_digit_gemm<Out>, tmA, tmB, reinterpret_cast<const int *>(base + 16), F,
                                               ldF, m, R, ldD, flags, status);
     if (le != cudaSuccess) return (int)le;
     return (int)cudaGetLastError();
+}
+
+extern "C" {
+
+SQ103_API unsigned long long sq103_tc_digits_bytes(int R, int K) {
+    return (unsigned long long)kTcHeader + (unsigned long long)kTcDigits * R * (unsigned long long)ld_pad(K) * 2ull;
+}
+
+SQ103_API unsigned long long sq103_tc_spins_bytes(int m, int K) {
+    return (unsigned long long)m * (unsigned long long)ld_pad(K) * 2ull;
+}
+
+static int make_digits(const float *J, int ldJ, int R, int K, int transpose, bool low, void *digits, void *stream) {
+    if (R <= 0 || K <= 0 || K >= (1 << 17) || !J || !digits || (reinterpret_cast<uintptr_t>(digits) & 255))
+        return kErrBadShape;
+    cudaStream_t st = (cudaStream_t)stream;
+    unsigned char *base = static_cast<unsigned char *>(digits);
+    unsigned *maxExp = reinterpret_cast<unsigned *>(base);
+    int *shift = reinterpret_cast<int *>(base + 16);
+    cudaError_t e = cudaMemsetAsync(maxExp, 0, sizeof(unsigned), st);
+    if (e != cudaSuccess) return (int)e;
+    const int rowsJ = transpose ? K : R, colsJ = transpose ? R : K;
+    tc_max_exponent<<<grid_for((size_t)rowsJ * colsJ), 256, 0, st>>>(J, ldJ, rowsJ, colsJ, maxExp);
+    const int ldD = ld_pad(K);
+    tc_make_digits<<<grid_for((size_t)R * ldD), 256, 0, st>>>(J, ldJ, R, K, ldD, transpose, low, maxExp, shift,
+                                                              reinterpret_cast<__nv_bfloat16 *>(base + kTcHeader));
+    return (int)cudaGetLastError();
+}
+
+SQ103_API int sq103_tc_make_digits(const float *J, int ldJ, int R, int K, int transpose, void *digits, void *stream) {
+    return make_digits(J, ldJ, R, K, transpose, false, digits, stream);
+}
+
+int sq103_tc_make_low_digits(const float *J, int ldJ, int R, int K, void *digits, cudaStream_t st) {
+    return make_digits(J, ldJ, R, K, 0, true, digits, st);
+}
+
+SQ103_API int sq103_tc_refresh(const void *digits, int R, int K, const int8_t *q, int ldq, int m, void *spinsBf16,
+                               float *F, int ldF, int flags, int *status, void *stream) {
+    return sq103_tc_refresh_after(digits, R, K, q, ldq, m, spinsBf16, F, ldF, flags, status, false,
+                                  (cudaStream_t)stream);
+}
+
+int sq103_tc_refresh_after(const void *digits, int R, int K, const int8_t *q, int ldq, int m, void *spinsBf16,
+                           float *F, int ldF, int flags, int *status, bool dependent, cudaStream_t st) {
+    if (R <= 0 || K <= 0 || m <= 0 || K >= (1 << 17) || !digits || !q || !spinsBf16 || !F ||
+        (reinterpret_cast<uintptr_t>(digits) & 255) || (reinterpret_cast<uintptr_t>(spinsBf16) & 15) ||
+        (flags & ~3))
+        return kErrBadShape;
+    const int ldD = ld_pad(K);
+    launch_dependent(dependent, tc_spins_bf16, dim3(grid_for((size_t)m * ldD)), dim3(256), 0, st, q, ldq, m, K, ldD,
+                     reinterpret_cast<__nv_bfloat16 *>(spinsBf16));
+    return launch_gemm<float>(digits, R, K, m, spinsBf16, F, ldF, flags, status, st);
+}
+
+// r (m x R) = the FP64 row sums of q from the digits and the low digits of one matrix
+int sq103_tc_row_sums(const void *digits, const void *lowDigits, int R, int K, const int8_t *q, int ldq, int m,
+                      void *spinsBf16, double *r, int *status, cudaStream_t st) {
+    if (R <= 0 || K <= 0 || m <= 0 || K >= (1 << 17) || !digits || !lowDigits || !q || !spinsBf16 || !r ||
+        (reinterpret_cast<uintptr_t>(digits) & 255) || (reinterpret_cast<uintptr_t>(lowDigits) & 255) ||
+        (reinterpret_cast<uintptr_t>(spinsBf16) & 15))
+        return kErrBadShape;
+    const int ldD = ld_pad(K);
+    launch_dependent(false, tc_spins_bf16, dim3(grid_for((size_t)m * ldD)), dim3(256), 0, st, q, ldq, m, K, ldD,
+                     reinterpret_cast<__nv_bfloat16 *>(spinsBf16));
+    const int rc = launch_gemm<double>(digits, R, K, m, spinsBf16, r, R, 0, status, st);
+    return rc != 0 ? rc : launch_gemm<double>(lowDigits, R, K, m, spinsBf16, r, R, kTcAdd, status, st);
 }
 
 // The dense refresh every path runs (single annealer, batch, server, bench): the
@@ -563,6 +625,18 @@ SQ103_API int sq103_bipartite_refresh_uses_tc(int N0, int N1, int m) {
     if ((long long)N0 * (long long)N1 < (1ll << 20) || m < 1) return 0;
     const long long tiles = (long long)((m + 127) / 128) * ((std::min(N0, N1) + 63) / 64);
     return tiles >= 64 ? 1 : 0;
+}
+
+// Where the bipartite annealer takes its half-step fields and energies to the tensor
+// cores: as above, and from about 80 M products a half-step on (m rounded up to a SIMT
+// tile's 16 rows).  ms, SIMT and tensor cores: 1024 x 1024, m = 64, 64 steps (67 M)
+// 2.89, 3.70; 1100 x 2900, m = 20, 32 steps (102 M) 3.00, 2.15; 1100 x 1100, m = 150
+// (194 M) 3.75, 2.62; 2900 x 2900, m = 30 (269 M) 5.01, 3.07.  Decisions are exact on
+// either, so the spins are the same; a path that returns energies (server) sums them the
+// way the annealer does.
+int sq103_bipartite_tc_pays(int N0, int N1, int m) {
+    if ((long long)N0 * (long long)N1 < (1ll << 20) || m < 1) return 0;
+    return sq103_bipartite_refresh_uses_tc(N0, N1, m) || (double)((m + 15) / 16 * 16) * N0 * N1 >= 8e7;
 }
 
 SQ103_API int sq103_dense_refresh(const float *J, int ldJ, const void *digits, void *spinsBf16, const int8_t *q,

@@ -60,3 +60,45 @@ def test_half_steps_on_tensor_cores_replay(orc):
         assert np.array_equal(np.array([p[0] for p in pairs]), q0)
         assert np.array_equal(np.array([p[1] for p in pairs]), q1)
         assert st["n_mismatch"] == st["n_mismatch_small"], st
+
+
+@pytest.mark.parametrize("N,m,spread", [(1024, 1, 0.0), (1025, 130, 3.0), (1501, 63, 0.0)])
+def test_dense_energies_on_tensor_cores(orc, N, m, spread):
+    """FP64 energies from the exact digit sums, couplings of one and of many magnitudes."""
+    import sqaod_gb300 as sq
+    rng = np.random.default_rng(N + m)
+    W = rng.uniform(-1, 1, (N, N)) * np.exp(spread * rng.standard_normal((N, N)))
+    W = (np.triu(W) + np.triu(W, 1).T).astype(np.float32)
+    for opt, sign in ((sq.minimize, 1.0), (sq.maximize, -1.0)):
+        a = sq.cuda.dense_graph_annealer(W, opt, n_trotters=m)
+        a.seed(1)
+        a.prepare()
+        a.randomize_spin()
+        a.make_solution()
+        q = np.array(a.get_q()).astype(np.float64)
+        h, J, _ = a.get_hamiltonian()
+        J64 = J.astype(np.float64)
+        W64 = sign * W.astype(np.float64)
+        c = -0.25 * (W64.sum() + np.trace(W64))
+        ref = sign * (-c - q @ h.astype(np.float64) - ((q @ J64) * q).sum(1))
+        scale = np.abs(J64).sum()
+        # one FP64 rounding per row sum and the final sums: a few ulp of the total magnitude
+        assert np.max(np.abs(a.get_E64() - ref)) <= 2.0**-50 * scale
+
+
+def test_bipartite_energies_on_tensor_cores():
+    import sqaod_gb300 as sq
+    N0, N1, m = 1200, 1030, 70
+    rng = np.random.default_rng(4)
+    b0, b1, W = (rng.uniform(-1, 1, s).astype(np.float32) for s in (N0, N1, (N1, N0)))
+    a = sq.cuda.bipartite_graph_annealer(b0, b1, W, n_trotters=m)
+    a.seed(1)
+    a.prepare()
+    a.randomize_spin()
+    a.make_solution()
+    q = a.get_q()
+    q0, q1 = np.array([p[0] for p in q]).astype(np.float64), np.array([p[1] for p in q]).astype(np.float64)
+    h0, h1, J, _ = (np.asarray(v, np.float64) for v in a.get_hamiltonian())
+    c = -0.25 * W.astype(np.float64).sum() - 0.5 * (b0.astype(np.float64).sum() + b1.astype(np.float64).sum())
+    ref = -c - q0 @ h0 - q1 @ h1 - ((q0 @ J.T) * q1).sum(1)
+    assert np.max(np.abs(a.get_E64() - ref)) <= 2.0**-50 * np.abs(J).sum()
