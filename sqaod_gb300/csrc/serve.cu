@@ -660,7 +660,7 @@ private:
             double *scratch = (double *)((unsigned char *)r->dt.q + al((size_t)m * N));
             if (r->digits) {  // as the single annealer; the low digits in a shared scratch
                 low_.ensure(sq103_tc_digits_bytes(N, N));
-                SQ_CHECK(sq103_tc_make_low_digits(r->dt.J, r->dt.ldJ, N, N, low_.p, st_.get()));
+                SQ_CHECK(sq103_tc_make_low_digits(r->dt.J, r->dt.ldJ, N, N, r->digits, low_.p, st_.get()));
                 SQ_CHECK(sq103_tc_row_sums(r->digits, low_.p, N, N, r->dt.q, N, m, r->spinsBf16, scratch, r->dStatus,
                                            st_.get()));
                 SQ_CHECK(sq103_dense_energy_of_sums(scratch, r->dt.h, r->c64, r->dt.q, N, m, r->optimize, r->dE,
@@ -682,7 +682,7 @@ private:
                     bf16 = bf16_.p;
                 }
                 low_.ensure(sq103_tc_digits_bytes(r->N1, r->N0));
-                SQ_CHECK(sq103_tc_make_low_digits(r->bt.J, r->N0, r->N1, r->N0, low_.p, st_.get()));
+                SQ_CHECK(sq103_tc_make_low_digits(r->bt.J, r->N0, r->N1, r->N0, digits, low_.p, st_.get()));
                 SQ_CHECK(sq103_tc_row_sums(digits, low_.p, r->N1, r->N0, r->bt.q0, r->N0, m, bf16, scratch, r->dStatus,
                                            st_.get()));
                 SQ_CHECK(sq103_bipartite_energy_of_sums(scratch, r->bt.h0, r->bt.h1, r->c64, r->bt.q0, r->bt.q1, r->N0,

@@ -358,7 +358,7 @@ public:
             // energies: 15.9 ms with the SIMT double-float sums (1.13 ms of it), 14.7 this way.
             if (!lowMade_) {
                 d_low_.ensure(sq103_tc_digits_bytes(N_, N_));
-                SQ_CHECK(sq103_tc_make_low_digits(d_J_.p, ldJ_, N_, N_, d_low_.p, st_.get()));
+                SQ_CHECK(sq103_tc_make_low_digits(d_J_.p, ldJ_, N_, N_, d_digits_.p, d_low_.p, st_.get()));
                 lowMade_ = true;
             }
             SQ_CHECK(sq103_tc_row_sums(d_digits_.p, d_low_.p, N_, N_, d_q_.p, N_, m_, d_Abf_.p, d_r_.p, d_status_.p,
@@ -914,7 +914,7 @@ public:
         else if (useTc()) {  // as DenseAnnealer::calculate_E
             if (!lowMade_) {
                 d_low1_.ensure(sq103_tc_digits_bytes(N1_, N0_));
-                SQ_CHECK(sq103_tc_make_low_digits(d_J_.p, N0_, N1_, N0_, d_low1_.p, st_.get()));
+                SQ_CHECK(sq103_tc_make_low_digits(d_J_.p, N0_, N1_, N0_, d_digits1_.p, d_low1_.p, st_.get()));
                 lowMade_ = true;
             }
             SQ_CHECK(sq103_tc_row_sums(d_digits1_.p, d_low1_.p, N1_, N0_, d_q0_.p, N0_, m_, d_Abf_.p, d_r_.p,
@@ -2228,7 +2228,7 @@ public:
         E64_.ensure(in.m);
         if (in.digits.p) {  // as the single annealer; the low digits in a shared scratch
             low_.ensure(sq103_tc_digits_bytes(in.N, in.N));
-            SQ_CHECK(sq103_tc_make_low_digits(in.J, in.ldJ, in.N, in.N, low_.p, st_.get()));
+            SQ_CHECK(sq103_tc_make_low_digits(in.J, in.ldJ, in.N, in.N, in.digits.p, low_.p, st_.get()));
             SQ_CHECK(sq103_tc_row_sums(in.digits.p, low_.p, in.N, in.N, in.q, in.N, in.m, in.Abf.p, r_.p, in.status,
                                        st_.get()));
             SQ_CHECK(sq103_dense_energy_of_sums(r_.p, in.h, in.c64, in.q, in.N, in.m, optimize_[i], E64_.p, nullptr,

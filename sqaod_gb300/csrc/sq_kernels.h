@@ -14,8 +14,9 @@ extern "C" int sq103_tc_refresh_after(const void *digits, int R, int K, const in
                                       cudaStream_t st);
 
 extern "C" int sq103_bipartite_tc_pays(int N0, int N1, int m);
-// the planes of what the digits of J (R x K, row stride ldJ) round away (the layout and size of its digits)
-extern "C" int sq103_tc_make_low_digits(const float *J, int ldJ, int R, int K, void *digits, cudaStream_t st);
+// the planes of what `high`, the digits of J (R x K, row stride ldJ), round away (same layout and size)
+extern "C" int sq103_tc_make_low_digits(const float *J, int ldJ, int R, int K, const void *high, void *digits,
+                                        cudaStream_t st);
 extern "C" int sq103_tc_row_sums(const void *digits, const void *lowDigits, int R, int K, const int8_t *q, int ldq,
                                  int m, void *spinsBf16, double *r, int *status, cudaStream_t st);
 // the FP64 energies from the row sums r (m x N of q J; m x N1 of q0 J^T)

@@ -396,16 +396,20 @@ __global__ void __launch_bounds__(kTcThreads) tc_digit_gemm(const __grid_constan
                      : "memory");
 }
 
-// largest biased exponent of the matrix (atomicMax over the float bit patterns)
-__global__ void tc_max_exponent(const float *B, int ld, int rows, int cols, unsigned *out) {
+// largest biased exponent of the matrix (atomicMax over the float bit patterns, one per
+// block: one per warp of a full grid took 20 us on the one word)
+__global__ void __launch_bounds__(256) tc_max_exponent(const float *B, int ld, int rows, int cols, unsigned *out) {
+    __shared__ unsigned top;
+    if (threadIdx.x == 0) top = 0u;
+    __syncthreads();
     unsigned e = 0;
-    const size_t n = (size_t)rows * cols;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const size_t r = i / cols, c = i - r * cols;
-        e = max(e, __float_as_uint(B[r * ld + c]) & 0x7f800000u);
-    }
+    for (int r = blockIdx.x; r < rows; r += gridDim.x)
+#pragma unroll 4
+        for (int c = threadIdx.x; c < cols; c += 256) e = max(e, __float_as_uint(B[(size_t)r * ld + c]) & 0x7f800000u);
     e = __reduce_max_sync(0xffffffffu, e);
-    if ((threadIdx.x & 31) == 0) atomicMax(out, e);
+    if ((threadIdx.x & 31) == 0) atomicMax(&top, e);
+    __syncthreads();
+    if (threadIdx.x == 0) atomicMax(out, top);
 }
 
 // shift S: |B| < 2^(E - 126) for the largest biased exponent E, so |B 2^S| < 2^30 with S = 156 - E
@@ -417,13 +421,17 @@ __device__ __forceinline__ int tc_shift(unsigned maxExpBits) {
 // B[r][k] = J[r][k] (transpose = 0) or J[k][r] (transpose = 1), J with row stride ldJ
 // low: the planes of 2^31 (B 2^S - rint(B 2^S)), the part the planes of B round away (shift S + 31)
 __global__ void tc_make_digits(const float *J, int ldJ, int R, int K, int ldD, int transpose, bool low,
-                               const unsigned *maxExp, int *shiftOut, __nv_bfloat16 *D) {
+                               const unsigned *maxExp, unsigned *header, __nv_bfloat16 *D) {
     const int S = tc_shift(*maxExp);
-    if (blockIdx.x == 0 && threadIdx.x == 0) *shiftOut = low ? S + 31 : S;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        if (low) header[0] = *maxExp;  // (the planes of B hold it already)
+        header[4] = (unsigned)(low ? S + 31 : S);
+    }
     const float scale = __int_as_float((S + 127) << 23);
-    const size_t n = (size_t)R * ldD, plane = n;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const int r = (int)(i / ldD), k = (int)(i - (size_t)r * ldD);
+    const size_t plane = (size_t)R * ldD;
+    for (int r = blockIdx.x; r < R; r += gridDim.x)
+    for (int k = threadIdx.x; k < ldD; k += blockDim.x) {
+        const size_t i = (size_t)r * ldD + k;
         int v = 0;
         if (k < K) {
             float x = __fmul_rn(transpose ? J[(size_t)k * ldJ + r] : J[(size_t)r * ldJ + k], scale);
@@ -554,29 +562,31 @@ SQ103_API unsigned long long sq103_tc_spins_bytes(int m, int K) {
     return (unsigned long long)m * (unsigned long long)ld_pad(K) * 2ull;
 }
 
-static int make_digits(const float *J, int ldJ, int R, int K, int transpose, bool low, void *digits, void *stream) {
+static int make_digits(const float *J, int ldJ, int R, int K, int transpose, const void *high, void *digits, void *stream) {
     if (R <= 0 || K <= 0 || K >= (1 << 17) || !J || !digits || (reinterpret_cast<uintptr_t>(digits) & 255))
         return kErrBadShape;
     cudaStream_t st = (cudaStream_t)stream;
     unsigned char *base = static_cast<unsigned char *>(digits);
-    unsigned *maxExp = reinterpret_cast<unsigned *>(base);
-    int *shift = reinterpret_cast<int *>(base + 16);
-    cudaError_t e = cudaMemsetAsync(maxExp, 0, sizeof(unsigned), st);
-    if (e != cudaSuccess) return (int)e;
-    const int rowsJ = transpose ? K : R, colsJ = transpose ? R : K;
-    tc_max_exponent<<<grid_for((size_t)rowsJ * colsJ), 256, 0, st>>>(J, ldJ, rowsJ, colsJ, maxExp);
-    const int ldD = ld_pad(K);
-    tc_make_digits<<<grid_for((size_t)R * ldD), 256, 0, st>>>(J, ldJ, R, K, ldD, transpose, low, maxExp, shift,
-                                                              reinterpret_cast<__nv_bfloat16 *>(base + kTcHeader));
+    unsigned *header = reinterpret_cast<unsigned *>(base);
+    if (!high) {
+        cudaError_t e = cudaMemsetAsync(header, 0, sizeof(unsigned), st);
+        if (e != cudaSuccess) return (int)e;
+        const int rowsJ = transpose ? K : R, colsJ = transpose ? R : K;
+        tc_max_exponent<<<std::min(rowsJ, 152 * 4), 256, 0, st>>>(J, ldJ, rowsJ, colsJ, header);
+    }
+    tc_make_digits<<<std::min(R, 152 * 16), 256, 0, st>>>(J, ldJ, R, K, ld_pad(K), transpose, high != nullptr,
+                                                          high ? static_cast<const unsigned *>(high) : header, header,
+                                                          reinterpret_cast<__nv_bfloat16 *>(base + kTcHeader));
     return (int)cudaGetLastError();
 }
 
 SQ103_API int sq103_tc_make_digits(const float *J, int ldJ, int R, int K, int transpose, void *digits, void *stream) {
-    return make_digits(J, ldJ, R, K, transpose, false, digits, stream);
+    return make_digits(J, ldJ, R, K, transpose, nullptr, digits, stream);
 }
 
-int sq103_tc_make_low_digits(const float *J, int ldJ, int R, int K, void *digits, cudaStream_t st) {
-    return make_digits(J, ldJ, R, K, 0, true, digits, st);
+int sq103_tc_make_low_digits(const float *J, int ldJ, int R, int K, const void *high, void *digits, cudaStream_t st) {
+    if (!high) return kErrBadShape;
+    return make_digits(J, ldJ, R, K, 0, high, digits, st);
 }
 
 SQ103_API int sq103_tc_refresh(const void *digits, int R, int K, const int8_t *q, int ldq, int m, void *spinsBf16,
