@@ -1,22 +1,22 @@
 // dense_multi.cu -- one CTA per trotter: the dense coloring / SA sweep of one
 // large instance across the whole GPU (cooperative launch, all CTAs resident).
 //
-// It runs the same trials, in the same colour order and with the same fp32
-// arithmetic, as the one-CTA-per-instance kernel in dense.cu, so both give
-// bit-identical spins and fields.
+// It runs the same trials in the same colour order as the one-CTA-per-instance
+// kernel in dense.cu, updates the fields in the same order with the same
+// rounding, and takes the same (exact) decisions, so both give bit-identical
+// spins and fields.
 //
-// Per CTA (trotter y), 256 threads:
+// Per CTA (trotter y), 256 threads (224 where four CTAs share an SM):
 //   warp 0  decider: the trotter's trials in batches of 32 iterations, lane i =
-//           iteration g0 + i.  A batch is decided in rounds: every undecided
-//           lane evaluates its trial with its current field and neighbour
-//           spins; the lowest accepting lane is final (all undecided lanes
-//           below it reject), and the lanes above it add d * J[x_f][x_i] to
-//           their fields and flip their spin copy when they share its site.
+//           iteration g0 + i.  A lane holds z = rate dE - L, L = -ln u (the trial
+//           accepts when z < 0) and a bound on its fp32 error.  A batch is decided
+//           in rounds: the lowest accepting lane is final (all undecided lanes
+//           below it reject), and a lane above it adds its product with
+//           d J[x_f][x_i] to z and changes signs when it shares the flipped site.
 //           A batch takes (accepted flips + 1) rounds instead of 32 sequential
 //           trials.  The batch's fields start from the resident row F[y][:],
 //           which the updaters keep one batch behind, plus the previous
-//           batch's flips d_f * J[x_f][x_i], gathered at the batch boundary and
-//           added after the next batch's ghost-row update.
+//           batch's flips d_f * J[x_f][x_i].
 //           Decisions are published as one 64-bit word per batch (accept
 //           bits, decided count, batch tag) with a single relaxed store after
 //           every accepting round and at the end of the batch: a reader that
@@ -25,18 +25,21 @@
 //   warp 1  helper: polls the two neighbours' accept words (both neighbours,
 //           two words ahead, in one round trip) and copies them into shared
 //           memory.
-//   warps 2-3 prefetchers, alternate batches: this trotter's own sites,
-//           uniforms and step constants, the in-batch gathers J[x_j][x_i]
-//           (j < i) for the lanes j predicted to accept, the neighbours' sites of the same iterations (a ring of
+//   warps 2-3 prefetchers, alternate batches: this trotter's own trials (PreTrial),
+//           the in-batch gathers J[x_j][x_i] (j < i) for the lanes j predicted to
+//           accept, the neighbours' sites of the same iterations (a ring of
 //           sites and one hashed-site bitmap per batch), and per lane the
-//           neighbour iterations of this and the previous batch that hit its
+//           neighbour iterations of this and the two previous batches that hit its
 //           site, into a ring of kPre batch buffers with a ready tag each.
-//   warps 4-6 updaters: F[y][:] += d * J[x][:] for the flips of the previous
+//   warps 4-6 (4-5) updaters: F[y][:] += d * J[x][:] for the flips of the previous
 //           batch, in trial order, while the decider works on the next one.
-//   warp 7  exact decisions: a trial whose fp32 outcome the rounding of the
+//   last warp exact decisions: a trial whose fp32 outcome the rounding of the
 //           resident field could change is decided in FP64 from its exact field
 //           (sq_common.cuh); the warp sleeps on a named barrier between requests
 //           and answers through a shared word the decider waits on (bounded).
+// What bounds it: the decider's chain, about 2500 cycles a batch without flips and
+// 1000 per flip at N = 4096, m = 256 (two CTAs per SM), at some ten cycles an
+// instruction; DRAM is idle and issue slots are three quarters free.
 // Colour order: trial (y, k) must see neighbour n after every neighbour trial
 // that precedes it (iteration < k, or = k when n's colour phase comes first:
 // even trotters, then trotter m-1 if m is odd, then odd trotters).  The
