@@ -472,8 +472,8 @@ def run_batched(args, world):
     torch.cuda.synchronize()
     t_add = time.perf_counter() - t_add
     t_tune = time.perf_counter()
-    # trotters per CTA: the one-CTA-per-trotter size limit (default 1024, from whole-run measurements;
-    # --autotune-routing times 8 steps per candidate instead); then the staging size, by measurement
+    # trotters per CTA: the one-CTA-per-trotter size limit (default 1024, below which the library takes
+    # smaller instances along; --autotune-routing times 8 steps per candidate instead); then the staging size, by measurement
     if args.autotune_routing and args.multicta_min_n is None:
         routing = b.autotune_routing(8)
     else:
@@ -782,8 +782,8 @@ def run_bf(args, world):
                          "note": "achieved = the reference formulation's arithmetic (X.W per tile plus the row "
                                  "dot, 2N^2+2N flops per state) per second; peak = the measured dense bf16 "
                                  "tensor rate, the ceiling of that formulation as a tensor-core GEMM.  This "
-                                 "search does not run the GEMM: 2^14-entry tables, about 3 lookups and adds "
-                                 "per state, issue-bound; frac > 1 means above the GEMM formulation's ceiling"},
+                                 "search does not run the GEMM: one packed addition and one three-input minimum "
+                                 "per two states, issue-bound; frac > 1 means above the GEMM formulation's ceiling"},
             "e2e": {"value": nStates / e2e_s, "unit": "states/s", "seconds": e2e_s, "h2d_bytes_per_step": W.nbytes,
                     "d2h_bytes_per_step": int(len(E_api) * 4 + np.asarray(x_api).size),
                     "Emin": float(np.min(E_api))},
@@ -850,7 +850,7 @@ def main():
     ap.add_argument("--autotune-routing", action="store_true",
                     help="batched mode: choose the one-CTA-per-trotter size limit by timing 8 steps per candidate")
     ap.add_argument("--multicta-min-n", type=int, default=None,
-                    help="batched mode: instances of at least this N take the one-CTA-per-trotter sweep (default 1024)")
+                    help="batched mode: instances of at least this N take the one-CTA-per-trotter sweep (default: the library's choice)")
     ap.add_argument("--cpu-leg", action="store_true", help="internal: time the CPU reference annealer alone")
     ap.add_argument("--min-seconds", type=float, default=CPU_LEG_MIN_SECONDS, help="--cpu-leg: minimum duration")
     ap.add_argument("--cpu-workers", type=int, default=0, help="--cpu-leg: host threads (0: all)")
@@ -1000,7 +1000,7 @@ def main():
         r_ms = float(sum(a.elapsed_time(b) for a, b in zip(mids, ends))) / K
         flops = 2.0 * N * N * m
         refresh_info = {"kernel": "tc_digit_gemm (tcgen05, 4 bf16 digit planes, exact)" if use_tc
-                        else "field_gemm_kernel (fp32 SIMT)", "ms_per_launch": r_ms,
+                        else "bip_field_kernel (fp32 SIMT)", "ms_per_launch": r_ms,
                         "algorithmic_tflops": flops / (r_ms / 1e3) / 1e12,
                         "mma_tflops": (4.0 if use_tc else 1.0) * flops / (r_ms / 1e3) / 1e12}
 

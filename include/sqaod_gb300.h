@@ -490,7 +490,8 @@ SQ103_API int sq103_dense_batch_set_schedule(void *handle, const float *G, const
 SQ103_API int sq103_dense_batch_prepare(void *handle);
 /* Instances of at least N spins (m >= 2, fitting the device) are stepped by the
  * one-CTA-per-trotter sweep in packed cooperative launches, the rest by the
- * persistent batch kernel; both give the same results.  Default 1024; 0 keeps
+ * persistent batch kernel; both give the same results.  Default 1024, and
+ * the packed launches take smaller ones along where that is faster; 0 keeps
  * every instance on the persistent kernel.  Takes effect at the next prepare. */
 SQ103_API int sq103_dense_batch_set_multicta_min_n(void *handle, int N);
 /* instances on the one-CTA-per-trotter sweep since the last prepare */
@@ -612,7 +613,7 @@ SQ103_API int sq103_server_result(void *handle, int id, double *E, int capE, int
 SQ103_API int sq103_server_stats(void *handle, int *queued, int *active, int *done,
                                  unsigned long long *bytesInUse);
 /* at most n large instances admitted at a time (default 64; dense: one CTA per
- * trotter, packed up to 16 per launch; bipartite: per-instance kernels) */
+ * trotter, packed up to 64 per launch; bipartite: per-instance kernels) */
 SQ103_API int sq103_server_set_large_limit(void *handle, int n);
 /* Fault injection from the host (tests; no counterpart in the reference): writes
  * `value` into the status word of active dense request `id`, in stream order, as a
