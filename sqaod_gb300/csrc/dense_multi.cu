@@ -62,6 +62,7 @@
 // the prefetchers' three to seven generators two rounds at a time: N = 1000, m = 250
 // 5.75 -> 5.56 ms, 128 uneven instances 27.1 -> 26.2 ms (instruction fetch)
 #define SQ103_PHILOX_UNROLL 2
+#include "mc_trial.h"
 #include "sq_common.cuh"
 #include "sq_kernels.h"
 
@@ -543,11 +544,9 @@ __global__ void __launch_bounds__(mc_threads(kPerSm), kPerSm) dense_sweep_multi(
             x = xN;
             const float *jg = Jg + buf * kJgStride + lane * 33;
 
-            // The trial accepts when z = rate dE - L < 0.  z = zA - ring, zA = cz q (h + 2F) - L
-            // and ring = cb q (qL + qR); unknown neighbour spins leave it in [z - sp, z + sp].
-            // A lane is decided when that interval lies outside [-tol, tol], the fp32 error
-            // bound (sq_common.cuh; the ring's part four times as wide here, for the sums kept
-            // over a batch's flips).  A flip adds cz q 2 d J to zA, and changes the signs of a
+            // The trial's decision: mc_trial.h.  The tolerance is the fp32 error bound of
+            // sq_common.cuh, the ring's part four times as wide here, for the sums kept over a
+            // batch's flips.  A flip adds cz q 2 d J to zA, and changes the signs of a
             // later trial at its site.  (A round that evaluated dE anew, with up to four
             // evaluations for unknown spins, took 970 cycles at two CTAs per SM; the decider is
             // the critical path, at 10 cycles an instruction.  N = 4096, m = 256, 64 steps: 24.2
@@ -578,8 +577,8 @@ __global__ void __launch_bounds__(mc_threads(kPerSm), kPerSm) dense_sweep_multi(
                     first = false;
                 }
                 const float z = zA - ring_;
-                const unsigned accM = __ballot_sync(FULL, z + sp < -tol) & pending;
-                const unsigned blkM = __ballot_sync(FULL, z - sp <= tol) & pending & ~accM;
+                const unsigned accM = __ballot_sync(FULL, mc_accepts(z, sp, tol)) & pending;
+                const unsigned blkM = __ballot_sync(FULL, mc_open(z, sp, tol)) & pending & ~accM;
                 const int fa = accM ? __ffs(accM) - 1 : 32;
                 const int fb = blkM ? __ffs(blkM) - 1 : 32;
                 if (fb < fa) {
@@ -607,7 +606,7 @@ __global__ void __launch_bounds__(mc_threads(kPerSm), kPerSm) dense_sweep_multi(
                             aborted = true;
                             break;
                         }
-                        if (lane == fb) zA = (S.exBits >> ((sum + 2) >> 1)) & 1 ? -3e38f : 3e38f;
+                        if (lane == fb) mc_answer((S.exBits >> ((sum + 2) >> 1)) & 1, zA, tol);
                         continue;
                     }
                     // fb waits for its neighbour trials
@@ -974,12 +973,11 @@ __global__ void __launch_bounds__(mc_threads(kPerSm), kPerSm) dense_sweep_multi(
                 PreTrial tr;
                 tr.x = x;
                 tr.h = hs[x];
-                tr.L = fminf(neg_log_unit(u), 1e30f);
-                tr.cz = sc.rate * (sa ? 2.f : sc.twoDivM);
-                // (0 for SA; G = 0 or beta = 0 make coef infinite: its sign then decides)
-                const float cb = sc.rate * sc.coef;
-                tr.cb = sa ? 0.f : isfinite(cb) ? cb : copysignf(1e30f, sc.coef);
-                tr.tolC = 4e-6f * fabsf(tr.cb) + 2e-6f + 1e-6f * tr.L;
+                const McConst c = mc_const(sa, sc.twoDivM, sc.coef, sc.rate, neg_log_unit(u));
+                tr.L = c.L;
+                tr.cz = c.cz;
+                tr.cb = c.cb;
+                tr.tolC = c.tolC;
                 tr.u = u;
                 tr.cand = cands;
                 pre[buf * 32 + lane] = tr;
