@@ -35,7 +35,15 @@ struct BipFixed {
     int side;          // the moving side
     float G, beta;
     const double *J64, *h64;
+    // the digit planes' shift S when the fields come from them: their couplings are
+    // rounded to multiples of 2^-S, so a field is off by up to NB 2^-(S + 1)
+    const int *shift = nullptr;
+    float one = 1.f;  // the constant of the trials' tolerance (trial_xtol)
 };
+
+__device__ __forceinline__ float bip_tol_one(const BipFixed &B) {  // S in [-126, 126]
+    return B.shift ? __fmaf_rn(65536.f * (float)B.NB, __int_as_float((126 - *B.shift) << 23), 1.f) : 1.f;
+}
 
 __device__ __forceinline__ double bip_exact_field(const BipFixed &B, int y, int i) {
     const int8_t *qb = B.qB + (size_t)y * B.NB;
@@ -95,7 +103,7 @@ __device__ __forceinline__ int bip_trial(bool active, int8_t *qA, const float *F
             dE = bip_sqa_dE(qyx, h[i], F[o], qL, qR, sc.twoDivM, sc.coef);
         }
         L = neg_log_unit(u);
-        acc = metropolis_log(dE, sc.rate, L, trial_xtol(tol, h[i], F[o], L), nearT);
+        acc = metropolis_log(dE, sc.rate, L, trial_xtol(tol, h[i], F[o], L, B.one), nearT);
     }
     auto decide = [&](double Fx) {
         const double hx = bip_exact_h(B, h, i);
@@ -135,6 +143,7 @@ __global__ void __launch_bounds__(256) bip_flip_phase(int8_t *qA, const float *F
     const int t = (int)(idx / Ns), i = (int)(idx - (long long)t * Ns);
     B.G = G;
     B.beta = beta;
+    B.one = bip_tol_one(B);
     const int acc = bip_trial<true>(active, qA, F, h, Ns, m, yb + t * ys, i, seed, step, tag, sc, algo, trace, bitBase, B);
     if (accepted) {
         unsigned ballot = __ballot_sync(0xffffffffu, acc);
@@ -164,6 +173,7 @@ __global__ void __launch_bounds__(256) bip_flip_half(int8_t *qA, const float *F,
     const StepConst sc = step_const(algo, m, G, beta);
     B.G = G;
     B.beta = beta;
+    B.one = bip_tol_one(B);
     const int pairs = m / 2;
     unsigned long long acc = 0;
     // before the fields are there: the step's constants and the draws of the thread's first pair
@@ -417,7 +427,8 @@ extern "C" SQ103_API int sq103_bipartite_anneal(const sq103_bipartite_task *task
             int8_t *qA = side ? T.q1 : T.q0;
             float *F = side ? T.F1 : T.F0;
             const float *h = side ? T.h1 : T.h0;
-            if (T.digits1 && T.digits0) {
+            const bool tc = T.digits1 && T.digits0;
+            if (tc) {
                 // side 1: F1 = q0 J^T (rows of J, K = N0); side 0: F0 = q1 J (rows of J^T, K = N1)
                 const int rc = side ? sq103_tc_refresh_after(T.digits1, T.N1, T.N0, T.q0, T.N0, m, T.spinsBf16, F,
                                                              T.N1, 0, T.status, dependent, st)
@@ -430,7 +441,8 @@ extern "C" SQ103_API int sq103_bipartite_anneal(const sq103_bipartite_task *task
             dependent = true;
             const uint32_t tag = (uint32_t)(sa ? kTagBipSA : kTagBipSweep) | ((uint32_t)side << 8);
             const BipFixed fixedSide{T.J, T.N0, side ? T.q0 : T.q1, side ? T.N0 : T.N1, side, 0.f, 0.f, T.J64,
-                                     side ? T.h1_64 : T.h0_64};
+                                     side ? T.h1_64 : T.h0_64,
+                                     tc ? sq103_tc_shift_of(side ? T.digits1 : T.digits0) : nullptr};
             if (!sa) {
                 // every colour phase of the half-step in one launch (blocks own whole columns)
                 const int C = flip_half_cols(m);

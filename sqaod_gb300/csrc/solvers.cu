@@ -1044,7 +1044,7 @@ private:
         SQ_CHECK(cudaMemsetAsync(d_status_.p, 0, sizeof(int), st_.get()));
         // large problems may compute the half-step fields on the tensor cores from
         // digit planes of J (for F1) and of J^T (for F0): made with the problem, used
-        // when the trotter count also allows (sq103_bipartite_refresh_uses_tc)
+        // when the trotter count and the couplings also allow (useTc, tcFields)
         if ((long long)N0_ * N1_ >= (1ll << 20)) {
             d_digits1_.ensure(sq103_tc_digits_bytes(N1_, N0_));
             d_digits0_.ensure(sq103_tc_digits_bytes(N0_, N1_));
@@ -1054,7 +1054,12 @@ private:
         }
     }
 
-    // half-step fields and energies on the tensor cores
+    // half-step fields on the tensor cores: the largest shapes always, the others only
+    // when the digits are as fine as the fp32 couplings for every spin
+    bool tcFields() const {
+        return useTc() && (!uneven_ || sq103_bipartite_refresh_uses_tc(N0_, N1_, m_));
+    }
+    // energies on the tensor cores
     bool useTc() const { return d_digits1_.p && sq103_bipartite_tc_pays(N0_, N1_, m_); }
 
     void makeDigits() {
@@ -1062,6 +1067,10 @@ private:
         if (!d_digits1_.p) return;
         SQ_CHECK(sq103_tc_make_digits(d_J_.p, N0_, N1_, N0_, 0, d_digits1_.p, st_.get()));
         SQ_CHECK(sq103_tc_make_digits(d_J_.p, N0_, N0_, N1_, 1, d_digits0_.p, st_.get()));
+        d_uneven_.ensure(1);
+        SQ_CHECK(sq103_tc_check_even(d_J_.p, N0_, N1_, N0_, d_digits1_.p, d_uneven_.p, st_.get()));
+        SQ_CHECK(cudaMemcpyAsync(&uneven_, d_uneven_.p, sizeof(int), cudaMemcpyDeviceToHost, st_.get()));
+        st_.sync();
     }
 
     void allocFP64() {
@@ -1135,7 +1144,7 @@ private:
         t.J64 = fp64_ ? d_J64_.p : nullptr;
         t.h0_64 = fp64_ ? d_h0_64_.p : nullptr;
         t.h1_64 = fp64_ ? d_h1_64_.p : nullptr;
-        const bool tc = useTc();
+        const bool tc = tcFields();
         t.digits1 = tc ? d_digits1_.p : nullptr;
         t.digits0 = tc ? d_digits0_.p : nullptr;
         t.spinsBf16 = tc ? d_Abf_.p : nullptr;
@@ -1167,7 +1176,8 @@ private:
     DevBuf<unsigned char> d_digits1_, d_digits0_, d_Abf_;  // tensor-core half-step fields
     DevBuf<unsigned char> d_low1_;                         // tensor-core energies
     bool lowMade_ = false;
-    DevBuf<int> d_status_;
+    int uneven_ = 0;  // the digits are coarser than fp32 for some spin
+    DevBuf<int> d_status_, d_uneven_;
     DevBuf<int8_t> d_q0_, d_q1_;
     DevBuf<unsigned long long> d_acc_;
     DevBuf<long long> d_ring_;

@@ -208,10 +208,11 @@ __device__ __forceinline__ int metropolis_log(float dE, float rate, float L, flo
     return (dE < 0.f || x < L) ? 1 : 0;
 }
 
-// x tolerance of a trial: kF (|h| + |Fp| + 1) + kC + 2.4e-7 L (Fp = 2F dense, F bipartite)
-__device__ __forceinline__ float trial_xtol(const DecisionTol &t, float h, float Fp, float L) {
+// x tolerance of a trial: kF (|h| + |Fp| + one) + kC + 2.4e-7 L (Fp = 2F dense, F bipartite).
+// one: 1, and for fields with an error e of their own (digit planes) 1 + 2^16 e.
+__device__ __forceinline__ float trial_xtol(const DecisionTol &t, float h, float Fp, float L, float one = 1.f) {
     const float base = __fadd_rn(t.kC, __fmul_rn(2.4e-7f, fminf(L, 1e30f)));
-    return __fmaf_rn(t.kF, __fadd_rn(__fadd_rn(fabsf(h), fabsf(Fp)), 1.f), base);
+    return __fmaf_rn(t.kF, __fadd_rn(__fadd_rn(fabsf(h), fabsf(Fp)), one), base);
 }
 
 // The exact local field sum_j J[j] q[j] (q = +-1) as an integer sum: every J[j]

@@ -449,6 +449,41 @@ __global__ void tc_make_digits(const float *J, int ldJ, int R, int K, int ldD, i
     }
 }
 
+// Sets *uneven when the digits are too coarse for some row or column of J (R x K): one
+// that holds a coupling the digits round and whose largest is below 2^24 quanta 2^-S, so
+// that the rounding exceeds the fp32 rounding of that largest coupling.  Couplings of one
+// magnitude, and integers below 2^30, are even; one coupling far above the rest makes the
+// other rows uneven.  Blocks below rowBlocks: a warp per row; the rest: 32 columns each.
+__global__ void __launch_bounds__(256) tc_check_even(const float *J, int ld, int R, int K, const unsigned *maxExp,
+                                                     int rowBlocks, int *uneven) {
+    __shared__ unsigned top[8][32];
+    const unsigned E = *maxExp, coarse = 5u << 23;
+    const float scale = __int_as_float((tc_shift(E) + 127) << 23);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned e = 0;  // the largest exponent, bit 0 set when a value is rounded
+    auto take = [&](float v) {
+        const float x = __fmul_rn(v, scale);
+        const unsigned b = __float_as_uint(v) & 0x7f800000u;
+        e = max(e & ~1u, b) | (e & 1u) | (x != rintf(x) ? 1u : 0u);
+    };
+    if ((int)blockIdx.x < rowBlocks) {
+        const int r = (int)blockIdx.x * 8 + warp;
+        if (r < R)
+#pragma unroll 4
+            for (int c = lane; c < K; c += 32) take(J[(size_t)r * ld + c]);
+        e = __reduce_max_sync(0xffffffffu, e & ~1u) | __reduce_or_sync(0xffffffffu, e & 1u);
+    } else {
+        const int c = ((int)blockIdx.x - rowBlocks) * 32 + lane;
+        if (c < K)
+#pragma unroll 4
+            for (int r = warp; r < R; r += 8) take(J[(size_t)r * ld + c]);
+        top[warp][lane] = e;
+        __syncthreads();
+        for (int w = 0; w < 8; ++w) e = max(e & ~1u, top[w][lane] & ~1u) | ((e | top[w][lane]) & 1u);
+    }
+    if (((e & 1u) && (e & ~1u) + coarse < E) || E == 0x7f800000u) *uneven = 1;
+}
+
 // spins (m x K int8, row stride ldq) -> bf16 (m x ldA), zero beyond K
 __global__ void tc_spins_bf16(const int8_t *q, int ldq, int m, int K, int ldA, __nv_bfloat16 *A) {
     pdl_trigger();
@@ -584,6 +619,16 @@ SQ103_API int sq103_tc_make_digits(const float *J, int ldJ, int R, int K, int tr
     return make_digits(J, ldJ, R, K, transpose, nullptr, digits, stream);
 }
 
+int sq103_tc_check_even(const float *J, int ldJ, int R, int K, const void *digits, int *uneven, cudaStream_t st) {
+    if (R <= 0 || K <= 0 || !J || !digits || !uneven) return kErrBadShape;
+    const cudaError_t e = cudaMemsetAsync(uneven, 0, sizeof(int), st);
+    if (e != cudaSuccess) return (int)e;
+    const int rowBlocks = (R + 7) / 8;
+    tc_check_even<<<rowBlocks + (K + 31) / 32, 256, 0, st>>>(J, ldJ, R, K, static_cast<const unsigned *>(digits),
+                                                            rowBlocks, uneven);
+    return (int)cudaGetLastError();
+}
+
 int sq103_tc_make_low_digits(const float *J, int ldJ, int R, int K, const void *high, void *digits, cudaStream_t st) {
     if (!high) return kErrBadShape;
     return make_digits(J, ldJ, R, K, 0, high, digits, st);
@@ -637,13 +682,13 @@ SQ103_API int sq103_bipartite_refresh_uses_tc(int N0, int N1, int m) {
     return tiles >= 64 ? 1 : 0;
 }
 
-// Where the bipartite annealer takes its half-step fields and energies to the tensor
-// cores: as above, and from about 80 M products a half-step on (m rounded up to a SIMT
-// tile's 16 rows).  ms, SIMT and tensor cores: 1024 x 1024, m = 64, 64 steps (67 M)
+// Where the bipartite annealer takes its energies, and its half-step fields when the
+// digits hold every row (sq103_tc_check_even), to the tensor cores: as above, and from
+// about 80 M products a half-step on (m rounded up to a SIMT tile's 16 rows).  ms, SIMT and tensor cores: 1024 x 1024, m = 64, 64 steps (67 M)
 // 2.89, 3.70; 1100 x 2900, m = 20, 32 steps (102 M) 3.00, 2.15; 1100 x 1100, m = 150
-// (194 M) 3.75, 2.62; 2900 x 2900, m = 30 (269 M) 5.01, 3.07.  Decisions are exact on
-// either, so the spins are the same; a path that returns energies (server) sums them the
-// way the annealer does.
+// (194 M) 3.75, 2.62; 2900 x 2900, m = 30 (269 M) 5.01, 3.07.  The
+// flips' tolerance covers the digits' rounding, so decisions are exact and the spins the
+// same on either; a path that returns energies (server) sums them the way the annealer does.
 int sq103_bipartite_tc_pays(int N0, int N1, int m) {
     if ((long long)N0 * (long long)N1 < (1ll << 20) || m < 1) return 0;
     return sq103_bipartite_refresh_uses_tc(N0, N1, m) || (double)((m + 15) / 16 * 16) * N0 * N1 >= 8e7;
