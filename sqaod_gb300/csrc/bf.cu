@@ -724,9 +724,8 @@ SQ103_API int sq103_dense_bf_range(const float *W, int N, uint64_t xBegin, uint6
     int subBits = 0;
     while (subBits < 4 && (runs << subBits) < (uint64_t)bf_grid(~0ull, 2)) ++subBits;
     if (runs > 0) {
-        cudaError_t e = cudaFuncSetAttribute(bf_run_pass<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)runSmem);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(bf_run_pass<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)runSmem);
+        static SmemLimitOnce limit;
+        const cudaError_t e = limit((int)(sizeof(RunShared) + sizeof(float) * 63 * 63), bf_run_pass<0>, bf_run_pass<1>);
         if (e != cudaSuccess) return (int)e;
     }
     for (int pass = 0; pass < 2; ++pass) {

@@ -54,6 +54,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <map>
 #include <mutex>
 #include <vector>
 
@@ -1076,36 +1077,55 @@ struct MultiCapacity {
     int two, four;
 };
 
+// Callers on several host threads share the kernels' shared memory limits (set once per
+// device, to the most that the device allows, and never lowered: another thread's launch
+// may need more than this caller's N) and the answers, kept per device and N.
 static MultiCapacity multi_capacity(int N) {
-    // the last answer is cached; callers on several host threads share it
+    struct Device {
+        int sms = 0, maxDyn = -1;
+        std::map<int, MultiCapacity> byN;
+    };
     static std::mutex mu;
-    static int cachedN = -1;
-    static MultiCapacity cached = {0, 0};
+    static std::map<int, Device> devices;
     std::lock_guard<std::mutex> lock(mu);
-    if (N == cachedN) return cached;
-    int dev = 0, sms = 0, optin = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) {
+        cudaGetLastError();
+        return {0, 0};
+    }
+    Device &d = devices[dev];
+    if (d.maxDyn < 0) {
+        int optin = 0, maxDyn = 1 << 30;
+        cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev);
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+        // every instance: the launch takes the one the tasks' flags and sizes ask for
+        for (int i = 0; i < 16; ++i) {
+            cudaFuncAttributes fa;
+            if (cudaFuncGetAttributes(&fa, multi_kernel(i)) != cudaSuccess ||
+                cudaFuncSetAttribute(multi_kernel(i), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     optin - (int)fa.sharedSizeBytes) != cudaSuccess) {
+                cudaGetLastError();
+                return {0, 0};
+            }
+            maxDyn = std::min(maxDyn, optin - (int)fa.sharedSizeBytes);
+        }
+        d.maxDyn = maxDyn;
+    }
     const size_t smem = multi_smem_bytes(N);
-    cudaFuncAttributes fa;
-    cudaFuncGetAttributes(&fa, multi_kernel(0));
-    if (smem + fa.sharedSizeBytes > (size_t)optin) return {0, 0};
-    // every instance: the launch takes the one the tasks' flags and sizes ask for
+    if (smem > (size_t)d.maxDyn) return {0, 0};
+    const auto known = d.byN.find(N);
+    if (known != d.byN.end()) return known->second;
     int perSm[2] = {1 << 30, 1 << 30};
     for (int i = 0; i < 16; ++i) {
-        const void *k = multi_kernel(i);
         int ps = 0;
-        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ps, k, mc_threads(i & 8 ? 4 : 2), smem) != cudaSuccess) {
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ps, multi_kernel(i), mc_threads(i & 8 ? 4 : 2), smem) !=
+            cudaSuccess) {
             cudaGetLastError();
             return {0, 0};
         }
         perSm[i >> 3] = std::min(perSm[i >> 3], ps);
     }
-    cachedN = N;
-    cached = {perSm[0] * sms, std::max(perSm[0], perSm[1]) * sms};
-    return cached;
+    return d.byN[N] = {perSm[0] * d.sms, std::max(perSm[0], perSm[1]) * d.sms};
 }
 
 }  // namespace sq103
@@ -1159,7 +1179,7 @@ static int launch_pack(const sq103_dense_task *tasks, int n, void *stream) {
         return rc != 0 ? rc : launch_pack(part[1].data(), (int)part[1].size(), stream);
     }
     for (int i = n; i <= kMaxPack; ++i) P.base[i] = ctas;
-    // every CTA resident at once (cooperative launch); also sets the kernel's shared-memory limit
+    // every CTA resident at once (cooperative launch); also sets the kernels' shared-memory limits
     const MultiCapacity cap = multi_capacity(maxN);
     if (cap.four < ctas) return kErrCapacity;
     void *args[] = {&P};

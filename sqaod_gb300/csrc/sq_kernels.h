@@ -5,6 +5,38 @@
 
 #include <cuda_runtime.h>
 
+#include <mutex>
+
+namespace sq103 {
+
+// A kernel's dynamic shared memory limit is an attribute of the device's context that
+// every host thread shares: it is set to the largest use, once per device, under a lock,
+// and never lowered, so a launch of another thread always finds it large enough.
+class SmemLimitOnce {
+public:
+    template <class... Kernels>
+    cudaError_t operator()(int bytes, Kernels... kernels) {
+        int dev = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e != cudaSuccess) return e;
+        std::lock_guard<std::mutex> lock(mu_);
+        const bool known = dev >= 0 && dev < 256;
+        if (known && set_[dev]) return cudaSuccess;
+        for (const void *k : {(const void *)kernels...}) {
+            e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+            if (e != cudaSuccess) return e;
+        }
+        if (known) set_[dev] = true;
+        return cudaSuccess;
+    }
+
+private:
+    std::mutex mu_;
+    bool set_[256] = {};
+};
+
+}  // namespace sq103
+
 // the half-step fields, launched to start while the stream's last kernel runs when
 // `dependent` (that kernel must be one of the bipartite anneal's own)
 extern "C" int sq103_bipartite_fields_after(const float *J, int N0, int N1, const int8_t *qFixed, int side, float *F,

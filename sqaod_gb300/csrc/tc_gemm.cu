@@ -51,7 +51,6 @@
 
 #include <algorithm>
 #include <cstdint>
-#include <mutex>
 
 #include "sq_common.cuh"
 #include "sq_kernels.h"
@@ -546,20 +545,9 @@ static int launch_gemm(const void *digits, int R, int K, int m, void *spinsBf16,
                 CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return kErrBadShape;
     }
-    // the shared-memory limit is a per-device kernel attribute: set once per device, under a lock
-    {
-        static std::mutex mu;
-        static bool attrSet[256] = {};  // (one per instance of this function: per output type)
-        int dev = 0;
-        cudaError_t e = cudaGetDevice(&dev);
-        if (e != cudaSuccess) return (int)e;
-        std::lock_guard<std::mutex> lock(mu);
-        if (dev < 0 || dev >= 256 || !attrSet[dev]) {
-            e = cudaFuncSetAttribute(tc_digit_gemm<Out>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmemBytes);
-            if (e != cudaSuccess) return (int)e;
-            if (dev >= 0 && dev < 256) attrSet[dev] = true;
-        }
-    }
+    static SmemLimitOnce limit;  // (one per instance of this function: per output type)
+    const cudaError_t limitErr = limit(kTcSmemBytes, tc_digit_gemm<Out>);
+    if (limitErr != cudaSuccess) return (int)limitErr;
     // K split over a cluster of up to 4 while the tiles times the split stay within one CTA
     // per SM and a CTA has two K blocks or more.  us per refresh with the spins' conversion,
     // by largest split 1, 2, 4, 8: R = K = 1501, m = 63 (24 tiles) 20.5, 20.5, 18.5, 18.4;
