@@ -506,6 +506,11 @@ SQ103_API int sq103_dense_batch_autotune_routing(void *handle, int trialSteps, c
                                                 int *chosen);
 SQ103_API int sq103_dense_batch_anneal(void *handle, int nSteps, int useGraph);
 SQ103_API int sq103_dense_batch_sync(void *handle);
+/* Fault injection from the host (tests; no counterpart in the reference): writes `value`
+ * into a status word of a prepared batch, in stream order, as a kernel that gave up a
+ * bounded device wait does.  which = 0: the sweeps and field refreshes; sync, get_E and
+ * get_q then fail until the next prepare.  which = 1: the energies; the next get_E fails. */
+SQ103_API int sq103_dense_batch_inject_status(void *handle, int which, int value);
 SQ103_API int sq103_dense_batch_info(void *handle, int *nInst, int *pos, int *grid, int *smemBytes);
 SQ103_API int sq103_dense_batch_get_E(void *handle, int index, double *E, int cap, int *n);
 SQ103_API int sq103_dense_batch_get_q(void *handle, int index, int8_t *q, int capRows, int *m);

@@ -1928,7 +1928,6 @@ public:
         float *J, *h, *c32, *F;
         double *c64;
         int8_t *q;
-        int *status;
     };
 
     ~DenseBatch() {
@@ -1957,10 +1956,8 @@ public:
         in.h = (float *)(b + oh);
         in.c32 = (float *)(b + oc);
         in.c64 = (double *)(b + oc64);
-        in.status = (int *)(b + oc64 + 8);
         in.F = (float *)(b + oF);
         in.q = (int8_t *)(b + oq);
-        SQ_CHECK(cudaMemsetAsync(in.status, 0, sizeof(int), st_.get()));
         if (sq103_dense_refresh_uses_tc(N)) {
             in.digits.ensure(sq103_tc_digits_bytes(N, N));
             in.Abf.ensure(sq103_tc_spins_bytes(m, N));
@@ -2037,6 +2034,9 @@ public:
             maxN = std::max(maxN, in.N);
             maxM = std::max(maxM, in.m);
         }
+        dStatus_.ensure(1);
+        SQ_CHECK(cudaMemsetAsync(dStatus_.p, 0, sizeof(int), st_.get()));
+        statusRead_ = false;
         buildRefreshJobs();
         refreshAll();
         // packed launches take instances of similar size together
@@ -2054,7 +2054,6 @@ public:
         dOrder_.ensure(nAlloc);
         dPos_.ensure(nAlloc);
         dQueue_.ensure(2);
-        dStatus_.ensure(1);
         if (n > 0) {
             SQ_CHECK(cudaMemcpyAsync(dTasks_.p, tasks.data(), sizeof(sq103_dense_task) * n, cudaMemcpyHostToDevice,
                                      st_.get()));
@@ -2062,7 +2061,6 @@ public:
         }
         SQ_CHECK(cudaMemsetAsync(dPos_.p, 0, sizeof(int) * nAlloc, st_.get()));
         SQ_CHECK(cudaMemsetAsync(dQueue_.p, 0, sizeof(int) * 2, st_.get()));
-        SQ_CHECK(cudaMemsetAsync(dStatus_.p, 0, sizeof(int), st_.get()));
         st_.sync();
         pos_ = 0;
         if (smem_ < 0) chooseConfig(-1);
@@ -2184,6 +2182,7 @@ public:
     void anneal(int nSteps, bool useGraph) {
         throwErrorIf(!prepared_, "prepare() first.");
         int left = std::min(nSteps, nSched_ - pos_);
+        if (left > 0) statusRead_ = false;
         while (left > 0) {
             if (pos_ > 0 && pos_ % kRefreshPeriod == 0) refreshAll();
             const int chunk = std::min(left, kRefreshPeriod - pos_ % kRefreshPeriod);
@@ -2203,10 +2202,19 @@ public:
 
     void sync() {
         st_.sync();
-        if (multi_.empty()) return;
-        int status = 0;
-        SQ_CHECK(cudaMemcpy(&status, dStatus_.p, sizeof(int), cudaMemcpyDeviceToHost));
-        if (status != 0) throw_cuda(status, "one-CTA-per-trotter batch sweep");
+        checkStatus();
+    }
+
+    // Fault injection from the host (tests): writes `value` into a status word, in stream
+    // order, as a kernel that gave up a bounded device wait does: 0 the sweeps' and field
+    // refreshes', 1 the energies'.
+    void injectStatus(int which, int value) {
+        throwErrorIf(!prepared_ || which < 0 || which > 1, "prepare() first; the status words are 0 and 1.");
+        if (which == 1) energyBuffer(1);
+        SQ_CHECK(cudaMemcpyAsync(which ? (int *)E64_.p : dStatus_.p, &value, sizeof(int), cudaMemcpyHostToDevice,
+                                 st_.get()));
+        st_.sync();
+        if (which == 0) statusRead_ = false;
     }
 
     // instances of at least N spins take the one-CTA-per-trotter sweep (0: none); before prepare()
@@ -2234,30 +2242,59 @@ public:
 
     void energies(int i, double *E) {
         const Inst &in = inst(i);
+        checkStatus();
         r_.ensure((size_t)in.m * in.N);
-        E64_.ensure(in.m);
+        energyBuffer(in.m);
+        double *dE = E64_.p + 1;
         if (in.digits.p) {  // as the single annealer; the low digits in a shared scratch
             low_.ensure(sq103_tc_digits_bytes(in.N, in.N));
             SQ_CHECK(sq103_tc_make_low_digits(in.J, in.ldJ, in.N, in.N, in.digits.p, low_.p, st_.get()));
-            SQ_CHECK(sq103_tc_row_sums(in.digits.p, low_.p, in.N, in.N, in.q, in.N, in.m, in.Abf.p, r_.p, in.status,
-                                       st_.get()));
-            SQ_CHECK(sq103_dense_energy_of_sums(r_.p, in.h, in.c64, in.q, in.N, in.m, optimize_[i], E64_.p, nullptr,
+            SQ_CHECK(sq103_tc_row_sums(in.digits.p, low_.p, in.N, in.N, in.q, in.N, in.m, in.Abf.p, r_.p,
+                                       (int *)E64_.p, st_.get()));
+            SQ_CHECK(sq103_dense_energy_of_sums(r_.p, in.h, in.c64, in.q, in.N, in.m, optimize_[i], dE, nullptr,
                                                 st_.get()));
         } else {
-            SQ_CHECK(sq103_dense_energy(in.J, in.ldJ, in.h, in.c64, in.q, in.N, in.m, optimize_[i], r_.p, E64_.p,
-                                        nullptr, st_.get()));
+            SQ_CHECK(sq103_dense_energy(in.J, in.ldJ, in.h, in.c64, in.q, in.N, in.m, optimize_[i], r_.p, dE, nullptr,
+                                        st_.get()));
         }
-        SQ_CHECK(cudaMemcpyAsync(E, E64_.p, sizeof(double) * in.m, cudaMemcpyDeviceToHost, st_.get()));
+        hE_.resize((size_t)in.m + 1);
+        SQ_CHECK(cudaMemcpyAsync(hE_.data(), E64_.p, sizeof(double) * (in.m + 1), cudaMemcpyDeviceToHost, st_.get()));
         st_.sync();
+        int status = 0;
+        memcpy(&status, hE_.data(), sizeof(int));
+        if (status != 0) {
+            SQ_CHECK(cudaMemsetAsync(E64_.p, 0, sizeof(double), st_.get()));
+            sq::throwError("energies of instance %d: device wait timed out (status %d).", i, status);
+        }
+        memcpy(E, hE_.data() + 1, sizeof(double) * in.m);
     }
 
     void spins(int i, int8_t *q) {
         const Inst &in = inst(i);
+        checkStatus();
         SQ_CHECK(cudaMemcpyAsync(q, in.q, (size_t)in.m * in.N, cudaMemcpyDeviceToHost, st_.get()));
         st_.sync();
     }
 
 private:
+    // Raises when a sweep or a field refresh gave up a bounded wait since prepare(): the
+    // batch's spins are not valid then.  Read once after the steps queued last.
+    void checkStatus() {
+        if (statusRead_ || !dStatus_.p) return;
+        int status = 0;
+        SQ_CHECK(cudaMemcpyAsync(&status, dStatus_.p, sizeof(int), cudaMemcpyDeviceToHost, st_.get()));
+        st_.sync();
+        throwErrorIf(status != 0, "batch: device wait timed out (status %d); spins are not valid.", status);
+        statusRead_ = true;
+    }
+
+    // E64_: the status word of the energies (it stays zero), then m energies
+    void energyBuffer(int m) {
+        if (E64_.p && E64_.n > (size_t)m) return;
+        E64_.ensure((size_t)m + 1);
+        SQ_CHECK(cudaMemsetAsync(E64_.p, 0, sizeof(double), st_.get()));
+    }
+
     void launchOne() {
         SQ_CHECK(sq103_dense_batch_launch(dTasks_.p, nSmall_, nullptr, dOrder_.p, dPos_.p, dQueue_.p, 1, grid_, smem_,
                                           st_.get()));
@@ -2351,7 +2388,7 @@ private:
         for (int k = 0; k < ns; ++k) SQ_CHECK(cudaStreamWaitEvent(side_[k].get(), fork_, 0));
         for (size_t i = 0; i < tcInsts_.size(); ++i) {
             Inst &in = *tcInsts_[i];
-            SQ_CHECK(sq103_dense_refresh(in.J, in.ldJ, in.digits.p, in.Abf.p, in.q, in.F, in.N, in.m, in.status,
+            SQ_CHECK(sq103_dense_refresh(in.J, in.ldJ, in.digits.p, in.Abf.p, in.q, in.F, in.N, in.m, dStatus_.p,
                                          side_[i % ns].get()));
         }
         for (int k = 0; k < ns; ++k) {
@@ -2374,6 +2411,7 @@ private:
     std::vector<int> optimize_;
     DevBuf<float> dW_, sched_;
     DevBuf<double> scratch_, r_, E64_;
+    std::vector<double> hE_;
     DevBuf<unsigned char> low_;  // low digits of the instance whose energies are computed
     DevBuf<sq103_dense_task> dTasks_;
     DevBuf<int> dOrder_, dPos_, dQueue_, dStatus_;
@@ -2389,6 +2427,7 @@ private:
     int nSched_ = 0, pos_ = 0, grid_ = 1, smem_ = -1, nSmall_ = 0, multiMinN_ = kDefaultMultiMinN;
     bool limitGiven_ = false;
     bool prepared_ = false;
+    bool statusRead_ = false;  // dStatus_ was read after the steps queued last
 };
 
 // ============================================================= formulas
