@@ -526,7 +526,7 @@ def run_batched(args, world):
                        "routing": ("autotuned (8 trial steps per candidate 0, 512, 768, 1024, 1400, 2048)"
                                    if args.autotune_routing and args.multicta_min_n is None
                                    else "given" if args.multicta_min_n is not None else "default"),
-                       "multicta_instances": b.multicta_count()},
+                       "multicta_instances": b.packed_count()},
             "batched": {"seconds": t_batch, "solves_per_s": len(work) / t_batch, "setup_s": t_add,
                         "results_s": t_out, "seconds_with_setup": t_total,
                         "solves_per_s_with_setup": len(work) / t_total, "autotune_s": t_tune,

@@ -490,12 +490,16 @@ SQ103_API int sq103_dense_batch_set_schedule(void *handle, const float *G, const
 SQ103_API int sq103_dense_batch_prepare(void *handle);
 /* Instances of at least N spins (m >= 2, fitting the device) are stepped by the
  * one-CTA-per-trotter sweep in packed cooperative launches, the rest by the
- * persistent batch kernel; both give the same results.  Default 1024, and
- * the packed launches take smaller ones along where that is faster; 0 keeps
- * every instance on the persistent kernel.  Takes effect at the next prepare. */
+ * persistent batch kernel; both give the same results.  Without a call, the
+ * limit is 1024 and the packed launches also take the smaller instances along,
+ * from 64 spins (128 in batches of more than 152 instances); 0 keeps every
+ * instance on the persistent kernel.  Takes effect at the next prepare. */
 SQ103_API int sq103_dense_batch_set_multicta_min_n(void *handle, int N);
-/* instances on the one-CTA-per-trotter sweep since the last prepare */
+/* instances of at least the limit (1024 without a call) on the one-CTA-per-trotter
+ * sweep since the last prepare, without the smaller ones taken along */
 SQ103_API int sq103_dense_batch_multicta_count(void *handle, int *n);
+/* every instance on the one-CTA-per-trotter sweep since the last prepare */
+SQ103_API int sq103_dense_batch_packed_count(void *handle, int *n);
 SQ103_API int sq103_dense_batch_autotune(void *handle, int trialSteps, int *smemBytes);
 /* Trotters per CTA by measurement (no counterpart in the reference): prepares the
  * batch with each candidate size limit of sq103_dense_batch_set_multicta_min_n

@@ -58,14 +58,24 @@ class DenseBatchAnnealer:
 
     def set_multicta_min_n(self, N):
         """Instances of at least N spins run on the one-CTA-per-trotter sweep
-        (packed launches); 0 keeps all on the persistent kernel.  Default 1024,
-        with smaller ones taken along where that is faster; results do not
-        depend on it.  Takes effect at the next prepare()."""
+        (packed launches); 0 keeps all on the persistent kernel.  Without a
+        call the limit is 1024 and the packed launches also take the smaller
+        instances along, from 64 spins (128 in batches of more than 152
+        instances); results do not depend on it.  Takes effect at the next
+        prepare()."""
         self._call("set_multicta_min_n", ctypes.c_int(N))
 
     def multicta_count(self):
+        """Instances of at least the limit in the packed launches since the last
+        prepare(), without the smaller ones taken along (packed_count())."""
         n = ctypes.c_int()
         self._call("multicta_count", ctypes.byref(n))
+        return n.value
+
+    def packed_count(self):
+        """Every instance in the packed launches since the last prepare()."""
+        n = ctypes.c_int()
+        self._call("packed_count", ctypes.byref(n))
         return n.value
 
     def autotune_routing(self, trial_steps=8, candidates=(0, 512, 768, 1024, 1400, 2048)):

@@ -2224,8 +2224,10 @@ public:
         limitGiven_ = true;
         prepared_ = false;
     }
-    // the instances of at least the size limit (the smaller ones that the packed
-    // launches take along without a limit of the caller's are not counted)
+    // the instances on the one-CTA-per-trotter sweep since the last prepare
+    int packedCount() const { return (int)multi_.size(); }
+    // those of at least the size limit; without a limit of the caller's that leaves out
+    // the ones below 1024 spins that the packed launches take along
     int multiCount() const {
         int n = 0;
         for (const Inst *in : multi_) n += in->N >= multiMinN_;
