@@ -57,6 +57,19 @@ public:
             release(s);
             SQ_CHECK(cudaMallocAsync((void **)&p, bytes, s));
         }
+        // replaces what it held; keeps that and returns false when there is no memory
+        bool tryGrow(size_t bytes, cudaStream_t s) {
+            unsigned char *grown = nullptr;
+            const cudaError_t e = cudaMallocAsync((void **)&grown, bytes, s);
+            if (e == cudaErrorMemoryAllocation) {
+                cudaGetLastError();
+                return false;
+            }
+            SQ_CHECK(e);
+            release(s);
+            p = grown;
+            return true;
+        }
         void release(cudaStream_t s) {
             if (p) cudaFreeAsync(p, s);
             p = nullptr;
@@ -128,6 +141,7 @@ public:
         int *dStatus = nullptr;        // this request's own timeout status word (dense sweeps)
         void *digits = nullptr;        // tensor-core refresh of a dense request with N >= 1024
         void *spinsBf16 = nullptr;
+        bool tcEnergies = false;       // energies on the tensor cores, with scratch_
         int status = 0;                // its value once the request is done
         // a search: the searcher handle, the next state to search, 2^N, the list cap
         void *bf = nullptr;
@@ -239,7 +253,7 @@ public:
             SQ_CHECK(sq103_bipartite_batch_launch(bTasks_.p, nB, counts_.p + 1, nullptr, bPos_.p, queues_.p + 2,
                                                   kStepsPerTick, std::min(bipGrid_, nB), side()));
         for (Request *r : large_) {
-            if (r->kind != 1) continue;
+            if (r->kind != 1 || r->pos >= r->nSteps) continue;
             sq103_bipartite_task t = r->bt;
             t.G = r->bt.G + r->pos;
             t.beta = r->bt.beta + r->pos;
@@ -251,7 +265,7 @@ public:
         // (instances of similar size together, as many trotters as can be resident)
         std::vector<Request *> big;
         for (Request *r : large_)
-            if (r->kind == 0) big.push_back(r);
+            if (r->kind == 0 && r->pos < r->nSteps) big.push_back(r);
         std::sort(big.begin(), big.end(), [](const Request *a, const Request *b) { return a->N0 < b->N0; });
         std::vector<sq103_dense_task> pack;
         int packM = 0, packN = 0;
@@ -280,8 +294,12 @@ public:
         int nTc = 0;  // tensor-core refreshes queued on the side streams
         for (auto &kv : active_) {
             Request *r = kv.second;
-            if (r->kind == kSearch) continue;   // advanced below
-            if (r->pos >= r->nSteps) continue;  // finishing: its results are being collected
+            if (r->kind == kSearch) continue;  // advanced below
+            if (r->done) continue;             // finishing: its results are being collected
+            if (r->pos >= r->nSteps) {         // its energies could not be queued at an earlier tick
+                finished.push_back(r);
+                continue;
+            }
             r->pos = std::min(r->pos + kStepsPerTick, r->nSteps);
             if (r->kind == 0 && r->pos < r->nSteps && r->pos % kRefreshPeriod == 0) {
                 if (r->digits) {  // on the side streams, forked from the work stream at the first
@@ -419,6 +437,9 @@ private:
         rq->bytes = footprint(*rq);
         throwErrorIf(rq->bytes > budget_, "request of %llu bytes exceeds the device-memory budget of %llu bytes.",
                      (unsigned long long)rq->bytes, budget_);
+        // energies as the single-instance annealers', unless their scratch would exceed the
+        // budget: then the SIMT sums, which need none (the last bits may differ)
+        rq->tcEnergies = tcEnergies(*rq) && rq->bytes + scratchBytes(*rq) <= budget_;
         Request *p = rq.get();
         all_[p->id] = std::move(rq);
         queue_.push_back(p);
@@ -451,6 +472,42 @@ private:
         return s;
     }
 
+    static bool tcEnergies(const Request &r) {
+        return r.kind == 0   ? sq103_dense_refresh_uses_tc(r.N0) != 0
+               : r.kind == 1 ? sq103_bipartite_tc_pays(r.N0, r.N1, r.m) != 0
+                             : false;
+    }
+    // device scratch of a request's tensor-core energies: the low digits, and the digits
+    // and the spins of a bipartite request that steps on the SIMT fields
+    static size_t scratchBytes(const Request &r) {
+        if (r.kind == 0) return al(sq103_tc_digits_bytes(r.N0, r.N0));
+        const size_t digits = al(sq103_tc_digits_bytes(r.N1, r.N0));
+        return sq103_bipartite_refresh_uses_tc(r.N0, r.N1, r.m) ? digits
+                                                                : 2 * digits + al(sq103_tc_spins_bytes(r.m, r.N0));
+    }
+    // what admitting r adds to used_ for the scratch, which the active requests share; the
+    // old scratch is freed after the new one is there, so both count until then
+    size_t scratchGrowth(const Request &r) const {
+        const size_t need = r.tcEnergies ? scratchBytes(r) : 0;
+        return need > scratchSize_ ? need : 0;
+    }
+    void growScratch(Request &r) {
+        const size_t need = scratchGrowth(r);
+        if (need == 0) return;
+        if (!scratch_.tryGrow(need, st_.get())) {
+            r.tcEnergies = false;
+            return;
+        }
+        used_ += need - scratchSize_;
+        scratchSize_ = need;
+    }
+    void releaseIdleScratch() {
+        if (!active_.empty() || scratchSize_ == 0) return;
+        scratch_.release(st_.get());
+        used_ -= scratchSize_;
+        scratchSize_ = 0;
+    }
+
     bool fitsStaging(const Request &r) const {
         const size_t base = (size_t)sq103_dense_batch_min_smem(r.m);  // the flip lists
         return base + (size_t)r.m * r.N0 * 5 + (size_t)r.N0 * 4 <= (size_t)stageSmem_;
@@ -469,13 +526,14 @@ private:
         if (r.kind != 0 || !sq103_dense_multicta_ok(r.N0, r.m, kColoring)) return false;
         // (dense: with the accept-word workspace inside the budget)
         return nLight_[0] < (r.N0 >= 128 ? kMaxLightDense : kMaxLightSmall) &&
-               used_ + r.bytes + al(sq103_dense_ws_bytes(r.N0, r.m, kStepsPerTick)) <= budget_;
+               used_ + r.bytes + scratchGrowth(r) + al(sq103_dense_ws_bytes(r.N0, r.m, kStepsPerTick)) <= budget_;
     }
 
     // Admits queued requests in arrival order as memory, slots and the large-instance
     // limit allow; a request that cannot start yet keeps its place and does not
     // block the ones behind it.
     void admit() {
+        releaseIdleScratch();
         bool changed = false;
         size_t i = 0;
         while (i < queue_.size()) {
@@ -488,7 +546,7 @@ private:
                                                     sq103_bipartite_refresh_uses_tc(r->N0, r->N1, r->m);
             const bool light = !heavy && light_(*r);
             const bool fits =
-                used_ + r->bytes <= budget_ &&
+                used_ + r->bytes + scratchGrowth(*r) <= budget_ &&
                 (r->kind == kSearch ? (int)searches_.size() < kMaxSearches
                  : heavy            ? nHeavy_ < maxLarge_  // each steps with the whole GPU every tick
                  : light            ? true
@@ -502,6 +560,7 @@ private:
             r->heavy = heavy;
             if (heavy) ++nHeavy_;
             if (light) ++nLight_[r->kind];
+            growScratch(*r);
             setup(r);
             used_ += r->bytes;
             r->state = kActive;
@@ -661,11 +720,10 @@ private:
         if (r->kind == 0) {
             const int N = r->N0;
             double *scratch = (double *)((unsigned char *)r->dt.q + al((size_t)m * N));
-            if (r->digits) {  // as the single annealer; the low digits in a shared scratch
-                low_.ensure(sq103_tc_digits_bytes(N, N));
-                SQ_CHECK(sq103_tc_make_low_digits(r->dt.J, r->dt.ldJ, N, N, r->digits, low_.p, st_.get()));
-                SQ_CHECK(sq103_tc_row_sums(r->digits, low_.p, N, N, r->dt.q, N, m, r->spinsBf16, scratch, r->dStatus,
-                                           st_.get()));
+            if (r->tcEnergies) {  // as the single annealer
+                SQ_CHECK(sq103_tc_make_low_digits(r->dt.J, r->dt.ldJ, N, N, r->digits, scratch_.p, st_.get()));
+                SQ_CHECK(sq103_tc_row_sums(r->digits, scratch_.p, N, N, r->dt.q, N, m, r->spinsBf16, scratch,
+                                           r->dStatus, st_.get()));
                 SQ_CHECK(sq103_dense_energy_of_sums(scratch, r->dt.h, r->c64, r->dt.q, N, m, r->optimize, r->dE,
                                                     nullptr, st_.get()));
             } else {
@@ -674,19 +732,19 @@ private:
             }
         } else {
             double *scratch = (double *)((unsigned char *)r->bt.F1 + al((size_t)m * r->N1 * 4));
-            if (sq103_bipartite_tc_pays(r->N0, r->N1, m)) {
+            if (r->tcEnergies) {
                 const void *digits = r->bt.digits1;
                 void *bf16 = r->bt.spinsBf16;
+                unsigned char *low = scratch_.p;
                 if (!digits) {  // a request that steps on the SIMT fields
-                    high_.ensure(sq103_tc_digits_bytes(r->N1, r->N0));
-                    bf16_.ensure(sq103_tc_spins_bytes(m, r->N0));
-                    SQ_CHECK(sq103_tc_make_digits(r->bt.J, r->N0, r->N1, r->N0, 0, high_.p, st_.get()));
-                    digits = high_.p;
-                    bf16 = bf16_.p;
+                    const size_t planes = al(sq103_tc_digits_bytes(r->N1, r->N0));
+                    low = scratch_.p + planes;
+                    bf16 = low + planes;
+                    SQ_CHECK(sq103_tc_make_digits(r->bt.J, r->N0, r->N1, r->N0, 0, scratch_.p, st_.get()));
+                    digits = scratch_.p;
                 }
-                low_.ensure(sq103_tc_digits_bytes(r->N1, r->N0));
-                SQ_CHECK(sq103_tc_make_low_digits(r->bt.J, r->N0, r->N1, r->N0, digits, low_.p, st_.get()));
-                SQ_CHECK(sq103_tc_row_sums(digits, low_.p, r->N1, r->N0, r->bt.q0, r->N0, m, bf16, scratch, r->dStatus,
+                SQ_CHECK(sq103_tc_make_low_digits(r->bt.J, r->N0, r->N1, r->N0, digits, low, st_.get()));
+                SQ_CHECK(sq103_tc_row_sums(digits, low, r->N1, r->N0, r->bt.q0, r->N0, m, bf16, scratch, r->dStatus,
                                            st_.get()));
                 SQ_CHECK(sq103_bipartite_energy_of_sums(scratch, r->bt.h0, r->bt.h1, r->c64, r->bt.q0, r->bt.q1, r->N0,
                                                         r->N1, m, r->optimize, r->dE, st_.get()));
@@ -695,8 +753,12 @@ private:
                                                 m, r->optimize, scratch, r->dE, nullptr, st_.get()));
             }
         }
-        SQ_CHECK(cudaEventCreateWithFlags(&r->done, cudaEventDisableTiming));
-        SQ_CHECK(cudaEventRecord(r->done, st_.get()));
+        cudaEvent_t done = nullptr;
+        SQ_CHECK(cudaEventCreateWithFlags(&done, cudaEventDisableTiming));
+        const cudaError_t recorded = cudaEventRecord(done, st_.get());
+        if (recorded != cudaSuccess) cudaEventDestroy(done);
+        SQ_CHECK(recorded);
+        r->done = done;
         // free the slot now (the kernels skip finished instances anyway): the last slot moves into it
         if (r->kind == 0 && !r->large) removeSlot(denseSlots_, r, dTasks_.p, dPos_.p, 0);
         if (r->kind == 1 && !r->large) removeSlot(bipSlots_, r, bTasks_.p, bPos_.p, 1);
@@ -771,6 +833,7 @@ private:
             ++done_;
             ++n;
         }
+        if (n > 0) releaseIdleScratch();
         return n;
     }
 
@@ -817,7 +880,10 @@ private:
     DevBuf<sq103_bipartite_task> bTasks_;
     DevBuf<int> dPos_, bPos_, counts_, queues_;
     DevBuf<float> dW_;
-    DevBuf<unsigned char> low_, high_, bf16_;  // digits and spins of the request whose energies are queued
+    // tensor-core energies: the scratch of the request whose energies are queued, as large as
+    // the active requests' largest need, part of used_
+    AsyncMem scratch_;
+    size_t scratchSize_ = 0;
     static constexpr int kMaxPack = 64;  // instances per packed launch (sq103_dense_anneal_pack)
     // light requests on the large ones' routes at a time: dense of N >= 128, dense below, bipartite
     static constexpr int kMaxLightDense = 512, kMaxLightSmall = 64, kMaxLightBip = 32;
