@@ -41,6 +41,20 @@ struct DevBuf {
         SQ_CHECK(cudaMalloc((void **)&p, sizeof(T) * count));
         n = count;
     }
+    // false, and nothing held, when the device has no memory for it
+    bool tryEnsure(size_t count) {
+        if (count <= n && p) return true;
+        release();
+        const cudaError_t e = cudaMalloc((void **)&p, sizeof(T) * count);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            p = nullptr;
+            return false;
+        }
+        SQ_CHECK(e);
+        n = count;
+        return true;
+    }
 };
 
 // owning pinned host buffer

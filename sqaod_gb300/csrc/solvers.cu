@@ -89,6 +89,30 @@ static void round_problem(const double *src, int rows, int cols, int lds, float 
     SQ_CHECK(cudaGetLastError());
 }
 
+// The low digit planes of a problem (8 bytes a coupling, for its tensor-core energies): made
+// with its first energies and kept up to this size (N = 11,500 dense); larger ones are
+// made for each call, at a fraction of what the sums then cost, and freed after it.
+constexpr size_t kLowKeepBytes = (size_t)1 << 30;
+struct LowDigits {
+    DevBuf<unsigned char> buf;
+    bool made = false;
+    // the planes of what `high`, the digits of J (R x K), round away; false when the
+    // device has no memory for them (the SIMT energies need none)
+    bool make(const float *J, int ldJ, int R, int K, const void *high, cudaStream_t st) {
+        if (made) return true;
+        if (!buf.tryEnsure(sq103_tc_digits_bytes(R, K))) return false;
+        SQ_CHECK(sq103_tc_make_low_digits(J, ldJ, R, K, high, buf.p, st));
+        made = true;
+        return true;
+    }
+    // after the energies
+    void trim() {
+        if (buf.n <= kLowKeepBytes) return;
+        buf.release();
+        made = false;
+    }
+};
+
 // a matrix with row stride = columns
 template <class real>
 static std::vector<real> dense_copy(const sq::MatrixType<real> &M) {
@@ -352,20 +376,16 @@ public:
         if (fp64_)
             SQ_CHECK(sq103_dense_energy64(d_J64_.p, d_h64_.p, c64h_, d_q_.p, N_, m_, om_ == sq::optMaximize,
                                           d_E64_.p, st_.get()));
-        else if (d_digits_.p) {
-            // row sums on the tensor cores, to FP64 accuracy with the low digits, which are
-            // made with the first energies of a problem.  N = 4096, m = 256, 64 steps and the
-            // energies: 15.9 ms with the SIMT double-float sums (1.13 ms of it), 14.7 this way.
-            if (!lowMade_) {
-                d_low_.ensure(sq103_tc_digits_bytes(N_, N_));
-                SQ_CHECK(sq103_tc_make_low_digits(d_J_.p, ldJ_, N_, N_, d_digits_.p, d_low_.p, st_.get()));
-                lowMade_ = true;
-            }
-            SQ_CHECK(sq103_tc_row_sums(d_digits_.p, d_low_.p, N_, N_, d_q_.p, N_, m_, d_Abf_.p, d_r_.p, d_status_.p,
+        else if (d_digits_.p && low_.make(d_J_.p, ldJ_, N_, N_, d_digits_.p, st_.get())) {
+            // row sums on the tensor cores, to FP64 accuracy with the low digits.  N = 4096,
+            // m = 256, 64 steps and the energies: 15.9 ms with the SIMT double-float sums
+            // (1.13 ms of it), 14.7 this way.
+            SQ_CHECK(sq103_tc_row_sums(d_digits_.p, low_.buf.p, N_, N_, d_q_.p, N_, m_, d_Abf_.p, d_r_.p, d_status_.p,
                                        st_.get()));
             SQ_CHECK(sq103_dense_energy_of_sums(d_r_.p, d_h_.p, d_c64_.p, d_q_.p, N_, m_, om_ == sq::optMaximize,
                                                 d_E64_.p, d_E32_.p, st_.get()));
             checkStatus();
+            low_.trim();
         } else
             SQ_CHECK(sq103_dense_energy(d_J_.p, ldJ_, d_h_.p, d_c64_.p, d_q_.p, N_, m_, om_ == sq::optMaximize,
                                         d_r_.p, d_E64_.p, d_E32_.p, st_.get()));
@@ -495,7 +515,7 @@ private:
     }
 
     void makeDigits() {
-        lowMade_ = false;
+        low_.made = false;
         if (d_digits_.p) SQ_CHECK(sq103_tc_make_digits(d_J_.p, ldJ_, N_, N_, 0, d_digits_.p, st_.get()));
     }
 
@@ -628,8 +648,7 @@ private:
     mutable Stream st_;
     DevBuf<float> d_J_, d_h_, d_c_, d_F_, d_E32_, d_sched_;
     DevBuf<unsigned char> d_digits_, d_Abf_;  // tensor-core refresh: digit planes of J, spins in bf16
-    DevBuf<unsigned char> d_low_;             // tensor-core energies: the low digit planes
-    bool lowMade_ = false;
+    LowDigits low_;                           // tensor-core energies
     DevBuf<double> d_J64_, d_h64_;            // FP64 problem of a <double> annealer (J64 row stride N)
     double c64h_ = 0.;
     bool fp64_ = false;
@@ -911,13 +930,9 @@ public:
         if (fp64_)
             SQ_CHECK(sq103_bipartite_energy64(d_J64_.p, d_h0_64_.p, d_h1_64_.p, c64h_, d_q0_.p, d_q1_.p, N0_, N1_, m_,
                                               om_ == sq::optMaximize, d_E64_.p, st_.get()));
-        else if (useTc()) {  // as DenseAnnealer::calculate_E
-            if (!lowMade_) {
-                d_low1_.ensure(sq103_tc_digits_bytes(N1_, N0_));
-                SQ_CHECK(sq103_tc_make_low_digits(d_J_.p, N0_, N1_, N0_, d_digits1_.p, d_low1_.p, st_.get()));
-                lowMade_ = true;
-            }
-            SQ_CHECK(sq103_tc_row_sums(d_digits1_.p, d_low1_.p, N1_, N0_, d_q0_.p, N0_, m_, d_Abf_.p, d_r_.p,
+        else if (useTc() && low_.make(d_J_.p, N0_, N1_, N0_, d_digits1_.p, st_.get())) {
+            // as DenseAnnealer::calculate_E
+            SQ_CHECK(sq103_tc_row_sums(d_digits1_.p, low_.buf.p, N1_, N0_, d_q0_.p, N0_, m_, d_Abf_.p, d_r_.p,
                                        d_status_.p, st_.get()));
             SQ_CHECK(sq103_bipartite_energy_of_sums(d_r_.p, d_h0_.p, d_h1_.p, d_c64_.p, d_q0_.p, d_q1_.p, N0_, N1_, m_,
                                                     om_ == sq::optMaximize, d_E64_.p, st_.get()));
@@ -928,6 +943,7 @@ public:
                 SQ_CHECK(cudaMemsetAsync(d_status_.p, 0, sizeof(int), st_.get()));
                 sq::throwError("calculate_E: device wait timed out (status %d); spins are not valid.", status);
             }
+            low_.trim();
         } else
             SQ_CHECK(sq103_bipartite_energy(d_J_.p, d_h0_.p, d_h1_.p, d_c64_.p, d_q0_.p, d_q1_.p, N0_, N1_, m_,
                                             om_ == sq::optMaximize, d_r_.p, d_E64_.p, nullptr, st_.get()));
@@ -1063,7 +1079,7 @@ private:
     bool useTc() const { return d_digits1_.p && sq103_bipartite_tc_pays(N0_, N1_, m_); }
 
     void makeDigits() {
-        lowMade_ = false;
+        low_.made = false;
         if (!d_digits1_.p) return;
         SQ_CHECK(sq103_tc_make_digits(d_J_.p, N0_, N1_, N0_, 0, d_digits1_.p, st_.get()));
         SQ_CHECK(sq103_tc_make_digits(d_J_.p, N0_, N0_, N1_, 1, d_digits0_.p, st_.get()));
@@ -1174,8 +1190,7 @@ private:
     DevBuf<double> d_c64_, d_scratch_, d_E64_, d_r_;
     DevBuf<double> d_J64_, d_h0_64_, d_h1_64_;        // FP64 problem of a <double> annealer
     DevBuf<unsigned char> d_digits1_, d_digits0_, d_Abf_;  // tensor-core half-step fields
-    DevBuf<unsigned char> d_low1_;                         // tensor-core energies
-    bool lowMade_ = false;
+    LowDigits low_;                                        // tensor-core energies
     int uneven_ = 0;  // the digits are coarser than fp32 for some spin
     DevBuf<int> d_status_, d_uneven_;
     DevBuf<int8_t> d_q0_, d_q1_;
@@ -2248,10 +2263,9 @@ public:
         r_.ensure((size_t)in.m * in.N);
         energyBuffer(in.m);
         double *dE = E64_.p + 1;
-        if (in.digits.p) {  // as the single annealer; the low digits in a shared scratch
-            low_.ensure(sq103_tc_digits_bytes(in.N, in.N));
-            SQ_CHECK(sq103_tc_make_low_digits(in.J, in.ldJ, in.N, in.N, in.digits.p, low_.p, st_.get()));
-            SQ_CHECK(sq103_tc_row_sums(in.digits.p, low_.p, in.N, in.N, in.q, in.N, in.m, in.Abf.p, r_.p,
+        low_.made = false;  // the buffer held another instance's
+        if (in.digits.p && low_.make(in.J, in.ldJ, in.N, in.N, in.digits.p, st_.get())) {  // as the single annealer
+            SQ_CHECK(sq103_tc_row_sums(in.digits.p, low_.buf.p, in.N, in.N, in.q, in.N, in.m, in.Abf.p, r_.p,
                                        (int *)E64_.p, st_.get()));
             SQ_CHECK(sq103_dense_energy_of_sums(r_.p, in.h, in.c64, in.q, in.N, in.m, optimize_[i], dE, nullptr,
                                                 st_.get()));
@@ -2262,6 +2276,7 @@ public:
         hE_.resize((size_t)in.m + 1);
         SQ_CHECK(cudaMemcpyAsync(hE_.data(), E64_.p, sizeof(double) * (in.m + 1), cudaMemcpyDeviceToHost, st_.get()));
         st_.sync();
+        low_.trim();
         int status = 0;
         memcpy(&status, hE_.data(), sizeof(int));
         if (status != 0) {
@@ -2414,7 +2429,7 @@ private:
     DevBuf<float> dW_, sched_;
     DevBuf<double> scratch_, r_, E64_;
     std::vector<double> hE_;
-    DevBuf<unsigned char> low_;  // low digits of the instance whose energies are computed
+    LowDigits low_;  // of the instance whose energies are computed
     DevBuf<sq103_dense_task> dTasks_;
     DevBuf<int> dOrder_, dPos_, dQueue_, dStatus_;
     DevBuf<sq103_field_job> dJobs_;  // the SIMT refresh of every instance below the tensor-core size
