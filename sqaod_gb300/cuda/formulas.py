@@ -120,6 +120,20 @@ def _dense_rows(W, x, caption):
     return np.ascontiguousarray(x.reshape(-1, W.shape[0]))
 
 
+def _symmetric(W, then=None):
+    """(W, then()) with the outcome of symmetrize(W) before the checks of `then`, without its
+    allclose pass: the exact check of a symmetric W follows on the device.  That check
+    passes over the diagonal, where symmetrize refuses a NaN; and where `then` raises, a W
+    that is refused is reported first."""
+    if np.isnan(W.diagonal()).any():
+        W = common.symmetrize(W)
+    try:
+        return W, then() if then else None
+    except Exception:
+        common.symmetrize(W)
+        raise
+
+
 def _bipartite_problem(v0, v1, M, names):
     _vector(names[0], v0)
     _vector(names[1], v1)
@@ -152,7 +166,7 @@ def dense_graph_batch_calculate_E(W, x, dtype):
     dtype = _check_dtype(dtype)
     W = common.fix_type(W, dtype)
     _square('W', W)
-    x = _dense_rows(W, common.fix_type(x, np.int8), 'W, x')
+    W, x = _symmetric(W, lambda: _dense_rows(W, common.fix_type(x, np.int8), 'W, x'))
     E = np.empty(x.shape[0], np.float64)
     common.submit_symmetric(W, dtype, lambda W: _dg(dtype)('calculate_E', ptr(W), _c_int(W.shape[0]), ptr(x),
                                                            _c_int(x.shape[0]), ptr(E)))
@@ -164,6 +178,7 @@ def dense_graph_calculate_hamiltonian(W, dtype):
     dtype = _check_dtype(dtype)
     W = common.fix_type(W, dtype)
     _square('W', W)
+    W, _ = _symmetric(W)
     N = W.shape[0]
     h = np.empty(N, dtype)
     J = np.empty((N, N), dtype)
@@ -184,10 +199,13 @@ def dense_graph_batch_calculate_E_from_spin(h, J, c, q, dtype):
     h, J = common.fix_type([h, J], dtype)
     _vector('h', h)
     _square('J', J)
-    _scalar('c', c)
-    if h.shape[0] != J.shape[0]:
-        _dims('h, J', h, J)
-    q = _dense_rows(J, q, 'J, q')
+
+    def rows():
+        _scalar('c', c)
+        if h.shape[0] != J.shape[0]:
+            _dims('h, J', h, J)
+        return _dense_rows(J, q, 'J, q')
+    J, q = _symmetric(J, rows)
     E = np.empty(q.shape[0], np.float64)
     common.submit_symmetric(J, dtype, lambda J: _dg(dtype)('calculate_E_from_spin', ptr(h), ptr(J),
                                                            _real(dtype)(float(c)), _c_int(J.shape[0]), ptr(q),
