@@ -20,6 +20,7 @@
 // D[j] (bf_bip_min); only the x1 whose minimum is within the slack are searched
 // state by state (bf_bip_pass: one CTA per x1, 7-bit-group lookups over x0).  A
 // range that does not hold every x0 is searched state by state in both passes.
+#include <algorithm>
 #include <cstdint>
 #include <cstring>
 
@@ -613,34 +614,44 @@ __global__ void __launch_bounds__(kBfThreads) bf_bip_pass(const float *b0, const
         bip_x1_states<PASS == 1>(S, b0, b1, W, N0, N1, x0b, x0e, x1, thr, ws, cand, cap);
 }
 
-// collection over all x0, after bf_bip_min: a CTA takes 8 x 32 x1 at a time and
-// searches those whose minimum over all x0 is within reach, thr and the slack
-// once more (the minimum and a state's energy are rounded differently).
-// A search of N0 = N1 = 15: 176 us (1181 us state by state).
+// collection over all x0, after bf_bip_min: the first nWarps warps of a CTA take a unit
+// each, a block of 32 x1 or one of its 2^partBits parts, and the CTA searches those of the
+// units' x1 whose minimum over all x0 is within reach, thr and the slack once more (the
+// minimum and a state's energy are rounded differently).  All may be within reach
+// (nonnegative W without biases), so few blocks are spread over the SMs: N0 = 17, N1 = 14
+// of that kind took 15.3 ms a search with eight blocks a CTA, 10.8 with about two units per
+// SM, 10.4 state by state in both passes.  Parts repeat the block's minima, so they are
+// for launches of fewer blocks than that (N0 of 25 and more, few x1).  A search of N0 = N1
+// = 15 with one minimum: 111 us (1100 us state by state).
 __global__ void __launch_bounds__(kBfThreads) bf_bip_collect(const float *b0, const float *b1, const float *W, int N0,
-                                                             int N1, uint64_t x1b, uint64_t x1e, float slack,
-                                                             BfWorkspace *ws, uint64_t *cand, int cap) {
+                                                             int N1, uint64_t x1b, uint64_t x1e, int nWarps,
+                                                             int partBits, float slack, BfWorkspace *ws, uint64_t *cand,
+                                                             int cap) {
     __shared__ BipShared S;
     constexpr int kWarps = kBfThreads / 32;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const float thr = dec_float(ws->minEnc) + slack;
-    for (uint64_t X0 = (x1b >> 5) + (uint64_t)blockIdx.x * kWarps; X0 <= (x1e - 1) >> 5;
-         X0 += (uint64_t)gridDim.x * kWarps) {
-        const uint64_t X = X0 + warp, x1 = (X << 5) + lane;
-        float e = __int_as_float(0x7f800000);
-        if (X <= (x1e - 1) >> 5) e = bip_min32(b0, b1, W, N0, N1, X);
-        const unsigned reach = __ballot_sync(0xffffffffu, x1 >= x1b && x1 < x1e && e <= thr + slack);
-        if (lane == 0) S.reach[warp] = reach;
+    const uint64_t Xb = x1b >> 5, units = (((x1e - 1) >> 5) - Xb + 1) << partBits;
+    for (uint64_t U0 = (uint64_t)blockIdx.x * nWarps; U0 < units; U0 += (uint64_t)gridDim.x * nWarps) {
+        if (warp < nWarps) {
+            const uint64_t U = U0 + warp, X = Xb + (U >> partBits), x1 = (X << 5) + lane;
+            float e = __int_as_float(0x7f800000);
+            if (U < units) e = bip_min32(b0, b1, W, N0, N1, X);  // (every lane: the minima are warp-wide)
+            const bool mine = lane >> (5 - partBits) == (int)(U & ((1u << partBits) - 1u));
+            const unsigned reach =
+                __ballot_sync(0xffffffffu, mine && U < units && x1 >= x1b && x1 < x1e && e <= thr + slack);
+            if (lane == 0) S.reach[warp] = reach;
+        }
         __syncthreads();
         unsigned todo[kWarps];
 #pragma unroll
-        for (int w = 0; w < kWarps; ++w) todo[w] = S.reach[w];
+        for (int w = 0; w < kWarps; ++w) todo[w] = w < nWarps ? S.reach[w] : 0u;
         __syncthreads();
 #pragma unroll
         for (int w = 0; w < kWarps; ++w)
             for (unsigned t = todo[w]; t; t &= t - 1u)
-                bip_x1_states<true>(S, b0, b1, W, N0, N1, 0, 1ull << N0, ((X0 + w) << 5) + (__ffs(t) - 1), thr, ws,
-                                    cand, cap);
+                bip_x1_states<true>(S, b0, b1, W, N0, N1, 0, 1ull << N0,
+                                    ((Xb + ((U0 + w) >> partBits)) << 5) + (__ffs(t) - 1), thr, ws, cand, cap);
     }
 }
 
@@ -784,7 +795,12 @@ SQ103_API int sq103_bipartite_bf_range(const float *b0, const float *b1, const f
     if (x0b == 0 && x0e == 1ull << N0 && (x1e - x1b >= 1ull << 13 || N0 >= 25 || (x1e - x1b) << N0 >= 1ull << 25)) {
         const int grid = bf_grid((((x1e - 1) >> 5) - (x1b >> 5) + kBfThreads / 32) / (kBfThreads / 32), 8);
         bf_bip_min<<<grid, kBfThreads, 0, s>>>(b0, b1, W, N0, N1, x1b, x1e, w);
-        bf_bip_collect<<<grid, kBfThreads, 0, s>>>(b0, b1, W, N0, N1, x1b, x1e, slack, w, cand, cap);
+        const uint64_t blocks = ((x1e - 1) >> 5) - (x1b >> 5) + 1, full = (uint64_t)bf_grid(~0ull, 2);
+        const int nWarps = (int)std::max<uint64_t>(1, std::min<uint64_t>(kBfThreads / 32, blocks / full));
+        int partBits = 0;
+        while (partBits < 5 && blocks << (partBits + 1) <= full) ++partBits;
+        bf_bip_collect<<<bf_grid(((blocks << partBits) + nWarps - 1) / nWarps, 8), kBfThreads, 0, s>>>(
+            b0, b1, W, N0, N1, x1b, x1e, nWarps, partBits, slack, w, cand, cap);
     } else {
         const int grid = bf_grid(x1e - x1b, 8);
         bf_bip_pass<0><<<grid, kBfThreads, 0, s>>>(b0, b1, W, N0, N1, x0b, x0e, x1b, x1e, slack, w, cand, cap);
