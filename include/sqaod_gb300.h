@@ -491,9 +491,9 @@ SQ103_API int sq103_dense_batch_prepare(void *handle);
 /* Instances of at least N spins (m >= 2, fitting the device) are stepped by the
  * one-CTA-per-trotter sweep in packed cooperative launches, the rest by the
  * persistent batch kernel; both give the same results.  Without a call, the
- * limit is 1024 and the packed launches also take the smaller instances along,
- * from 64 spins (128 in batches of more than 152 instances); 0 keeps every
- * instance on the persistent kernel.  Takes effect at the next prepare. */
+ * limit is 1024 and the packed launches also take smaller instances along, down
+ * to the size, 64 spins or more, with the least estimated time for the batch; 0
+ * keeps every instance on the persistent kernel.  Takes effect at the next prepare. */
 SQ103_API int sq103_dense_batch_set_multicta_min_n(void *handle, int N);
 /* instances of at least the limit (1024 without a call) on the one-CTA-per-trotter
  * sweep since the last prepare, without the smaller ones taken along */

@@ -59,10 +59,10 @@ class DenseBatchAnnealer:
     def set_multicta_min_n(self, N):
         """Instances of at least N spins run on the one-CTA-per-trotter sweep
         (packed launches); 0 keeps all on the persistent kernel.  Without a
-        call the limit is 1024 and the packed launches also take the smaller
-        instances along, from 64 spins (128 in batches of more than 152
-        instances); results do not depend on it.  Takes effect at the next
-        prepare()."""
+        call the limit is 1024 and the packed launches also take smaller
+        instances along, down to the size, 64 spins or more, with the least
+        estimated time for the batch; results do not depend on it.  Takes
+        effect at the next prepare()."""
         self._call("set_multicta_min_n", ctypes.c_int(N))
 
     def multicta_count(self):

@@ -30,6 +30,7 @@
 #include <sqaodc/sqaodc.h>
 
 #include "host_util.h"
+#include "route_cost.h"
 #include "sq_common.cuh"
 #include "sq_kernels.h"
 
@@ -1926,7 +1927,7 @@ private:
 class DenseBatch : public sq::NullBase {
 public:
     static constexpr int kRefreshPeriod = 8;
-    static constexpr int kPackMax = 64;          // instances per packed launch
+    static constexpr int kPackMax = kPackInstances;
     static constexpr int kDefaultMultiMinN = 1024;
 
     // Instances of at least a size limit (prepare(); with m >= 2 that fit the device)
@@ -2007,17 +2008,7 @@ public:
         std::vector<sq103_dense_task> tasks;
         std::vector<Inst *> smallInsts;
         multi_.clear();
-        // Without a limit of the caller's, the packed launches also take the smaller
-        // instances: the persistent kernel's step lasts as long as its longest chain
-        // (two phases of about 4 us per iteration), a packed launch takes 32 iterations
-        // in about 3 us.  Measured, 16 steps of n instances of 64 to 2048 spins, ms by
-        // size limit:    n      1024   512   256   128    64
-        //               16      72.3  31.7   9.9   6.1   4.1
-        //              128       133  43.7  35.6  26.0  25.1
-        //              300       164  89.1  65.3  57.8  59.7
-        //             1024       246   184   178   185   191
-        // so 64 (the kernel's least) for few instances and 128 for many.
-        const int minN = limitGiven_ ? multiMinN_ : nAll <= 152 ? 64 : 128;
+        const int minN = limitGiven_ ? multiMinN_ : defaultLimit();
         int maxN = 0, maxM = 0;
         for (int i = 0; i < nAll; ++i) {
             Inst &in = *insts_[i];
@@ -2294,6 +2285,27 @@ public:
     }
 
 private:
+    // Without a limit of the caller's, the packed launches also take the smaller instances
+    // along, down to the size with the least estimate for the whole batch (route_cost.h): the
+    // persistent kernel's step lasts as long as its longest chain, the packed launches as
+    // long as all of them together.  128 uneven instances of 64 to 2048 spins, 16 steps:
+    // 133 ms with a limit of 1024, 25 with the one chosen.
+    int defaultLimit() const {
+        std::vector<DenseRoute> items;
+        int dev = 0, sms = 0;
+        SQ_CHECK(cudaGetDevice(&dev));
+        SQ_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        const int stage = smem_ < 0 ? std::min(sq103_dense_batch_max_smem(), 96 * 1024) : smem_;
+        for (const auto &p : insts_) {
+            const int N = p->N, m = p->m;
+            const bool packs = m >= 2 && sq103_dense_multicta_ok(N, m, kColoring);
+            const bool staged = (long long)sq103_dense_batch_min_smem(m) + (long long)m * N * 5 + 4ll * N <= stage;
+            items.push_back({N, m, packs ? sq103_dense_multicta_capacity(N) : 0, dense_persistent_us(N, m, staged),
+                             packs && N >= kDefaultMultiMinN});
+        }
+        return std::min(dense_route_limit(items, 2 * sms, 1 << 30), kDefaultMultiMinN);
+    }
+
     // Raises when a sweep or a field refresh gave up a bounded wait since prepare(): the
     // batch's spins are not valid then.  Read once after the steps queued last.
     void checkStatus() {

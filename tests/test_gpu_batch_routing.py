@@ -1,17 +1,23 @@
 """Which instances a batch steps in packed one-CTA-per-trotter launches: those of at least
-the caller's limit, or without one those of 64 spins (128 in batches of more than 152)."""
+the caller's limit; without one, small ones where they are few or have few trotters, and
+none of them where their packed launches, one after another, would take longer than the
+persistent kernel, which runs all at once (measured for each of these: 2 to 20 times)."""
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
 
+ALL = [(64, 4), (65, 4), (100, 4)]
 
-@pytest.mark.parametrize("copies,limit,least", [(1, None, 64), (51, None, 128), (51, 65, 65), (1, 1024, 1024),
-                                                (1, 0, None)])
-def test_packed_count(copies, limit, least):
+
+@pytest.mark.parametrize("sizes,limit,packed", [
+    (ALL, None, 3), (ALL * 60, None, 180), ([(64, 256)] * 4, None, 4),
+    ([(64, 256)] * 60, None, 0), ([(64, 64)] * 150, None, 0), ([(64, 64)] * 150 + [(2000, 8)], None, 1),
+    ([(63, 4), (64, 1), (128, 4)], None, 1),
+    ([(64, 256)] * 60, 64, 60), (ALL, 65, 2), (ALL, 1024, 0), (ALL, 0, 0)])
+def test_packed_count(sizes, limit, packed):
     import sqaod_gb300 as sq
     from sqaod_gb300.batch import DenseBatchAnnealer
-    sizes = [(63, 4), (64, 4), (127, 1), (128, 4)] * copies if copies == 1 else [(127, 4), (128, 4), (64, 4)] * copies
     b = DenseBatchAnnealer()
     problems = {}
     for N, m in sizes:
@@ -23,4 +29,4 @@ def test_packed_count(copies, limit, least):
     if limit is not None:
         b.set_multicta_min_n(limit)
     b.prepare()
-    assert b.packed_count() == sum(1 for N, m in sizes if least is not None and N >= least and m >= 2)
+    assert b.packed_count() == packed
