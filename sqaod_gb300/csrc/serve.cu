@@ -30,6 +30,7 @@
 #include <vector>
 
 #include "host_util.h"
+#include "route_cost.h"
 #include "sq_common.cuh"
 #include "sq_kernels.h"
 
@@ -135,6 +136,8 @@ public:
         int slot = -1;   // batch slot, -1 for the per-instance kernel
         bool large = false;  // outside the persistent kernels: packed launches (dense), a side stream (bipartite)
         bool heavy = false;  // large by its size alone (counts against the large-request limit)
+        int packCap = 0;           // dense: resident trotters of a packed launch (0: none takes it)
+        double persistentUs = 0.;  // a tick in the persistent kernel (estimate)
         sq103_dense_task dt = {};
         sq103_bipartite_task bt = {};
         double *c64 = nullptr;
@@ -235,17 +238,17 @@ public:
     // next range of every active search; returns the number of requests completed
     int tick() {
         const int nDone = finalizeReady(false);
+        join();  // (nothing is taken, unless an earlier tick raised)
         admit();
         const int nD = (int)denseSlots_.size(), nB = (int)bipSlots_.size();
         // The persistent kernels, and the bipartite requests outside them (each one's
         // launches in order), go to the side streams: each fills only part of the GPU, and
         // they run side by side and beside the packed launches below (24 mixed requests, 32
         // steps: 15.7 ms with the persistent kernels first on the work stream, 14.2 so).
+        // A tick with nothing but one persistent kernel leaves it on the work stream.
         int nSide = 0;
-        auto side = [&]() -> cudaStream_t {
-            if (nSide == 0) fork();
-            return side_[nSide++ % kRefreshStreams].get();
-        };
+        const bool alone = (nD > 0) + (nB > 0) + (int)large_.size() == 1;
+        auto side = [&]() -> cudaStream_t { return alone ? st_.get() : fork(nSide++); };
         if (nD > 0)
             SQ_CHECK(sq103_dense_batch_launch(dTasks_.p, nD, counts_.p, nullptr, dPos_.p, queues_.p, kStepsPerTick,
                                               std::min(denseGrid_, nD), stageSmem_, side()));
@@ -287,7 +290,7 @@ public:
             packN = std::max(packN, r->N0);
         }
         flush();
-        if (nSide > 0) join();
+        join();
         std::vector<Request *> finished;
         jobs_.clear();
         tileJob_.clear();
@@ -303,10 +306,8 @@ public:
             r->pos = std::min(r->pos + kStepsPerTick, r->nSteps);
             if (r->kind == 0 && r->pos < r->nSteps && r->pos % kRefreshPeriod == 0) {
                 if (r->digits) {  // on the side streams, forked from the work stream at the first
-                    if (nTc == 0) fork();
                     SQ_CHECK(sq103_dense_refresh(r->dt.J, r->dt.ldJ, r->digits, r->spinsBf16, r->dt.q, r->dt.F, r->N0,
-                                                 r->m, r->dStatus, side_[nTc % kRefreshStreams].get()));
-                    ++nTc;
+                                                 r->m, r->dStatus, fork(nTc++)));
                 } else {  // below the tensor-core size: with the others, in one launch
                     sq103_field_job j = {};
                     j.J = r->dt.J;
@@ -330,7 +331,7 @@ public:
             stage_.copy(dTileJob_.p, tileJob_.data(), sizeof(int) * tileJob_.size(), st_.get());
             SQ_CHECK(sq103_dense_field_refresh_batch(dJobs_.p, dTileJob_.p, (int)tileJob_.size(), st_.get()));
         }
-        if (nTc > 0) join();  // the next work on the stream sees every refreshed field
+        join();  // the next work on the stream sees every refreshed field
         for (Request *r : finished) finish(r);
         // searches: the next range of each, on the searcher's stream (the anneals
         // queued above run meanwhile)
@@ -355,17 +356,21 @@ public:
         return nDone + nSearched;
     }
 
-    // the side streams start after the work queued so far on the work stream ...
-    void fork() {
-        SQ_CHECK(cudaEventRecord(fork_, st_.get()));
-        for (Stream &x : side_) SQ_CHECK(cudaStreamWaitEvent(x.get(), fork_, 0));
+    // Side stream i (modulo their number): it starts after the work queued on the work
+    // stream when the first one was taken since the last join ...
+    cudaStream_t fork(int i) {
+        const int k = i % kRefreshStreams;
+        if (forked_ == 0) SQ_CHECK(cudaEventRecord(fork_, st_.get()));
+        for (; forked_ <= k; ++forked_) SQ_CHECK(cudaStreamWaitEvent(side_[forked_].get(), fork_, 0));
+        return side_[k].get();
     }
-    // ... and the work stream continues after everything queued on them
+    // ... and the work stream continues after everything queued on those taken
     void join() {
-        for (int k = 0; k < kRefreshStreams; ++k) {
+        for (int k = 0; k < forked_; ++k) {
             SQ_CHECK(cudaEventRecord(join_[k], side_[k].get()));
             SQ_CHECK(cudaStreamWaitEvent(st_.get(), join_[k], 0));
         }
+        forked_ = 0;
     }
 
     int state(int id) const {
@@ -439,6 +444,10 @@ private:
                      (unsigned long long)rq->bytes, budget_);
         // energies as the single-instance annealers', unless their scratch would exceed the
         // budget: then the SIMT sums, which need none (the last bits may differ)
+        rq->packCap = rq->kind == 0 && sq103_dense_multicta_ok(rq->N0, m, kColoring) ? sq103_dense_multicta_capacity(rq->N0) : 0;
+        rq->persistentUs = rq->kind == 0   ? dense_persistent_us(rq->N0, m, fitsStaging(*rq))
+                           : rq->kind == 1 ? bipartite_persistent_us(rq->N0, rq->N1, m)
+                                           : 0.;
         rq->tcEnergies = tcEnergies(*rq) && rq->bytes + scratchBytes(*rq) <= budget_;
         Request *p = rq.get();
         all_[p->id] = std::move(rq);
@@ -513,20 +522,48 @@ private:
         return base + (size_t)r.m * r.N0 * 5 + (size_t)r.N0 * 4 <= (size_t)stageSmem_;
     }
 
-    // A request the persistent kernels could hold takes a large one's route while few
-    // are there: one CTA runs a request's whole tick in the persistent kernels (8 steps
-    // of N = 1000, m = 16: 9.9 ms; of a 400 x 300, m = 256 bipartite one: 6.6 ms), and
-    // a tick lasts as long as its longest request.  The packed launch takes 8 steps of
-    // N = 1000 in 0.8 ms, and the per-instance bipartite kernels about 0.3 ms, but each
-    // bipartite request so costs 32 launches a tick, which the limits below keep in
-    // proportion.  Mixed set of 24 requests, 32 steps: 84.8 ms with the persistent
-    // kernels, 20.1 ms this way.
+    // A request the persistent kernels could hold takes a large one's route where that
+    // shortens the tick (route_cost.h): there one CTA runs a request's whole tick (8 steps of
+    // N = 1000, m = 16: 9.9 ms; of a 400 x 300, m = 256 bipartite one: 6.6 ms), and the tick
+    // lasts as long as its longest request; the packed launches, and the host's launches for
+    // bipartite requests (32 a tick each), follow one another.  planRoutes() weighs the
+    // requests in the queue against each other and those that run.  Mixed set of 24
+    // requests, 32 steps: 84.8 ms with the persistent kernels alone, 14.3 this way.
+    void planRoutes() {
+        std::vector<DenseRoute> dense;
+        std::vector<double> bip;
+        double running = 0.;
+        for (const auto &kv : active_) {
+            const Request *r = kv.second;
+            if (r->done || r->kind == kSearch) continue;
+            if (r->kind == 0)
+                dense.push_back({r->N0, r->m, r->large ? r->packCap : 0, r->persistentUs, r->large});
+            else if (!r->large)
+                running = std::max(running, r->persistentUs);
+        }
+        for (const Request *r : queue_) {
+            if (r->kind == 0)
+                dense.push_back({r->N0, r->m, r->packCap, r->persistentUs, heavy_(*r)});
+            else if (r->kind == 1 && !heavy_(*r))
+                bip.push_back(r->persistentUs);
+        }
+        lightFrom_ = dense_route_limit(dense, 2 * sms_, 1 << 30);
+        bipCut_ = bipartite_route_cut(bip, running, nLight_[1], kMaxLightBip - nLight_[1]);
+    }
     bool light_(const Request &r) const {
-        if (r.kind == 1) return nLight_[1] < kMaxLightBip;
-        if (r.kind != 0 || !sq103_dense_multicta_ok(r.N0, r.m, kColoring)) return false;
+        if (r.kind == 1) return nLight_[1] < kMaxLightBip && r.persistentUs >= bipCut_;
         // (dense: with the accept-word workspace inside the budget)
-        return nLight_[0] < (r.N0 >= 128 ? kMaxLightDense : kMaxLightSmall) &&
+        return r.kind == 0 && r.packCap > 0 && r.N0 >= lightFrom_ &&
+               nLight_[0] < (r.N0 >= 128 ? kMaxLightDense : kMaxLightSmall) &&
                used_ + r.bytes + scratchGrowth(r) + al(sq103_dense_ws_bytes(r.N0, r.m, kStepsPerTick)) <= budget_;
+    }
+    // large by its size alone; bipartite requests whose fields the single-instance annealer
+    // computes on the tensor cores at any coupling take the per-instance kernels, as it does
+    bool heavy_(const Request &r) const {
+        return r.kind == kSearch ? false
+               : r.kind == 0     ? !fitsStaging(r) && r.packCap > 0
+                                 : (size_t)r.m * r.N0 * r.N1 > kBipLargeWork ||
+                                   sq103_bipartite_refresh_uses_tc(r.N0, r.N1, r.m);
     }
 
     // Admits queued requests in arrival order as memory, slots and the large-instance
@@ -534,16 +571,12 @@ private:
     // block the ones behind it.
     void admit() {
         releaseIdleScratch();
+        if (!queue_.empty()) planRoutes();
         bool changed = false;
         size_t i = 0;
         while (i < queue_.size()) {
             Request *r = queue_[i];
-            // bipartite requests whose fields the single-instance annealer computes on the
-            // tensor cores take the per-instance kernels, which do the same
-            const bool heavy = r->kind == kSearch ? false
-                               : r->kind == 0 ? !fitsStaging(*r) && sq103_dense_multicta_ok(r->N0, r->m, kColoring)
-                                              : (size_t)r->m * r->N0 * r->N1 > kBipLargeWork ||
-                                                    sq103_bipartite_refresh_uses_tc(r->N0, r->N1, r->m);
+            const bool heavy = heavy_(*r);
             const bool light = !heavy && light_(*r);
             const bool fits =
                 used_ + r->bytes + scratchGrowth(*r) <= budget_ &&
@@ -860,6 +893,7 @@ private:
     static constexpr int kRefreshStreams = 8;  // (24 mixed requests: 14.45 ms with 4, 14.2 with 8)
     Stream side_[kRefreshStreams];
     cudaEvent_t fork_ = nullptr, join_[kRefreshStreams] = {};
+    int forked_ = 0;  // side streams taken since the last join
     // this tick's SIMT field refreshes (host table, device copy)
     std::vector<sq103_field_job> jobs_;
     std::vector<int> tileJob_;
@@ -884,10 +918,14 @@ private:
     // the active requests' largest need, part of used_
     AsyncMem scratch_;
     size_t scratchSize_ = 0;
-    static constexpr int kMaxPack = 64;  // instances per packed launch (sq103_dense_anneal_pack)
+    static constexpr int kMaxPack = kPackInstances;
     // light requests on the large ones' routes at a time: dense of N >= 128, dense below, bipartite
     static constexpr int kMaxLightDense = 512, kMaxLightSmall = 64, kMaxLightBip = 32;
     int nHeavy_ = 0, nLight_[2] = {0, 0};
+    // this tick's routes (planRoutes): dense requests of at least this size, and bipartite
+    // ones of at least this persistent time, take the large ones' routes
+    int lightFrom_ = 1 << 30;
+    double bipCut_ = 1e300;
 };
 
 }  // namespace sq103
