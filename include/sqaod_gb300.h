@@ -133,9 +133,11 @@ SQ103_API int sq103_tc_refresh(const void *digits, int R, int K, const int8_t *q
                                float *F, int ldF, int flags, int *status, void *stream);
 /* 1 when the dense annealers refresh N-spin fields on the tensor cores (N >= 1024) */
 SQ103_API int sq103_dense_refresh_uses_tc(int N);
-/* 1 when the bipartite annealers compute the half-step fields on the tensor cores
- * (N0 N1 >= 2^20 and at least 64 output tiles of 128 trotters x 64 spins per half
- * step); the task then carries the digits of J and J^T */
+/* 1 when the half-step fields come from the tensor cores whatever the couplings (N0 N1
+ * >= 2^20 and at least 64 output tiles of 128 trotters x 64 spins per half step); the
+ * task then carries the digits of J and J^T.  The single-instance annealer also takes
+ * them for fewer tiles, from about 80 M products a half-step, when the digits hold
+ * every spin's couplings as finely as fp32.  Decisions are exact on either kind. */
 SQ103_API int sq103_bipartite_refresh_uses_tc(int N0, int N1, int m);
 /* the dense refresh of every path: sq103_tc_refresh from `digits` (of J, R = K = N)
  * when given, else sq103_dense_field_refresh */
@@ -367,7 +369,9 @@ SQ103_API int sq103_dg_annealer_get_checkpoint(void *handle, int8_t *q, float *F
 SQ103_API int sq103_dg_annealer_set_checkpoint(void *handle, const int8_t *q, const float *F, int m, int N,
                                                unsigned long long seed, uint32_t step, int sinceRefresh);
 SQ103_API int sq103_dg_annealer_set_trace(void *handle, int enable);
-/* kernel selection for the sweep: 0 = automatic, 1 = one CTA per instance, 2 = one CTA per trotter */
+/* kernel selection for the sweep: 0 = automatic, 1 = one CTA per instance, 2 = one CTA per
+ * trotter (N >= 64, 2 <= m <= sq103_dense_multicta_capacity(N), 608 at most on 152 SMs;
+ * a sweep outside that is refused) */
 SQ103_API int sq103_dg_annealer_set_kernel(void *handle, int flags);
 SQ103_API int sq103_dg_annealer_get_trace(void *handle, uint32_t *bits, int nwords);
 
@@ -622,7 +626,9 @@ SQ103_API int sq103_server_result(void *handle, int id, double *E, int capE, int
 SQ103_API int sq103_server_stats(void *handle, int *queued, int *active, int *done,
                                  unsigned long long *bytesInUse);
 /* at most n large instances admitted at a time (default 64; dense: one CTA per
- * trotter, packed up to 64 per launch; bipartite: per-instance kernels) */
+ * trotter, packed up to 64 per launch; bipartite: per-instance kernels).  Smaller
+ * requests that the server steps in the same launches, where that shortens a tick, do
+ * not count. */
 SQ103_API int sq103_server_set_large_limit(void *handle, int n);
 /* Fault injection from the host (tests; no counterpart in the reference): writes
  * `value` into the status word of active dense request `id`, in stream order, as a

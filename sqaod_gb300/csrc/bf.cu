@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(128) bf_lo_table(const float *W, int N, int L,
 //   E = (E_ll + tB[lo & 31]) + (tA1[lo >> 10] + tA2[(lo >> 5) & 31]),
 // tA1 holding E_hh(hi).  That is one packed addition (two states) and one
 // three-input minimum (two more states) per pair, the additions on the FMA pipe
-// and the minima on the ALU, so a state costs about 1.3 instructions; the
+// and the minima on the ALU, so a state costs about 1.5 instructions; the
 // per-state lookups of bf_dense_pass cost about 15.  The sums over hi split into
 // the run's upper bits (21 short FP64 sums per run) and tables over its six low
 // bits (once per CTA).  The rounding is of the same count as bf_dense_pass's and
@@ -445,7 +445,7 @@ __global__ void __launch_bounds__(kBfThreads) bf_dense_pass(const float *W, int 
 
 // The minimum over all x0 of each of the 32 x1 that share their bits from 5 on
 // (X5 = x1 >> 5), warp-wide; lane t returns that of x1 = 32 X5 + t.  Lane j holds
-// D[j] (and j + 32), lane 31 b1.x1; a Gray walk over the low five bits changes
+// D[j] (and j + 32), every lane b1.x1; a Gray walk over the low five bits changes
 // them by one FP64 row per x1.  The negative D, rounded to fp32, are summed by a
 // fixed tree.
 __device__ __forceinline__ float bip_min32(const float *b0, const float *b1, const float *W, int N0, int N1,

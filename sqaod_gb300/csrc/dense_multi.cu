@@ -258,8 +258,7 @@ struct McPack {
 // (short waits, a trotter that withholds its accept words).  kSA: simulated
 // annealing, without the neighbours' code.  Code that never runs is not free here:
 // the warps' roles share the instruction caches, and SA at N = 1501, m = 63 took
-// SAOLD ms for 64 steps with the neighbours' and the trace's code compiled in,
-// SANEW ms without.
+// 3.24 ms for 64 steps with the neighbours' code compiled in, 3.12 without.
 // kSmall: rows of at most kSmallN spins, where the neighbours' sites hit a lane's
 // site often: each prefetcher finds a lane's neighbour candidates from a table
 // of the positions at each site of batches p - 2 .. p (one per batch and
@@ -269,9 +268,9 @@ struct McPack {
 // makes the prefetchers wait for each other).  Both give the same candidates.
 // kPerSm: the CTAs per SM the registers are allotted for.  The trotters of a launch
 // are all resident, so the limit on m is kPerSm * 152 (where shared memory allows
-// as many: N <= 3100 for four).  Two leave 118 registers a thread and the fastest
-// decider; four have 64 (8 bytes spilled) and take the launches that exceed two.
-// N = 2000, m = 500, 8 steps: 7.4 ms with four per SM; one CTA for the whole
+// as many: N <= 3100 for four).  Two leave 114 registers a thread and the fastest
+// decider; four have 72 (up to 16 bytes spilled) and take the launches that exceed two.
+// N = 2000, m = 500, 8 steps: 3.7 ms with four per SM; one CTA for the whole
 // instance, which such sizes fell back to before, 1090 ms.
 template <bool kHooks, bool kSmall, bool kSA, int kPerSm>
 __global__ void __launch_bounds__(mc_threads(kPerSm), kPerSm) dense_sweep_multi(const __grid_constant__ McPack P) {

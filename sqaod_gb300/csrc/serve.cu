@@ -9,7 +9,8 @@
 // period):
 //   - dense instances whose spins and fields fit in shared memory, and small
 //     bipartite instances, in the persistent batch kernels (one launch each,
-//     instance count read on the device);
+//     instance count read on the device), unless the tick is shorter with some of
+//     them in the launches below (planRoutes);
 //   - large dense instances with the one-CTA-per-trotter kernel and large
 //     bipartite instances with the per-instance kernels, a few at a time;
 //   - dense fields are refreshed every 8 steps, as the single-instance annealer
@@ -683,7 +684,9 @@ private:
             }
         } else {
             const size_t N0 = r->N0, N1 = r->N1;
-            const bool tc = sq103_bipartite_refresh_uses_tc((int)N0, (int)N1, m);  // as the single-instance annealer
+            // digit fields for the largest shapes alone, where the single-instance annealer takes
+            // them for others too: the decisions are exact on either, so the spins are the same
+            const bool tc = sq103_bipartite_refresh_uses_tc((int)N0, (int)N1, m);
             size_t oG = 0, oB = al(n * 4), oJ = oB + al(n * 4), oh0 = oJ + al(N0 * N1 * 4), oh1 = oh0 + al(N0 * 4),
                    oc = oh1 + al(N1 * 4), oq0 = oc + 512, oq1 = oq0 + al(m * N0), oF0 = oq1 + al(m * N1),
                    oF1 = oF0 + al(m * N0 * 4), oR = oF1 + al(m * N1 * 4), oE = oR + al(std::max(m * N1, N0 + N1) * 8),

@@ -672,11 +672,13 @@ SQ103_API int sq103_bipartite_refresh_uses_tc(int N0, int N1, int m) {
 
 // Where the bipartite annealer takes its energies, and its half-step fields when the
 // digits hold every row (sq103_tc_check_even), to the tensor cores: as above, and from
-// about 80 M products a half-step on (m rounded up to a SIMT tile's 16 rows).  ms, SIMT and tensor cores: 1024 x 1024, m = 64, 64 steps (67 M)
-// 2.89, 3.70; 1100 x 2900, m = 20, 32 steps (102 M) 3.00, 2.15; 1100 x 1100, m = 150
-// (194 M) 3.75, 2.62; 2900 x 2900, m = 30 (269 M) 5.01, 3.07.  The
-// flips' tolerance covers the digits' rounding, so decisions are exact and the spins the
-// same on either; a path that returns energies (server) sums them the way the annealer does.
+// about 80 M products a half-step on (m rounded up to a SIMT tile's 16 rows).  32 steps in
+// ms, SIMT and tensor cores: 1024 x 1024, m = 64 (67 M) 1.10, 1.18, m = 65 (84 M) 1.57,
+// 1.20; 1100 x 1900, m = 33 (100 M) 2.17, 1.28; 600 x 9000, m = 1 (86 M) 5.33, 1.38; 2300 x
+// 2300, m = 1 (85 M) 2.21, 1.26, m = 16 2.50, 1.55, m = 129 6.72, 2.19.  (Below the line
+// larger sides gain too: 2048 x 2048, m = 1 1.97, 1.13.)  The flips' tolerance covers the
+// digits' rounding, so decisions are exact and the spins the same on either; a path that
+// returns energies (server) sums them the way the annealer does.
 int sq103_bipartite_tc_pays(int N0, int N1, int m) {
     if ((long long)N0 * (long long)N1 < (1ll << 20) || m < 1) return 0;
     return sq103_bipartite_refresh_uses_tc(N0, N1, m) || (double)((m + 15) / 16 * 16) * N0 * N1 >= 8e7;

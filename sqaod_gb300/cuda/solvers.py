@@ -264,7 +264,8 @@ class DenseGraphAnnealer(_Handle):
         return out
 
     def set_kernel(self, flags):
-        """Sweep kernel: 0 automatic, 1 one CTA per instance, 2 one CTA per trotter (extension)."""
+        """Sweep kernel: 0 automatic, 1 one CTA per instance, 2 one CTA per trotter (extension; up
+        to four trotters per SM, a sweep of more is refused)."""
         self._call('set_kernel', _c_int(flags))
 
 

@@ -130,7 +130,9 @@ class AnnealServer:
 
     def set_large_limit(self, n):
         """At most n large instances admitted at a time (default 64): dense ones on the
-        one-CTA-per-trotter path (packed launches), bipartite ones on the per-instance kernels."""
+        one-CTA-per-trotter path (packed launches), bipartite ones on the per-instance kernels.
+        Smaller requests that step in the same launches, where that shortens a tick, do not
+        count."""
         self._call("set_large_limit", ctypes.c_int(int(n)))
 
     def completed(self, cap=4096):
