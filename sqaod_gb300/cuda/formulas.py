@@ -120,18 +120,22 @@ def _dense_rows(W, x, caption):
     return np.ascontiguousarray(x.reshape(-1, W.shape[0]))
 
 
-def _symmetric(W, then=None):
-    """(W, then()) with the outcome of symmetrize(W) before the checks of `then`, without its
-    allclose pass: the exact check of a symmetric W follows on the device.  That check
-    passes over the diagonal, where symmetrize refuses a NaN; and where `then` raises, a W
-    that is refused is reported first."""
-    if np.isnan(W.diagonal()).any():
-        W = common.symmetrize(W)
+def _symmetric(W, dtype, submit, check=lambda: None):
+    """submit(W, check()) with the outcome of symmetrize(W) before both, without its allclose
+    pass: a symmetric W is checked exactly on the device.  That check passes over the
+    diagonal, where symmetrize refuses a NaN.  A NaN there makes the first value that submit
+    returns one, except that the float64 energies skip what a bit vector does not select, so
+    W is looked at again then, and in float64 its diagonal always (reading it takes some 5
+    us at N = 1000).  Where anything raises, a W that symmetrize refuses is reported first."""
     try:
-        return W, then() if then else None
+        arg = check()
+        result = common.submit_symmetric(W, dtype, lambda W: submit(W, arg))
     except Exception:
         common.symmetrize(W)
         raise
+    if result[0] != result[0] or (dtype == np.float64 and np.isnan(W.diagonal()).any()):
+        common.symmetrize(W)
+    return result
 
 
 def _bipartite_problem(v0, v1, M, names):
@@ -166,11 +170,12 @@ def dense_graph_batch_calculate_E(W, x, dtype):
     dtype = _check_dtype(dtype)
     W = common.fix_type(W, dtype)
     _square('W', W)
-    W, x = _symmetric(W, lambda: _dense_rows(W, common.fix_type(x, np.int8), 'W, x'))
-    E = np.empty(x.shape[0], np.float64)
-    common.submit_symmetric(W, dtype, lambda W: _dg(dtype)('calculate_E', ptr(W), _c_int(W.shape[0]), ptr(x),
-                                                           _c_int(x.shape[0]), ptr(E)))
-    return E.astype(dtype)
+
+    def submit(W, x):
+        E = np.empty(x.shape[0], np.float64)
+        _dg(dtype)('calculate_E', ptr(W), _c_int(W.shape[0]), ptr(x), _c_int(x.shape[0]), ptr(E))
+        return E
+    return _symmetric(W, dtype, submit, lambda: _dense_rows(W, common.fix_type(x, np.int8), 'W, x')).astype(dtype)
 
 
 def dense_graph_calculate_hamiltonian(W, dtype):
@@ -178,13 +183,15 @@ def dense_graph_calculate_hamiltonian(W, dtype):
     dtype = _check_dtype(dtype)
     W = common.fix_type(W, dtype)
     _square('W', W)
-    W, _ = _symmetric(W)
     N = W.shape[0]
     h = np.empty(N, dtype)
     J = np.empty((N, N), dtype)
     c = np.empty(1, dtype)
-    common.submit_symmetric(W, dtype, lambda W: _dg(dtype)('calculate_hamiltonian', ptr(W), _c_int(N), ptr(h), ptr(J),
-                                                           ptr(c)))
+
+    def submit(W, _):
+        _dg(dtype)('calculate_hamiltonian', ptr(W), _c_int(N), ptr(h), ptr(J), ptr(c))
+        return c
+    _symmetric(W, dtype, submit)
     return h, J, c[0]
 
 
@@ -205,12 +212,13 @@ def dense_graph_batch_calculate_E_from_spin(h, J, c, q, dtype):
         if h.shape[0] != J.shape[0]:
             _dims('h, J', h, J)
         return _dense_rows(J, q, 'J, q')
-    J, q = _symmetric(J, rows)
-    E = np.empty(q.shape[0], np.float64)
-    common.submit_symmetric(J, dtype, lambda J: _dg(dtype)('calculate_E_from_spin', ptr(h), ptr(J),
-                                                           _real(dtype)(float(c)), _c_int(J.shape[0]), ptr(q),
-                                                           _c_int(q.shape[0]), ptr(E)))
-    return E.astype(dtype)
+
+    def submit(J, q):
+        E = np.empty(q.shape[0], np.float64)
+        _dg(dtype)('calculate_E_from_spin', ptr(h), ptr(J), _real(dtype)(float(c)), _c_int(J.shape[0]), ptr(q),
+                   _c_int(q.shape[0]), ptr(E))
+        return E
+    return _symmetric(J, dtype, submit, rows).astype(dtype)
 
 
 # --------------------------------------------------------------- bipartite graph
