@@ -542,7 +542,8 @@ private:
             else if (!r->large)
                 running = std::max(running, r->persistentUs);
         }
-        for (const Request *r : queue_) {
+        for (size_t i = 0; i < std::min<size_t>(queue_.size(), 1024); ++i) {  // (the rest wait behind these)
+            const Request *r = queue_[i];
             if (r->kind == 0)
                 dense.push_back({r->N0, r->m, r->packCap, r->persistentUs, heavy_(*r)});
             else if (r->kind == 1 && !heavy_(*r))
