@@ -30,7 +30,8 @@ struct McConst {
 // negative, NaN or too large: simulated annealing at G = 0, an infinite beta; a ring
 // coefficient that is NaN or too large) gets constants that leave z = 0 within the
 // tolerance, so that every trial takes its FP64 outcome.  With coef = -inf (SQA at G = 0,
-// beta = 0) the sign of a nonzero spin sum decides, and a sum of zero its FP64 outcome.
+// beta = 0) the sign of a nonzero spin sum decides, whatever the field, and a sum of zero
+// takes its FP64 outcome.
 SQ103_HD McConst mc_const(bool sa, float twoDivM, float coef, float rate, float L) {
     McConst c;
     c.cz = rate * (sa ? 2.f : twoDivM);
@@ -40,6 +41,7 @@ SQ103_HD McConst mc_const(bool sa, float twoDivM, float coef, float rate, float 
         c.L = fminf(L, kMcCap);
         c.tolC = 4e-6f * fabsf(c.cb) + 2e-6f + 1e-6f * c.L;
         if (ringOnly) {
+            c.cz = 0.f;
             c.cb = -1e37f;
             c.tolC = 1e37f;
         }

@@ -151,7 +151,11 @@ __device__ __forceinline__ bool metropolis(float dE, float rate, float u) {
     return expf(__fmul_rn(-dE, rate)) > u;
 }
 
-// per-step constants, evaluated on the device by every kernel with the same code
+// per-step constants, evaluated on the device by every kernel with the same code.  An
+// infinite rate (G = 0, beta = inf) is held as the largest float, so that a trial whose
+// fp32 dE is zero has a product to compare (0 times infinity would reject it unflagged)
+// and is decided from its exact dE.
+constexpr float kRateMax = 3.402823466e38f;
 struct StepConst {
     float twoDivM, coef, rate;
 };
@@ -167,6 +171,7 @@ __device__ __forceinline__ StepConst step_const(int algo, int m, float G, float 
         s.coef = __fdiv_rn(logf(tanhf(arg)), beta);
         s.rate = beta;
     }
+    if (s.rate > kRateMax) s.rate = kRateMax;
     return s;
 }
 
@@ -398,7 +403,7 @@ __device__ __forceinline__ int exact_accept_log(bool sa, bool twoF, float q, dou
     const double b = __dmul_rn((double)(q * (float)sum), (double)sc.coef);  // coef = 0 for SA
     const double d = __dsub_rn(__dmul_rn(__dsub_rn(a, b), (double)sc.rate), (double)L);
     const float bound = __fadd_rn(tol.kC, __fmul_rn(2.4e-7f, fminf(L, 1e30f)));
-    if (fabs(d) <= (double)bound) return -1;
+    if (fabs(d) <= (double)bound || sc.rate == kRateMax) return -1;
     return d < 0.0 ? 1 : 0;
 }
 #endif

@@ -68,7 +68,8 @@ static unsigned sequential(const Batch &B) {
 // the rounds; false if they do not end
 static bool rounds(const Batch &B, unsigned &accBits, int &exact) {
     const float twoDivM = 2.f / B.m;
-    const float coef = B.sa ? 0.f : logf(tanhf(B.G * B.beta / B.m)) / B.beta, rate = B.sa ? 1.f / B.G : B.beta;
+    const float coef = B.sa ? 0.f : logf(tanhf(B.G * B.beta / B.m)) / B.beta;
+    const float rate = fminf(B.sa ? 1.f / B.G : B.beta, std::numeric_limits<float>::max());  // (step_const)
     McConst c[kLanes];
     float qx[kLanes], c2[kLanes], zA[kLanes], tol[kLanes];
     bool unknown[kLanes][2];
