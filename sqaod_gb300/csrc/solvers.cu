@@ -1071,10 +1071,12 @@ private:
         }
     }
 
-    // half-step fields on the tensor cores: the largest shapes always, the others only
-    // when the digits are as fine as the fp32 couplings for every spin
+    // Half-step fields on the tensor cores: only with digits as fine as the fp32 couplings
+    // for every spin; on the largest shapes up to a spread of 2^20, where the trials that
+    // the digits' rounding flags still cost less than the SIMT fields (2900 x 1100, m = 129,
+    // 32 steps: one coupling of 1e6 6.9 ms SIMT, 4.7 on digits; 1e7 (1100 x 2900) 13.1, 28.2).
     bool tcFields() const {
-        return useTc() && (!uneven_ || sq103_bipartite_refresh_uses_tc(N0_, N1_, m_));
+        return useTc() && spread_ <= (sq103_bipartite_refresh_uses_tc(N0_, N1_, m_) ? 20 : 5);
     }
     // energies on the tensor cores
     bool useTc() const { return d_digits1_.p && sq103_bipartite_tc_pays(N0_, N1_, m_); }
@@ -1084,9 +1086,9 @@ private:
         if (!d_digits1_.p) return;
         SQ_CHECK(sq103_tc_make_digits(d_J_.p, N0_, N1_, N0_, 0, d_digits1_.p, st_.get()));
         SQ_CHECK(sq103_tc_make_digits(d_J_.p, N0_, N0_, N1_, 1, d_digits0_.p, st_.get()));
-        d_uneven_.ensure(1);
-        SQ_CHECK(sq103_tc_check_even(d_J_.p, N0_, N1_, N0_, d_digits1_.p, d_uneven_.p, st_.get()));
-        SQ_CHECK(cudaMemcpyAsync(&uneven_, d_uneven_.p, sizeof(int), cudaMemcpyDeviceToHost, st_.get()));
+        d_spread_.ensure(1);
+        SQ_CHECK(sq103_tc_spread(d_J_.p, N0_, N1_, N0_, d_digits1_.p, d_spread_.p, st_.get()));
+        SQ_CHECK(cudaMemcpyAsync(&spread_, d_spread_.p, sizeof(int), cudaMemcpyDeviceToHost, st_.get()));
         st_.sync();
     }
 
@@ -1192,8 +1194,8 @@ private:
     DevBuf<double> d_J64_, d_h0_64_, d_h1_64_;        // FP64 problem of a <double> annealer
     DevBuf<unsigned char> d_digits1_, d_digits0_, d_Abf_;  // tensor-core half-step fields
     LowDigits low_;                                        // tensor-core energies
-    int uneven_ = 0;  // the digits are coarser than fp32 for some spin
-    DevBuf<int> d_status_, d_uneven_;
+    int spread_ = 0;  // sq103_tc_spread of the digits
+    DevBuf<int> d_status_, d_spread_;
     DevBuf<int8_t> d_q0_, d_q1_;
     DevBuf<unsigned long long> d_acc_;
     DevBuf<long long> d_ring_;

@@ -48,10 +48,9 @@ extern "C" int sq103_tc_refresh_after(const void *digits, int R, int K, const in
 extern "C" int sq103_bipartite_tc_pays(int N0, int N1, int m);
 // the shift S of a digit buffer (device memory): its matrix is rounded to multiples of 2^-S
 inline const int *sq103_tc_shift_of(const void *digits) { return static_cast<const int *>(digits) + 4; }
-// *uneven (device) = 1 when the digits of J (R x K, row stride ldJ), for J or J^T, would
-// hold a row less finely than fp32 holds its largest coupling
-extern "C" int sq103_tc_check_even(const float *J, int ldJ, int R, int K, const void *digits, int *uneven,
-                                   cudaStream_t st);
+// *spread (device) = how many powers of two the largest coupling of a row or column of J (R x
+// K, row stride ldJ), of those that the digits round, lies below the largest of all
+extern "C" int sq103_tc_spread(const float *J, int ldJ, int R, int K, const void *digits, int *spread, cudaStream_t st);
 // the planes of what `high`, the digits of J (R x K, row stride ldJ), round away (same layout and size)
 extern "C" int sq103_tc_make_low_digits(const float *J, int ldJ, int R, int K, const void *high, void *digits,
                                         cudaStream_t st);

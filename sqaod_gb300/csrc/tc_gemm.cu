@@ -448,15 +448,16 @@ __global__ void tc_make_digits(const float *J, int ldJ, int R, int K, int ldD, i
     }
 }
 
-// Sets *uneven when the digits are too coarse for some row or column of J (R x K): one
-// that holds a coupling the digits round and whose largest is below 2^24 quanta 2^-S, so
-// that the rounding exceeds the fp32 rounding of that largest coupling.  Couplings of one
-// magnitude, and integers below 2^30, are even; one coupling far above the rest makes the
-// other rows uneven.  Blocks below rowBlocks: a warp per row; the rest: 32 columns each.
-__global__ void __launch_bounds__(256) tc_check_even(const float *J, int ld, int R, int K, const unsigned *maxExp,
-                                                     int rowBlocks, int *uneven) {
+// *spread = how far, in powers of two, the largest coupling of some row or column of J (R x
+// K) lies below the matrix's, of those that hold a coupling the digits round (255 with a
+// non-finite coupling).  Up to 5, the digits are as fine as fp32 holds a row's largest
+// coupling (2^24 quanta 2^-S or more).  Couplings of one magnitude, and integers below
+// 2^30, have no spread; one coupling far above the rest gives the other rows one.
+// Blocks below rowBlocks: a warp per row; the rest: 32 columns each.
+__global__ void __launch_bounds__(256) tc_spread(const float *J, int ld, int R, int K, const unsigned *maxExp,
+                                                 int rowBlocks, int *spread) {
     __shared__ unsigned top[8][32];
-    const unsigned E = *maxExp, coarse = 5u << 23;
+    const unsigned E = *maxExp;
     const float scale = __int_as_float((tc_shift(E) + 127) << 23);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned e = 0;  // the largest exponent, bit 0 set when a value is rounded
@@ -480,7 +481,8 @@ __global__ void __launch_bounds__(256) tc_check_even(const float *J, int ld, int
         __syncthreads();
         for (int w = 0; w < 8; ++w) e = max(e & ~1u, top[w][lane] & ~1u) | ((e | top[w][lane]) & 1u);
     }
-    if (((e & 1u) && (e & ~1u) + coarse < E) || E == 0x7f800000u) *uneven = 1;
+    const int gap = E == 0x7f800000u ? 255 : (e & 1u) ? (int)((E - (e & ~1u)) >> 23) : 0;
+    if (gap > *spread) atomicMax(spread, gap);
 }
 
 // spins (m x K int8, row stride ldq) -> bf16 (m x ldA), zero beyond K
@@ -607,13 +609,13 @@ SQ103_API int sq103_tc_make_digits(const float *J, int ldJ, int R, int K, int tr
     return make_digits(J, ldJ, R, K, transpose, nullptr, digits, stream);
 }
 
-int sq103_tc_check_even(const float *J, int ldJ, int R, int K, const void *digits, int *uneven, cudaStream_t st) {
-    if (R <= 0 || K <= 0 || !J || !digits || !uneven) return kErrBadShape;
-    const cudaError_t e = cudaMemsetAsync(uneven, 0, sizeof(int), st);
+int sq103_tc_spread(const float *J, int ldJ, int R, int K, const void *digits, int *spread, cudaStream_t st) {
+    if (R <= 0 || K <= 0 || !J || !digits || !spread) return kErrBadShape;
+    const cudaError_t e = cudaMemsetAsync(spread, 0, sizeof(int), st);
     if (e != cudaSuccess) return (int)e;
     const int rowBlocks = (R + 7) / 8;
-    tc_check_even<<<rowBlocks + (K + 31) / 32, 256, 0, st>>>(J, ldJ, R, K, static_cast<const unsigned *>(digits),
-                                                            rowBlocks, uneven);
+    tc_spread<<<rowBlocks + (K + 31) / 32, 256, 0, st>>>(J, ldJ, R, K, static_cast<const unsigned *>(digits), rowBlocks,
+                                                        spread);
     return (int)cudaGetLastError();
 }
 
@@ -671,7 +673,7 @@ SQ103_API int sq103_bipartite_refresh_uses_tc(int N0, int N1, int m) {
 }
 
 // Where the bipartite annealer takes its energies, and its half-step fields when the
-// digits hold every row (sq103_tc_check_even), to the tensor cores: as above, and from
+// digits hold every row (sq103_tc_spread), to the tensor cores: as above, and from
 // about 80 M products a half-step on (m rounded up to a SIMT tile's 16 rows).  32 steps in
 // ms, SIMT and tensor cores: 1024 x 1024, m = 64 (67 M) 1.10, 1.18, m = 65 (84 M) 1.57,
 // 1.20; 1100 x 1900, m = 33 (100 M) 2.17, 1.28; 600 x 9000, m = 1 (86 M) 5.33, 1.38; 2300 x

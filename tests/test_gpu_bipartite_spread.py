@@ -25,7 +25,8 @@ def _problem(N0, N1, outlier, integer):
 @pytest.mark.parametrize("N0,N1,m,algo,outlier,integer", [
     (1100, 2900, 20, "coloring", 1e5, False), (1100, 2900, 20, "coloring", -1e6, True),
     (2900, 1100, 20, "sa_coloring", 1e6, False), (1100, 2900, 20, "coloring", 20.0, False),
-    (1030, 1100, 400, "coloring", 1e5, False), (1030, 1100, 400, "sa_coloring", 1e4, False)])
+    (1030, 1100, 400, "coloring", 1e5, False), (1030, 1100, 400, "sa_coloring", 1e4, False),
+    (1030, 1100, 400, "coloring", 1e9, False)])
 def test_one_large_coupling_replays(orc, N0, N1, m, algo, outlier, integer):
     import sqaod_gb300 as sq
     b0, b1, W = _problem(N0, N1, outlier, integer)
