@@ -131,7 +131,9 @@ SQ103_API int sq103_tc_make_digits(const float *J, int ldJ, int R, int K, int tr
  * block's copies are never issued, 2 = waits give up after 1 ms. */
 SQ103_API int sq103_tc_refresh(const void *digits, int R, int K, const int8_t *q, int ldq, int m, void *spinsBf16,
                                float *F, int ldF, int flags, int *status, void *stream);
-/* 1 when the dense annealers refresh N-spin fields on the tensor cores (N >= 1024) */
+/* 1 when the dense annealers refresh N-spin fields on the tensor cores (N >= 1024), which
+ * they do unless one coupling is so far above the others that the digits, on one scale
+ * for the whole matrix, are too coarse for these: then as below 1024 */
 SQ103_API int sq103_dense_refresh_uses_tc(int N);
 /* 1 when the half-step fields come from the tensor cores whatever the couplings (N0 N1
  * >= 2^20 and at least 64 output tiles of 128 trotters x 64 spins per half step); the

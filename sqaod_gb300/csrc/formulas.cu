@@ -194,6 +194,15 @@ __global__ void __launch_bounds__(256) field_batch_kernel(const sq103_field_job 
     bip_field_tile<false, false, float>(jb.q, jb.N, jb.J, jb.ldJ, jb.F, jb.N, jb.m, jb.N, jb.N, y0, n0, bip_smem);
 }
 
+// The single refresh's fields, over those of coarse digits (sq_kernels.h).
+__global__ void __launch_bounds__(256) field_if_coarse(const int8_t *q, const float *J, int ldJ, float *F, int N, int m,
+                                                       const sq103_tc_header *header) {
+    extern __shared__ __align__(16) float bip_smem[];
+    if (!digits_coarse(header->shift, header->spread, N)) return;
+    bip_field_tile<false, false, float>(q, N, J, ldJ, F, N, m, N, N, blockIdx.y * kBipTileM, blockIdx.x * kBipTileN,
+                                        bip_smem);
+}
+
 }  // namespace sq103
 
 using namespace sq103;
@@ -228,6 +237,15 @@ SQ103_API int sq103_dense_field_refresh(const float *J, int ldJ, const int8_t *q
     // 16 x 32 tiles with K split over the CTA's warps; 64 x 64 tiles that walked the whole K
     // took, in us (these: second): N = 128, m = 16 10.1, 4.6; 512, 128 36.3, 7.5; 1000, 250 70.9, 36.1
     launch_bip_field<false, false, float>(q, N, J, ldJ, F, N, m, N, N, s);
+    return (int)cudaGetLastError();
+}
+
+int sq103_dense_refresh_checked(const float *J, int ldJ, const void *digits, void *spinsBf16, const int8_t *q, float *F,
+                                int N, int m, int *status, cudaStream_t st) {
+    const int rc = sq103_dense_refresh(J, ldJ, digits, spinsBf16, q, F, N, m, status, st);
+    if (rc != 0 || !digits) return rc;
+    field_if_coarse<<<dim3((N + kBipTileN - 1) / kBipTileN, (m + kBipTileM - 1) / kBipTileM), 256, kBipFieldSmem, st>>>(
+        q, J, ldJ, F, N, m, static_cast<const sq103_tc_header *>(digits));
     return (int)cudaGetLastError();
 }
 

@@ -307,7 +307,7 @@ public:
             r->pos = std::min(r->pos + kStepsPerTick, r->nSteps);
             if (r->kind == 0 && r->pos < r->nSteps && r->pos % kRefreshPeriod == 0) {
                 if (r->digits) {  // on the side streams, forked from the work stream at the first
-                    SQ_CHECK(sq103_dense_refresh(r->dt.J, r->dt.ldJ, r->digits, r->spinsBf16, r->dt.q, r->dt.F, r->N0,
+                    SQ_CHECK(sq103_dense_refresh_checked(r->dt.J, r->dt.ldJ, r->digits, r->spinsBf16, r->dt.q, r->dt.F, r->N0,
                                                  r->m, r->dStatus, fork(nTc++)));
                 } else {  // below the tensor-core size: with the others, in one launch
                     sq103_field_job j = {};
@@ -663,7 +663,7 @@ private:
                                              st_.get()));
             if (r->digits) SQ_CHECK(sq103_tc_make_digits(J, (int)ldJ, (int)N, (int)N, 0, r->digits, st_.get()));
             SQ_CHECK(sq103_randomize_spins(q, (int)N, m, r->seed, 0, 0, st_.get()));
-            SQ_CHECK(sq103_dense_refresh(J, (int)ldJ, r->digits, r->spinsBf16, q, F, (int)N, m, r->dStatus,
+            SQ_CHECK(sq103_dense_refresh_checked(J, (int)ldJ, r->digits, r->spinsBf16, q, F, (int)N, m, r->dStatus,
                                          st_.get()));
             sq103_dense_task &t = r->dt;
             t = sq103_dense_task{};

@@ -114,6 +114,14 @@ struct LowDigits {
     }
 };
 
+// the header of a digit buffer (waits for the stream)
+static sq103_tc_header digit_header(const void *digits, Stream &st) {
+    sq103_tc_header h;
+    SQ_CHECK(cudaMemcpyAsync(&h, digits, sizeof(h), cudaMemcpyDeviceToHost, st.get()));
+    st.sync();
+    return h;
+}
+
 // a matrix with row stride = columns
 template <class real>
 static std::vector<real> dense_copy(const sq::MatrixType<real> &M) {
@@ -517,7 +525,10 @@ private:
 
     void makeDigits() {
         low_.made = false;
-        if (d_digits_.p) SQ_CHECK(sq103_tc_make_digits(d_J_.p, ldJ_, N_, N_, 0, d_digits_.p, st_.get()));
+        if (!d_digits_.p) return;
+        SQ_CHECK(sq103_tc_make_digits(d_J_.p, ldJ_, N_, N_, 0, d_digits_.p, st_.get()));
+        const sq103_tc_header h = digit_header(d_digits_.p, st_);
+        coarse_ = digits_coarse(h.shift, h.spread, N_);
     }
 
     void allocFP64() {
@@ -554,7 +565,7 @@ private:
     }
 
     void refreshFields() {
-        SQ_CHECK(sq103_dense_refresh(d_J_.p, ldJ_, d_digits_.p, d_Abf_.p, d_q_.p, d_F_.p, N_, m_, d_status_.p,
+        SQ_CHECK(sq103_dense_refresh(d_J_.p, ldJ_, coarse_ ? nullptr : d_digits_.p, d_Abf_.p, d_q_.p, d_F_.p, N_, m_, d_status_.p,
                                      st_.get()));
         stepsSinceRefresh_ = 0;
     }
@@ -649,6 +660,7 @@ private:
     mutable Stream st_;
     DevBuf<float> d_J_, d_h_, d_c_, d_F_, d_E32_, d_sched_;
     DevBuf<unsigned char> d_digits_, d_Abf_;  // tensor-core refresh: digit planes of J, spins in bf16
+    bool coarse_ = false;                     // the digits are too coarse for fields
     LowDigits low_;                           // tensor-core energies
     DevBuf<double> d_J64_, d_h64_;            // FP64 problem of a <double> annealer (J64 row stride N)
     double c64h_ = 0.;
@@ -1076,7 +1088,7 @@ private:
     // the digits' rounding flags still cost less than the SIMT fields (2900 x 1100, m = 129,
     // 32 steps: one coupling of 1e6 6.9 ms SIMT, 4.7 on digits; 1e7 (1100 x 2900) 13.1, 28.2).
     bool tcFields() const {
-        return useTc() && spread_ <= (sq103_bipartite_refresh_uses_tc(N0_, N1_, m_) ? 20 : 5);
+        return useTc() && spread_ <= (sq103_bipartite_refresh_uses_tc(N0_, N1_, m_) ? 20 : kEvenSpread);
     }
     // energies on the tensor cores
     bool useTc() const { return d_digits1_.p && sq103_bipartite_tc_pays(N0_, N1_, m_); }
@@ -1086,10 +1098,7 @@ private:
         if (!d_digits1_.p) return;
         SQ_CHECK(sq103_tc_make_digits(d_J_.p, N0_, N1_, N0_, 0, d_digits1_.p, st_.get()));
         SQ_CHECK(sq103_tc_make_digits(d_J_.p, N0_, N0_, N1_, 1, d_digits0_.p, st_.get()));
-        d_spread_.ensure(1);
-        SQ_CHECK(sq103_tc_spread(d_J_.p, N0_, N1_, N0_, d_digits1_.p, d_spread_.p, st_.get()));
-        SQ_CHECK(cudaMemcpyAsync(&spread_, d_spread_.p, sizeof(int), cudaMemcpyDeviceToHost, st_.get()));
-        st_.sync();
+        spread_ = digit_header(d_digits1_.p, st_).spread;
     }
 
     void allocFP64() {
@@ -1194,8 +1203,8 @@ private:
     DevBuf<double> d_J64_, d_h0_64_, d_h1_64_;        // FP64 problem of a <double> annealer
     DevBuf<unsigned char> d_digits1_, d_digits0_, d_Abf_;  // tensor-core half-step fields
     LowDigits low_;                                        // tensor-core energies
-    int spread_ = 0;  // sq103_tc_spread of the digits
-    DevBuf<int> d_status_, d_spread_;
+    int spread_ = 0;  // of the digits (sq103_tc_header)
+    DevBuf<int> d_status_;
     DevBuf<int8_t> d_q0_, d_q1_;
     DevBuf<unsigned long long> d_acc_;
     DevBuf<long long> d_ring_;
@@ -1939,6 +1948,7 @@ public:
     struct Inst {
         int N, m, ldJ;  // J rows on a 16-byte stride (the one-CTA-per-trotter sweep reads them as float4)
         bool multi = false;
+        bool coarse = false;  // digits too coarse for fields
         unsigned long long seed;
         DevBuf<unsigned char> mem, ws;
         DevBuf<unsigned char> digits, Abf;  // tensor-core refresh (N >= 1024), as the single annealer
@@ -1986,7 +1996,11 @@ public:
         SQ_CHECK(cudaMemsetAsync(in.J, 0, sizeof(float) * N * in.ldJ, st_.get()));  // zero row padding
         SQ_CHECK(sq103_dense_hamiltonian(dW_.p, N, N, optimize, in.h, in.J, in.ldJ, in.c32, in.c64, scratch_.p,
                                          st_.get()));
-        if (in.digits.p) SQ_CHECK(sq103_tc_make_digits(in.J, in.ldJ, N, N, 0, in.digits.p, st_.get()));
+        if (in.digits.p) {
+            SQ_CHECK(sq103_tc_make_digits(in.J, in.ldJ, N, N, 0, in.digits.p, st_.get()));
+            const sq103_tc_header h = digit_header(in.digits.p, st_);
+            in.coarse = digits_coarse(h.shift, h.spread, N);
+        }
         st_.sync();
         optimize_.push_back(optimize);
         return (int)insts_.size() - 1;
@@ -2377,7 +2391,7 @@ private:
         tcInsts_.clear();
         for (auto &p : insts_) {
             Inst &in = *p;
-            if (in.digits.p) {
+            if (in.digits.p && !in.coarse) {
                 tcInsts_.push_back(&in);
                 continue;
             }

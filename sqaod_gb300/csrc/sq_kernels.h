@@ -46,11 +46,28 @@ extern "C" int sq103_tc_refresh_after(const void *digits, int R, int K, const in
                                       cudaStream_t st);
 
 extern "C" int sq103_bipartite_tc_pays(int N0, int N1, int m);
-// the shift S of a digit buffer (device memory): its matrix is rounded to multiples of 2^-S
-inline const int *sq103_tc_shift_of(const void *digits) { return static_cast<const int *>(digits) + 4; }
-// *spread (device) = how many powers of two the largest coupling of a row or column of J (R x
-// K, row stride ldJ), of those that the digits round, lies below the largest of all
-extern "C" int sq103_tc_spread(const float *J, int ldJ, int R, int K, const void *digits, int *spread, cudaStream_t st);
+// the head of a digit buffer (device memory): its matrix is rounded to multiples of 2^-shift
+struct sq103_tc_header {
+    unsigned maxExp;
+    int pad0[3];
+    int shift;
+    int pad1[3];
+    int spread;  // of the matrix (tc_spread; 0 in the digits of a transpose)
+};
+inline const int *sq103_tc_shift_of(const void *digits) { return &static_cast<const sq103_tc_header *>(digits)->shift; }
+namespace sq103 {
+constexpr int kEvenSpread = 5;  // up to here the digits are as fine as fp32 for every row
+// The digits of an uneven matrix with K columns are too coarse for fields where their
+// rounding, up to K 2^-(shift + 1) a field, may exceed half of the drift that the dense
+// decisions allow for at any field (2^-16 in h + 2F).
+__host__ __device__ inline bool digits_coarse(int shift, int spread, int K) {
+    return spread > kEvenSpread && (shift <= 0 || (shift < 40 && ((long long)K << 17) > 1ll << shift));
+}
+}  // namespace sq103
+// sq103_dense_refresh where the host has not seen the header: the tensor-core fields, and
+// over them the SIMT ones when the digits are coarse
+extern "C" int sq103_dense_refresh_checked(const float *J, int ldJ, const void *digits, void *spinsBf16,
+                                           const int8_t *q, float *F, int N, int m, int *status, cudaStream_t st);
 // the planes of what `high`, the digits of J (R x K, row stride ldJ), round away (same layout and size)
 extern "C" int sq103_tc_make_low_digits(const float *J, int ldJ, int R, int K, const void *high, void *digits,
                                         cudaStream_t st);

@@ -482,7 +482,7 @@ __global__ void __launch_bounds__(256) tc_spread(const float *J, int ld, int R, 
         for (int w = 0; w < 8; ++w) e = max(e & ~1u, top[w][lane] & ~1u) | ((e | top[w][lane]) & 1u);
     }
     const int gap = E == 0x7f800000u ? 255 : (e & 1u) ? (int)((E - (e & ~1u)) >> 23) : 0;
-    if (gap > *spread) atomicMax(spread, gap);
+    if (gap > 0) atomicMax(spread, gap);  // (few rows of an ordinary matrix have one)
 }
 
 // spins (m x K int8, row stride ldq) -> bf16 (m x ldA), zero beyond K
@@ -594,7 +594,7 @@ static int make_digits(const float *J, int ldJ, int R, int K, int transpose, con
     unsigned char *base = static_cast<unsigned char *>(digits);
     unsigned *header = reinterpret_cast<unsigned *>(base);
     if (!high) {
-        cudaError_t e = cudaMemsetAsync(header, 0, sizeof(unsigned), st);
+        cudaError_t e = cudaMemsetAsync(header, 0, sizeof(sq103_tc_header), st);
         if (e != cudaSuccess) return (int)e;
         const int rowsJ = transpose ? K : R, colsJ = transpose ? R : K;
         tc_max_exponent<<<std::min(rowsJ, 152 * 4), 256, 0, st>>>(J, ldJ, rowsJ, colsJ, header);
@@ -602,21 +602,16 @@ static int make_digits(const float *J, int ldJ, int R, int K, int transpose, con
     tc_make_digits<<<std::min(R, 152 * 16), 256, 0, st>>>(J, ldJ, R, K, ld_pad(K), transpose, high != nullptr,
                                                           high ? static_cast<const unsigned *>(high) : header, header,
                                                           reinterpret_cast<__nv_bfloat16 *>(base + kTcHeader));
+    if (!high && !transpose) {
+        const int rowBlocks = (R + 7) / 8;
+        tc_spread<<<rowBlocks + (K + 31) / 32, 256, 0, st>>>(J, ldJ, R, K, header, rowBlocks,
+                                                            &static_cast<sq103_tc_header *>(digits)->spread);
+    }
     return (int)cudaGetLastError();
 }
 
 SQ103_API int sq103_tc_make_digits(const float *J, int ldJ, int R, int K, int transpose, void *digits, void *stream) {
     return make_digits(J, ldJ, R, K, transpose, nullptr, digits, stream);
-}
-
-int sq103_tc_spread(const float *J, int ldJ, int R, int K, const void *digits, int *spread, cudaStream_t st) {
-    if (R <= 0 || K <= 0 || !J || !digits || !spread) return kErrBadShape;
-    const cudaError_t e = cudaMemsetAsync(spread, 0, sizeof(int), st);
-    if (e != cudaSuccess) return (int)e;
-    const int rowBlocks = (R + 7) / 8;
-    tc_spread<<<rowBlocks + (K + 31) / 32, 256, 0, st>>>(J, ldJ, R, K, static_cast<const unsigned *>(digits), rowBlocks,
-                                                        spread);
-    return (int)cudaGetLastError();
 }
 
 int sq103_tc_make_low_digits(const float *J, int ldJ, int R, int K, const void *high, void *digits, cudaStream_t st) {
@@ -658,8 +653,9 @@ int sq103_tc_row_sums(const void *digits, const void *lowDigits, int R, int K, c
 
 // The dense refresh every path runs (single annealer, batch, server, bench): the
 // tensor-core digit contraction when a digit buffer is given, else the SIMT spin
-// GEMM.  Which one a path uses is decided by sq103_dense_refresh_uses_tc(N) alone,
-// so every path that anneals the same instance holds the same fields.
+// GEMM.  Which one a path uses is decided by sq103_dense_refresh_uses_tc(N) and
+// digits_coarse() of its digits, so every path that anneals the same instance holds the
+// same fields.
 SQ103_API int sq103_dense_refresh_uses_tc(int N) { return N >= 1024 ? 1 : 0; }
 
 // Bipartite half-step fields on the tensor cores for problems of at least 2^20
@@ -673,7 +669,7 @@ SQ103_API int sq103_bipartite_refresh_uses_tc(int N0, int N1, int m) {
 }
 
 // Where the bipartite annealer takes its energies, and its half-step fields when the
-// digits hold every row (sq103_tc_spread), to the tensor cores: as above, and from
+// digits hold every row (kEvenSpread), to the tensor cores: as above, and from
 // about 80 M products a half-step on (m rounded up to a SIMT tile's 16 rows).  32 steps in
 // ms, SIMT and tensor cores: 1024 x 1024, m = 64 (67 M) 1.10, 1.18, m = 65 (84 M) 1.57,
 // 1.20; 1100 x 1900, m = 33 (100 M) 2.17, 1.28; 600 x 9000, m = 1 (86 M) 5.33, 1.38; 2300 x
