@@ -120,24 +120,6 @@ def _dense_rows(W, x, caption):
     return np.ascontiguousarray(x.reshape(-1, W.shape[0]))
 
 
-def _symmetric(W, dtype, submit, check=lambda: None):
-    """submit(W, check()) with the outcome of symmetrize(W) before both, without its allclose
-    pass: a symmetric W is checked exactly on the device.  That check passes over the
-    diagonal, where symmetrize refuses a NaN.  A NaN there makes the first value that submit
-    returns one, except that the float64 energies skip what a bit vector does not select, so
-    W is looked at again then, and in float64 its diagonal always (reading it takes some 5
-    us at N = 1000).  Where anything raises, a W that symmetrize refuses is reported first."""
-    try:
-        arg = check()
-        result = common.submit_symmetric(W, dtype, lambda W: submit(W, arg))
-    except Exception:
-        common.symmetrize(W)
-        raise
-    if result[0] != result[0] or (dtype == np.float64 and np.isnan(W.diagonal()).any()):
-        common.symmetrize(W)
-    return result
-
-
 def _bipartite_problem(v0, v1, M, names):
     _vector(names[0], v0)
     _vector(names[1], v1)
@@ -165,17 +147,28 @@ def dense_graph_calculate_E(W, x, dtype):
     return dense_graph_batch_calculate_E(W, x, dtype)[0]
 
 
+# A symmetric W is checked exactly on the device, without symmetrize's allclose pass, and the
+# outcome is as if symmetrize(W) came first: where anything raises, a W that it refuses is
+# reported, and one with a NaN on its diagonal, which the device check passes over, is
+# found by the NaN in the first result (the float64 energies skip what a bit vector does
+# not select, so there the diagonal is read).
+
 def dense_graph_batch_calculate_E(W, x, dtype):
     """QUBO energies of the rows of x (1-D x is one row)."""
     dtype = _check_dtype(dtype)
     W = common.fix_type(W, dtype)
     _square('W', W)
-
-    def submit(W, x):
+    try:
+        x = _dense_rows(W, common.fix_type(x, np.int8), 'W, x')
         E = np.empty(x.shape[0], np.float64)
-        _dg(dtype)('calculate_E', ptr(W), _c_int(W.shape[0]), ptr(x), _c_int(x.shape[0]), ptr(E))
-        return E
-    return _symmetric(W, dtype, submit, lambda: _dense_rows(W, common.fix_type(x, np.int8), 'W, x')).astype(dtype)
+        common.submit_symmetric(W, dtype, lambda W: _dg(dtype)('calculate_E', ptr(W), _c_int(W.shape[0]), ptr(x),
+                                                               _c_int(x.shape[0]), ptr(E)))
+    except Exception:
+        common.symmetrize(W)
+        raise
+    if E[0] != E[0] or (dtype is np.float64 and np.isnan(W.trace())):
+        common.symmetrize(W)
+    return E.astype(dtype)
 
 
 def dense_graph_calculate_hamiltonian(W, dtype):
@@ -187,11 +180,10 @@ def dense_graph_calculate_hamiltonian(W, dtype):
     h = np.empty(N, dtype)
     J = np.empty((N, N), dtype)
     c = np.empty(1, dtype)
-
-    def submit(W, _):
-        _dg(dtype)('calculate_hamiltonian', ptr(W), _c_int(N), ptr(h), ptr(J), ptr(c))
-        return c
-    _symmetric(W, dtype, submit)
+    common.submit_symmetric(W, dtype, lambda W: _dg(dtype)('calculate_hamiltonian', ptr(W), _c_int(N), ptr(h), ptr(J),
+                                                           ptr(c)))
+    if c[0] != c[0]:
+        common.symmetrize(W)
     return h, J, c[0]
 
 
@@ -206,19 +198,21 @@ def dense_graph_batch_calculate_E_from_spin(h, J, c, q, dtype):
     h, J = common.fix_type([h, J], dtype)
     _vector('h', h)
     _square('J', J)
-
-    def rows():
+    try:
         _scalar('c', c)
         if h.shape[0] != J.shape[0]:
             _dims('h, J', h, J)
-        return _dense_rows(J, q, 'J, q')
-
-    def submit(J, q):
+        q = _dense_rows(J, q, 'J, q')
         E = np.empty(q.shape[0], np.float64)
-        _dg(dtype)('calculate_E_from_spin', ptr(h), ptr(J), _real(dtype)(float(c)), _c_int(J.shape[0]), ptr(q),
-                   _c_int(q.shape[0]), ptr(E))
-        return E
-    return _symmetric(J, dtype, submit, rows).astype(dtype)
+        common.submit_symmetric(J, dtype, lambda J: _dg(dtype)('calculate_E_from_spin', ptr(h), ptr(J),
+                                                               _real(dtype)(float(c)), _c_int(J.shape[0]), ptr(q),
+                                                               _c_int(q.shape[0]), ptr(E)))
+    except Exception:
+        common.symmetrize(J)
+        raise
+    if E[0] != E[0]:
+        common.symmetrize(J)
+    return E.astype(dtype)
 
 
 # --------------------------------------------------------------- bipartite graph
