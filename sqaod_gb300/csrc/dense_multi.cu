@@ -749,6 +749,7 @@ __global__ void __launch_bounds__(mc_threads(kPerSm), kPerSm) dense_sweep_multi(
             ++s;
         }
         StepConst sc = {0.f, 0.f, 0.f};
+        McConst mc = {0.f, 0.f, 0.f, 0.f};
         int own0 = -1, own1 = -1;  // kSmall: the neighbours' sites of this warp's last batch (p - 2)
         for (int p = pw; p < nBatches; p += kPf) {
             // buffer p % kPre is free once the decider has finished batch p - kPre,
@@ -779,6 +780,7 @@ __global__ void __launch_bounds__(mc_threads(kPerSm), kPerSm) dense_sweep_multi(
                 if (s != cs) {
                     const float G = T.G ? T.G[s] : T.Gs, beta = T.beta ? T.beta[s] : T.betas;
                     sc = step_const(T.algo, m, G, beta);
+                    mc = mc_const(sa, sc.twoDivM, sc.coef, sc.rate);
                     cs = s;
                 }
             }
@@ -973,11 +975,10 @@ __global__ void __launch_bounds__(mc_threads(kPerSm), kPerSm) dense_sweep_multi(
                 PreTrial tr;
                 tr.x = x;
                 tr.h = hs[x];
-                const McConst c = mc_const(sa, sc.twoDivM, sc.coef, sc.rate, neg_log_unit(u));
-                tr.L = c.L;
-                tr.cz = c.cz;
-                tr.cb = c.cb;
-                tr.tolC = c.tolC;
+                tr.L = mc_L(mc, neg_log_unit(u));
+                tr.cz = mc.cz;
+                tr.cb = mc.cb;
+                tr.tolC = mc_tol(mc, tr.L);
                 tr.u = u;
                 tr.cand = cands;
                 pre[buf * 32 + lane] = tr;

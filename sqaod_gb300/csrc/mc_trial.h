@@ -20,37 +20,38 @@ namespace sq103 {
 
 constexpr float kMcCap = 1e30f;  // largest factor that the fp32 form takes
 
-// dE's factors of h + 2F and of the spin sum times the rate, L, and the part of the
-// tolerance that does not depend on the field
+// A step's constants: dE's factors of h + 2F and of the spin sum times the rate, the
+// largest L, and the part of the tolerance that depends on neither the field nor L.
 struct McConst {
-    float cz, cb, L, tolC;
+    float cz, cb, maxL, tol;
 };
 
-// L is +inf for u = 0.  A step outside the fp32 form's range (a rate that is infinite,
-// negative, NaN or too large: simulated annealing at G = 0, an infinite beta; a ring
-// coefficient that is NaN or too large) gets constants that leave z = 0 within the
-// tolerance, so that every trial takes its FP64 outcome.  With coef = -inf (SQA at G = 0,
-// beta = 0) the sign of a nonzero spin sum decides, whatever the field, and a sum of zero
-// takes its FP64 outcome.
-SQ103_HD McConst mc_const(bool sa, float twoDivM, float coef, float rate, float L) {
+// A step outside the fp32 form's range (a rate that is infinite, negative, NaN or too
+// large: simulated annealing at G = 0, an infinite beta; a ring coefficient that is NaN or
+// too large) gets constants that leave z = 0 within the tolerance, so that every trial
+// takes its FP64 outcome.  With coef = -inf (SQA at G = 0, beta = 0) the sign of a nonzero
+// spin sum decides, whatever the field, and a sum of zero takes its FP64 outcome.
+SQ103_HD McConst mc_const(bool sa, float twoDivM, float coef, float rate) {
     McConst c;
     c.cz = rate * (sa ? 2.f : twoDivM);
     c.cb = sa ? 0.f : rate * coef;
+    c.maxL = kMcCap;
+    c.tol = 4e-6f * fabsf(c.cb) + 2e-6f;
     const bool ringOnly = !sa && coef == -INFINITY;
-    if (c.cz >= 0.f && c.cz <= kMcCap && (ringOnly || fabsf(c.cb) <= kMcCap)) {
-        c.L = fminf(L, kMcCap);
-        c.tolC = 4e-6f * fabsf(c.cb) + 2e-6f + 1e-6f * c.L;
-        if (ringOnly) {
-            c.cz = 0.f;
-            c.cb = -1e37f;
-            c.tolC = 1e37f;
-        }
-    } else {
-        c.cz = c.cb = c.L = 0.f;
-        c.tolC = kMcCap;
+    if (!(c.cz >= 0.f && c.cz <= kMcCap && (ringOnly || fabsf(c.cb) <= kMcCap))) {
+        c.cz = c.cb = c.maxL = 0.f;
+        c.tol = kMcCap;
+    } else if (ringOnly) {
+        c.cz = 0.f;
+        c.cb = -1e37f;
+        c.tol = 1e37f;
     }
     return c;
 }
+
+// a trial's L = -ln u (+inf for u = 0) and tolerance without the field's part
+SQ103_HD float mc_L(const McConst &c, float negLogU) { return fminf(negLogU, c.maxL); }
+SQ103_HD float mc_tol(const McConst &c, float L) { return c.tol + 1e-6f * L; }
 
 // certain to accept; neither certain to accept nor to reject (a NaN rejects)
 SQ103_HD bool mc_accepts(float z, float sp, float tol) { return z + sp < -tol; }

@@ -70,18 +70,18 @@ static bool rounds(const Batch &B, unsigned &accBits, int &exact) {
     const float twoDivM = 2.f / B.m;
     const float coef = B.sa ? 0.f : logf(tanhf(B.G * B.beta / B.m)) / B.beta;
     const float rate = fminf(B.sa ? 1.f / B.G : B.beta, std::numeric_limits<float>::max());  // (step_const)
-    McConst c[kLanes];
-    float qx[kLanes], c2[kLanes], zA[kLanes], tol[kLanes];
+    const McConst c = mc_const(B.sa, twoDivM, coef, rate);
+    float L[kLanes], qx[kLanes], c2[kLanes], zA[kLanes], tol[kLanes];
     bool unknown[kLanes][2];
     double F64[kSites], q64[kSites];  // what the exact warp sums
     for (int i = 0; i < kSites; ++i) F64[i] = B.F[i], q64[i] = B.q[i];
     for (int l = 0; l < kLanes; ++l) {
         const Trial &t = B.t[l];
-        c[l] = mc_const(B.sa, twoDivM, coef, rate, t.u > 0.f ? -logf(t.u) : INFINITY);
+        L[l] = mc_L(c, t.u > 0.f ? -logf(t.u) : INFINITY);
         qx[l] = B.q[t.x];
-        c2[l] = 2.f * c[l].cz * qx[l];
-        zA[l] = fmaf(c[l].cz * qx[l], fmaf(2.f, B.F[t.x], B.h[t.x]), -c[l].L);
-        tol[l] = fmaf(fabsf(c[l].cz) * 1.52587890625e-5f, fabsf(B.h[t.x]) + 2.f * fabsf(B.F[t.x]) + 1.f, c[l].tolC);
+        c2[l] = 2.f * c.cz * qx[l];
+        zA[l] = fmaf(c.cz * qx[l], fmaf(2.f, B.F[t.x], B.h[t.x]), -L[l]);
+        tol[l] = fmaf(fabsf(c.cz) * 1.52587890625e-5f, fabsf(B.h[t.x]) + 2.f * fabsf(B.F[t.x]) + 1.f, mc_tol(c, L[l]));
         for (int n = 0; n < 2; ++n) unknown[l][n] = !B.sa && t.unknown[n];
     }
     unsigned pending = ~0u;
@@ -95,7 +95,7 @@ static bool rounds(const Batch &B, unsigned &accBits, int &exact) {
             int known = B.t[l].sum, n = unknown[l][0] + unknown[l][1];
             if (n == 2) known = 0;
             if (n == 1) known = B.t[l].sum == 0 ? (unknown[l][0] ? 1 : -1) : B.t[l].sum / 2;
-            const float cbq = c[l].cb * qx[l], z = zA[l] - cbq * (float)known, sp = fabsf(cbq) * (float)n;
+            const float cbq = c.cb * qx[l], z = zA[l] - cbq * (float)known, sp = fabsf(cbq) * (float)n;
             if (mc_accepts(z, sp, tol[l]))
                 fa = l;
             else if (mc_open(z, sp, tol[l]))
@@ -123,11 +123,11 @@ static bool rounds(const Batch &B, unsigned &accBits, int &exact) {
         for (int l = fa + 1; l < kLanes; ++l) {
             const float dJ = df * B.J[xf][B.t[l].x];
             zA[l] = fmaf(c2[l], dJ, zA[l]);
-            tol[l] = fmaf(2.f * fabsf(c[l].cz) * 1.52587890625e-5f, fabsf(dJ), tol[l]);
+            tol[l] = fmaf(2.f * fabsf(c.cz) * 1.52587890625e-5f, fabsf(dJ), tol[l]);
             if (B.t[l].x == xf) {
                 qx[l] = -qx[l];
                 c2[l] = -c2[l];
-                zA[l] = -(zA[l] + c[l].L) - c[l].L;
+                zA[l] = -(zA[l] + L[l]) - L[l];
             }
         }
     }
