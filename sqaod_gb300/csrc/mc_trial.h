@@ -18,7 +18,10 @@
 
 namespace sq103 {
 
-constexpr float kMcCap = 1e30f;  // largest factor that the fp32 form takes
+// largest factor of the fp32 form: its products with fields up to 1e23 stay finite, so that
+// the flips of a batch add up (an infinite z would stay so)
+constexpr float kMcCap = 1e15f;
+constexpr float kMcMaxL = 1e30f;
 
 // A step's constants: dE's factors of h + 2F and of the spin sum times the rate, the
 // largest L, and the part of the tolerance that depends on neither the field nor L.
@@ -35,7 +38,7 @@ SQ103_HD McConst mc_const(bool sa, float twoDivM, float coef, float rate) {
     McConst c;
     c.cz = rate * (sa ? 2.f : twoDivM);
     c.cb = sa ? 0.f : rate * coef;
-    c.maxL = kMcCap;
+    c.maxL = kMcMaxL;
     c.tol = 4e-6f * fabsf(c.cb) + 2e-6f;
     const bool ringOnly = !sa && coef == -INFINITY;
     if (!(c.cz >= 0.f && c.cz <= kMcCap && (ringOnly || fabsf(c.cb) <= kMcCap))) {

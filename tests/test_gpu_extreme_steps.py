@@ -39,6 +39,8 @@ def _anneal(W, m, algo, G, beta, kernel):
     (81, 88, "sa_naive", [4.5, 0.0], 1.0, "sparse"),
     (113, 224, "coloring", [5.0, 0.5, 0.05], INF, "sparse"),
     (196, 23, "coloring", [3.0, 1.0, 0.0], 1e30, 1e20),
+    (82, 24, "coloring", [5.0, 1.0, 0.3, 0.1, 0.03, 0.01], 1e30, 1e22),
+    (75, 7, "coloring", [5.0, 1.0, 0.3, 0.1, 0.03, 0.01], 1e30, 1e27),
 ])
 def test_extreme_steps_equal_the_one_cta_kernel(N, m, algo, G, beta, coupling):
     rng = np.random.default_rng(N + m)
