@@ -269,7 +269,7 @@ struct McPack {
 // kPerSm: the CTAs per SM the registers are allotted for.  The trotters of a launch
 // are all resident, so the limit on m is kPerSm * 152 (where shared memory allows
 // as many: N <= 3100 for four).  Two leave 114 registers a thread and the fastest
-// decider; four have 72 (up to 16 bytes spilled) and take the launches that exceed two.
+// decider; four have 72 (up to 24 bytes spilled) and take the launches that exceed two.
 // N = 2000, m = 500, 8 steps: 3.7 ms with four per SM; one CTA for the whole
 // instance, which such sizes fell back to before, 1090 ms.
 template <bool kHooks, bool kSmall, bool kSA, int kPerSm>
